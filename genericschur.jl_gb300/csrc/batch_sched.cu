@@ -142,10 +142,6 @@ BinTuning default_tuning_mixed32() {
   return BinTuning{{32, 64, 96, 128}, {64, 64, 128, 128}, {1, 1, 0, 0}, {0, 0, 0, 0}};
 }
 
-// Largest dynamic shared memory a CTA may use on sm_103 (227 KiB), less the kernels'
-// static shared memory.
-static constexpr size_t kMaxDynSmem = 227 * 1024 - 1024;
-
 bool tuning_shape_ok(int kind, int nmax, int nt, int hsmem) {
   bool known = false;
   for (int t : kTuneThreads) known |= (t == nt);

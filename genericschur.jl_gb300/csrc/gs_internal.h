@@ -10,6 +10,10 @@ namespace gsk {
 // Largest matrix order handled by the one-CTA-per-matrix kernels.
 constexpr int kSmallMax = 128;
 
+// Largest dynamic shared memory a CTA may use on sm_103 (227 KiB), less the kernels'
+// static shared memory.
+constexpr size_t kMaxDynSmem = 227 * 1024 - 1024;
+
 // Per-matrix status codes (also the C-ABI return codes).
 enum : int { ST_OK = 0, ST_UNCONVERGED = 1, ST_BADARG = 2, ST_CUDA = 3 };
 // Internal per-matrix status of the mixed batched form: the refinement handed the matrix

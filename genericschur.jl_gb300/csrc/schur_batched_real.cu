@@ -1,29 +1,18 @@
 // Batched real Schur decomposition, one CTA per matrix (n <= 128), FP64 (and an FP32
-// instance of the same code for the FP32 stage of the mixed-precision form).
+// instance of the same code for Float32 batches and the FP32 stage of the mixed form).
 //
-// Each CTA pulls matrix indices from its size bin's work queue (a ticket counter
-// in global memory) and runs, for one matrix:
-//   1. load + _scale! (util.jl:14-29);
-//   2. Householder Hessenberg reduction (hessenberg.jl:3-17; reflector as in
-//      householder.jl:12-54, lmul!/rmul! as householder.jl:140-172), in shared
-//      memory for the small bins and in the L2-resident output buffer for the
-//      large ones;
-//   3. Q formation (hessenberg.jl:150-166) straight into the Z output, each thread
-//      owning whole rows of Z so that Z never needs a barrier;
-//   4. the real double-shift Francis iteration of gschur!(H::Hessenberg{<:Real}, Z)
-//      (GenericSchur.jl:513-699) with doubleShiftQR! (837-952) and _gs2x2!
-//      (716-803) on a packed copy of H in shared memory (column j keeps rows
-//      1..j+3: the Hessenberg part and the two rows of the 3x3 bulge), which lets
-//      three 128x128 matrices share one SM;
-//   5. T, eigenvalues and status written back, undoing the scaling.
-//
-// Bulge chase, one barrier per step: warp 0 owns the near-diagonal block of step k
-// (left update of columns k..k+2, right update of rows k..k+3) and then computes
-// the reflector of step k+1 from column k, while the other warps apply step k to
-// the far columns (k+3..n) and far rows (1..k-1).  The two sets are disjoint, and
-// everything step k+1 reads was written by one side or the other before the
-// barrier.  Each sweep's reflectors are logged and applied to the Z rows in one
-// streaming pass afterwards (every thread owns rows of Z).
+// Per size bin two launches over the bin's queue of matrices (largest first):
+//   k_hess_real   load + _scale! (util.jl:14-29), Householder Hessenberg reduction
+//                 (hessenberg.jl:3-17; reflector as in householder.jl:12-54, lmul!/rmul!
+//                 as householder.jl:140-172) and Q formation (hessenberg.jl:150-166);
+//   k_schur_real  the real double-shift Francis iteration of gschur!(H::Hessenberg{<:Real}, Z)
+//                 (GenericSchur.jl:513-699) with doubleShiftQR! (837-952) and _gs2x2!
+//                 (716-803) on a packed copy of H in shared memory (column j keeps rows
+//                 1..j+3: the Hessenberg part and the two rows of the 3x3 bulge); T,
+//                 eigenvalues and status written back, undoing the scaling.
+// They are separate kernels because they want different shapes: the reduction needs the full
+// matrix (and Z) in shared memory and many threads, the iteration is a chain of short
+// dependent steps per matrix that wants as many matrices per SM as fit.
 #include <type_traits>
 
 #include "device_common.cuh"
@@ -37,159 +26,452 @@ struct Refl {
   T t1, t2, t3, v2, v3;
 };
 
-template <class T>
-struct Ctl {
-  T v[3];        // start vector of the sweep
-  Refl<T> r[2];  // reflector of the current step / the next step
-  T s[4];        // shifts r1r, r1i, r2r, r2i
-  T g[2];        // Givens cs, sn of a 2x2 deflation
-  T blk[4];      // standardised 2x2 block
-  int split;
-  int mx;
-};
-
 // Packed QR layout: column j (1-based) holds rows 1..j+3.
 __host__ __device__ __forceinline__ int rpk(int j) { return ((j - 1) * (j + 6)) >> 1; }
 
-#define AA(i, j) A[((i) - 1) + ((j) - 1) * lda]
 #define HH(i, j) H[rpk(j) + (i) - 1]
 
-template <class T, int NT>
-__device__ void hessenberg_real(int n, T* A, int lda, T* tau, T* red) {
-  const int tid = threadIdx.x;
-  const T sfmin = T(2) * Prec<T>::fmin / Prec<T>::eps;
-  for (int i = 1; i <= n - 2; ++i) {
-    const int m = n - i;          // reflector length: rows i+1..n
-    T* col = &AA(i + 1, i);  // col[0] = alpha, col[1..m-1] = x
-    T lmax = T(0);
-    for (int r = 1 + tid; r < m; r += NT) lmax = fmax(lmax, fabs(col[r]));
-    const T big = block_max<NT>(lmax, red);
-    T tau_i = T(0);
-    if (big != T(0)) {
-      const bool safe = (big < Prec<T>::safe_hi && big > Prec<T>::safe_lo);
-      const T sc = safe ? T(1) : T(1) / big;
-      T ls = T(0);
-      for (int r = 1 + tid; r < m; r += NT) { const T t = col[r] * sc; ls = fma(t, t, ls); }
-      const T ssq = block_sum<NT>(ls, red);
-      T xnorm = safe ? sqrt(ssq) : big * sqrt(ssq);
-      T alpha = col[0];
-      T beta = -copysign(hypot(alpha, xnorm), alpha);
-      int kount = 0;
-      if (fabs(beta) < sfmin) {
-        // underflow guard (householder.jl:25-42): rescale x, alpha and beta
-        const T rsfmin = T(1) / sfmin;
-        T bb = beta;
-        do { ++kount; bb *= rsfmin; alpha *= rsfmin; } while (fabs(bb) < sfmin && kount < 20);
+// ---------------------------------------------------------------------------------
+// Hessenberg reduction and Q formation.
+//
+// 4*NC threads (NC >= n): the dot product of a column (or row) with the reflector keeps two
+// accumulators, over alternate elements, and each has its own thread: thread (c, par) of the
+// first 2*NC holds column c (left update) or row c (right update) of A, the last 2*NC hold the
+// rows of Z, whose update only needs the reflector and runs beside the left update of A.
+// Bound: FP64, the FP64 pipe (4n^3 FMAs: 4.1 of the 5 n^3 / 3 needed are full warps);
+// FP32, the latency of the seven barrier-separated steps per column.  With the matrix read
+// from the L2-resident output buffer, one column per thread (32 lines per warp load), this phase
+// took 31M cycles of an FP32 matrix of order 128 (57% of its time) and 17M of an FP64 one.
+struct HessCtl {
+  double tau, t, beta;  // of the current column (exact for T = float too)
+  int mode;             // 0: zero column, 1: reflector ready, 2: underflow guard needed
+};
+
+// max |.| over nonnegative values by their bit patterns: NaN compares largest, as block_max
+template <class T> __device__ __forceinline__ unsigned long long abs_bits(T v);
+template <> __device__ __forceinline__ unsigned long long abs_bits<double>(double v) {
+  return (unsigned long long)__double_as_longlong(fabs(v));
+}
+template <> __device__ __forceinline__ unsigned long long abs_bits<float>(float v) {
+  return (unsigned long long)__float_as_uint(fabsf(v));
+}
+template <class T> __device__ __forceinline__ T bits_abs(unsigned long long b);
+template <> __device__ __forceinline__ double bits_abs<double>(unsigned long long b) { return __longlong_as_double((long long)b); }
+template <> __device__ __forceinline__ float bits_abs<float>(unsigned long long b) { return __uint_as_float((unsigned)b); }
+
+template <class T, class W, int NC>
+__global__ void __launch_bounds__(4 * NC) k_hess_real(RealBatchT<T, W> bt, const int* __restrict__ order,
+                                                      const int* __restrict__ sched, int bin, int nmax, int cap) {
+  constexpr int NT = 4 * NC;
+  extern __shared__ double smem_raw[];
+  __shared__ T part[4][NC];
+  __shared__ T red[32];
+  __shared__ unsigned long long gmax[4];
+  __shared__ T gssq[4];
+  __shared__ HessCtl hc;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int start = sched[3 * bin], end = sched[3 * bin + 1];
+  const bool isz = tid >= 2 * NC;
+  const int c = tid % NC, par = (tid / NC) & 1;
+  for (int job = start + blockIdx.x; job < end; job += gridDim.x) {
+    const int b = order[job];
+    const int n = bt.ns[b];
+    if (n <= 0 || n > nmax) continue;  // k_schur_real reports it
+    T* __restrict__ Ag = bt.A + bt.offs[b];
+    T* __restrict__ Zg = bt.wantz ? bt.Z + bt.offs[b] : nullptr;
+    const int ld = n | 1;
+    T* A = (T*)smem_raw;
+    // Z in shared memory beside A where the launch left room for it
+    const bool zs = Zg && 2 * n * ld <= cap;
+    T* Z = zs ? A + n * ld : Zg;
+    const int ldz = zs ? ld : n;
+    __syncthreads();  // the previous matrix is out of shared memory
+    double amax = 0.0;
+    for (int idx = tid; idx < n * n; idx += NT) {
+      const int i = idx % n, j = idx / n;
+      const T a = Ag[idx];
+      A[i + j * ld] = a;
+      if (Zg) Z[i + j * ldz] = (i == j) ? T(1) : T(0);
+      const double aa = fabs((double)a);
+      amax = (aa > amax || aa != aa) ? aa : amax;
+    }
+    amax = (double)block_max<NT>((T)amax, red);
+    __syncthreads();
+    if (bt.scale) {
+      const double smlnum = sqrt((double)Prec<T>::fmin) / (double)Prec<T>::eps;
+      const double bignum = 1.0 / smlnum;
+      double cscale = 0.0;
+      if (amax > 0.0 && amax < smlnum) cscale = smlnum;
+      else if (amax > bignum) cscale = bignum;
+      if (cscale != 0.0) {
+        double mul[8];
+        const int nf = safescale_factors(amax, cscale, mul);
+        for (int f = 0; f < nf; ++f)
+          for (int idx = tid; idx < n * n; idx += NT) {
+            const int i = idx % n, j = idx / n;
+            A[i + j * ld] = (T)((double)A[i + j * ld] * mul[f]);
+          }
         __syncthreads();
-        for (int r = 1 + tid; r < m; r += NT) {
-          T t = col[r];
-          for (int q = 0; q < kount; ++q) t *= rsfmin;
-          col[r] = t;
-        }
-        __syncthreads();
-        T lm2 = T(0);
-        for (int r = 1 + tid; r < m; r += NT) lm2 = fmax(lm2, fabs(col[r]));
-        const T big2 = block_max<NT>(lm2, red);
-        const T sc2 = (big2 > T(0)) ? T(1) / big2 : T(0);
-        T ls2 = T(0);
-        for (int r = 1 + tid; r < m; r += NT) { const T t = col[r] * sc2; ls2 = fma(t, t, ls2); }
-        const T ssq2 = block_sum<NT>(ls2, red);
-        xnorm = big2 * sqrt(ssq2);
-        beta = -copysign(hypot(alpha, xnorm), alpha);
       }
-      tau_i = (beta - alpha) / beta;
-      const T t = T(1) / (alpha - beta);
-      for (int r = 1 + tid; r < m; r += NT) col[r] *= t;
-      for (int q = 0; q < kount; ++q) beta *= sfmin;
+    }
+    const T sfmin = T(2) * Prec<T>::fmin / Prec<T>::eps;
+    for (int i = 1; i <= n - 2; ++i) {
+      const int m = n - i;                     // reflector length: rows i+1..n
+      T* col = A + i + (size_t)(i - 1) * ld;   // col[0] = alpha, col[1..m-1] = x
+      // norm of x: elements 1+32w..32+32w are warp w's, summed by a tree, the warps' sums in order
+      if (warp < 4) {
+        const T x = (1 + tid < m) ? col[1 + tid] : T(0);
+        unsigned long long mb = abs_bits<T>(x);
+        T q = fma(x, x, T(0));
+        for (int o = 16; o > 0; o >>= 1) {
+          const unsigned long long w = __shfl_xor_sync(0xffffffffu, mb, o);
+          mb = w > mb ? w : mb;
+          q += __shfl_xor_sync(0xffffffffu, q, o);
+        }
+        if (lane == 0) { gmax[warp] = mb; gssq[warp] = q; }
+      }
+      __syncthreads();
+      if (warp == 0) {
+        unsigned long long mb = gmax[0];
+        for (int w = 1; w < 4; ++w) mb = gmax[w] > mb ? gmax[w] : mb;
+        const T big = bits_abs<T>(mb);
+        int mode = 0;
+        T tau = T(0), t = T(0), beta = T(0);
+        if (big != T(0)) {
+          mode = 2;
+          if (big < Prec<T>::safe_hi && big > Prec<T>::safe_lo) {
+            T ssq = gssq[0];
+            for (int w = 1; w < 4; ++w) ssq += gssq[w];
+            const T xnorm = sqrt(ssq);
+            const T alpha = col[0];
+            beta = -copysign(hypot(alpha, xnorm), alpha);
+            if (!(fabs(beta) < sfmin)) {
+              mode = 1;
+              tau = (beta - alpha) / beta;
+              t = T(1) / (alpha - beta);
+            }
+          }
+        }
+        if (lane == 0) { hc.mode = mode; hc.tau = (double)tau; hc.t = (double)t; hc.beta = (double)beta; }
+      }
+      __syncthreads();
+      const int mode = hc.mode;
+      if (mode == 0) continue;
+      T tau = (T)hc.tau, t = (T)hc.t, beta = (T)hc.beta;
+      if (mode == 2) {
+        // entries outside the range where squaring is safe, or the underflow guard
+        // (householder.jl:25-42): rescale x, alpha and beta
+        T big = T(0);
+        for (int w = 0; w < 4; ++w) { const T v = bits_abs<T>(gmax[w]); big = (v > big || v != v) ? v : big; }
+        const bool safe = (big < Prec<T>::safe_hi && big > Prec<T>::safe_lo);
+        const T sc = safe ? T(1) : T(1) / big;
+        T ls = T(0);
+        for (int r = 1 + tid; r < m; r += NT) { const T v = col[r] * sc; ls = fma(v, v, ls); }
+        const T ssq = block_sum<NT>(ls, red);
+        T xnorm = safe ? sqrt(ssq) : big * sqrt(ssq);
+        T alpha = col[0];
+        beta = -copysign(hypot(alpha, xnorm), alpha);
+        int kount = 0;
+        if (fabs(beta) < sfmin) {
+          const T rsfmin = T(1) / sfmin;
+          T bb = beta;
+          do { ++kount; bb *= rsfmin; alpha *= rsfmin; } while (fabs(bb) < sfmin && kount < 20);
+          __syncthreads();
+          for (int r = 1 + tid; r < m; r += NT) {
+            T v = col[r];
+            for (int q = 0; q < kount; ++q) v *= rsfmin;
+            col[r] = v;
+          }
+          __syncthreads();
+          T lm2 = T(0);
+          for (int r = 1 + tid; r < m; r += NT) lm2 = fmax(lm2, fabs(col[r]));
+          const T big2 = block_max<NT>(lm2, red);
+          const T sc2 = (big2 > T(0)) ? T(1) / big2 : T(0);
+          T ls2 = T(0);
+          for (int r = 1 + tid; r < m; r += NT) { const T v = col[r] * sc2; ls2 = fma(v, v, ls2); }
+          const T ssq2 = block_sum<NT>(ls2, red);
+          xnorm = big2 * sqrt(ssq2);
+          beta = -copysign(hypot(alpha, xnorm), alpha);
+        }
+        tau = (beta - alpha) / beta;
+        t = T(1) / (alpha - beta);
+        for (int q = 0; q < kount; ++q) beta *= sfmin;
+      }
+      if (1 + tid < m) col[1 + tid] *= t;
       __syncthreads();
       if (tid == 0) col[0] = beta;
+      if (tau == T(0)) { __syncthreads(); continue; }
+      // lmul!(H', A[i+1:n, i+1:n]), a column of A per pair of threads, and rmul!(Z, H), a row
+      // of Z per pair: both are x[0], x[1..m-1] against 1, col[1..m-1]
+      {
+        T* x = nullptr;
+        int st = 1;
+        if (!isz) { if (c < m) x = A + i + (size_t)(i + c) * ld; }
+        else if (Zg && c < n) { x = Z + c + (size_t)i * ldz; st = ldz; }
+        T a = T(0);
+        if (x) {
+          if (par == 0) {
+            a = x[0];
+#pragma unroll 4
+            for (int r = 1; r < m; r += 2) a = fma(col[r], x[r * st], a);
+          } else {
+#pragma unroll 4
+            for (int r = 2; r < m; r += 2) a = fma(col[r], x[r * st], a);
+          }
+        }
+        part[tid / NC][c] = a;
+        __syncthreads();
+        if (x) {
+          const int g = isz ? 2 : 0;
+          const T va = (part[g][c] + part[g + 1][c]) * tau;
+          if (par == 0) {
+            x[0] -= va;
+#pragma unroll 4
+            for (int r = 1; r < m; r += 2) x[r * st] = fma(-va, col[r], x[r * st]);
+          } else {
+#pragma unroll 4
+            for (int r = 2; r < m; r += 2) x[r * st] = fma(-va, col[r], x[r * st]);
+          }
+        }
+      }
+      __syncthreads();
+      // rmul!(A[:, i+1:n], H): a row of A per pair of threads
+      {
+        T* x = (!isz && c < n) ? A + c + (size_t)i * ld : nullptr;
+        T a = T(0);
+        if (x) {
+          if (par == 0) {
+            a = x[0];
+#pragma unroll 4
+            for (int q = 1; q < m; q += 2) a = fma(x[q * ld], col[q], a);
+          } else {
+#pragma unroll 4
+            for (int q = 2; q < m; q += 2) a = fma(x[q * ld], col[q], a);
+          }
+          part[par][c] = a;
+        }
+        __syncthreads();
+        if (x) {
+          const T va = (part[0][c] + part[1][c]) * tau;
+          if (par == 0) {
+            x[0] -= va;
+#pragma unroll 4
+            for (int q = 1; q < m; q += 2) x[q * ld] = fma(-va, col[q], x[q * ld]);
+          } else {
+#pragma unroll 4
+            for (int q = 2; q < m; q += 2) x[q * ld] = fma(-va, col[q], x[q * ld]);
+          }
+        }
+      }
+      __syncthreads();
     }
-    if (tid == 0) tau[i - 1] = tau_i;
     __syncthreads();
-    if (tau_i == T(0)) continue;
-    // lmul!(H', A[i+1:n, i+1:n]): one column per thread
-    for (int j = i + 1 + tid; j <= n; j += NT) {
-      T* hj = &AA(i + 1, j);
-      T va0 = hj[0], va1 = T(0);
-      int r = 1;
-      for (; r + 1 < m; r += 2) { va0 = fma(col[r], hj[r], va0); va1 = fma(col[r + 1], hj[r + 1], va1); }
-      if (r < m) va0 = fma(col[r], hj[r], va0);
-      const T va = (va0 + va1) * tau_i;
-      hj[0] -= va;
-      for (r = 1; r < m; ++r) hj[r] = fma(-va, col[r], hj[r]);
+    for (int idx = tid; idx < n * n; idx += NT) {
+      const int i = idx % n, j = idx / n;
+      if (i <= j + 1) Ag[idx] = A[i + j * ld];
+      if (zs) Zg[idx] = Z[i + j * ld];
     }
-    __syncthreads();
-    // rmul!(A[:, i+1:n], H): one row per thread
-    for (int r = tid; r < n; r += NT) {
-      T* hr = &A[r + i * lda];  // row r+1, column i+1
-      T x0 = hr[0], x1 = T(0);
-      int q = 1;
-      for (; q + 1 < m; q += 2) { x0 = fma(hr[q * lda], col[q], x0); x1 = fma(hr[(q + 1) * lda], col[q + 1], x1); }
-      if (q < m) x0 = fma(hr[q * lda], col[q], x0);
-      const T x = (x0 + x1) * tau_i;
-      hr[0] -= x;
-      for (q = 1; q < m; ++q) hr[q * lda] = fma(-x, col[q], hr[q * lda]);
-    }
-    __syncthreads();
+    if (tid == 0) bt.wr[bt.woffs[b]] = (W)amax;  // for the unscaling; k_schur_real overwrites it
   }
 }
 
-// Apply reflector r (order 3) from the left to column j, rows k..k+2 of packed H.
+// ---------------------------------------------------------------------------------
+// Francis iteration.
+//
+// Warp specialisation: one warp (the chain warp) runs the serial part of the sweeps -- the
+// deflation scan, the shifts, the start row, and the bulge chase inside a window of at most
+// kWin rows around the diagonal -- and the other warps apply the reflectors it logged, a chunk of steps
+// at a time and one phase later, to the columns right of the window, the rows above it and
+// Z (the far work).  One CTA barrier per phase.  Every element sees the same operations in the
+// same order as in the step-by-step iteration: for an element right of the window the
+// left updates of a chunk come before its right updates of later chunks, and
+//   - the columns that enter the next window get this chunk's left updates from the chain warp
+//     itself at the start of the next phase (urgent columns), the rest from the far warps;
+//   - row ka-1 (just above the window) stays with the chain warp, so that the diagonal and
+//     both its neighbours are final when a sweep's last chunk is done, and the next sweep's scan,
+//     shifts and start row overlap the far work of that chunk;
+//   - the next sweep's first window must not reach the columns ka.. of that chunk above its
+//     rows: its first chunk is shortened, or the chain warp skips a phase.
+// The 2x2 blocks are standardised together at the end, a block per thread (GenericSchur.jl
+// standardises each as it deflates; the block, its eigenvalues and Z see the same operations,
+// entries above a block see its rotation after instead of before later sweeps' reflectors).
+//
+// Why: with one CTA barrier per chase step (the near block and the next reflector on one
+// warp, far updates on the others, the Z pass after each sweep), a step of an order-128 matrix took
+// 1040 cycles in FP32 and 3880 in FP64 plus 400 / 1020 for its part of the Z pass.
 template <class T>
-__device__ __forceinline__ void left3(T* H, int k, int j, const Refl<T>& r) {
-  T* h = &HH(k, j);
-  const T ss = fma(r.v3, h[2], fma(r.v2, h[1], h[0]));
-  h[0] = fma(-ss, r.t1, h[0]);
-  h[1] = fma(-ss, r.t2, h[1]);
-  h[2] = fma(-ss, r.t3, h[2]);
+struct Cmd {
+  int type;  // 0 nothing, 1 chunk, 2 done
+  int ka;    // first step
+  int n3;    // steps with a 3-element reflector
+  int last2; // then a 2-element one
+  int jfar;  // first column of the far left updates
+};
+
+constexpr int kWin = 28;    // most steps of a chunk (kWin + 3 columns, kWin + 3 rows in a warp's lanes)
+constexpr int kChunk = 16;  // steps of a chunk of a longer sweep
+constexpr int kMinChunk = 4;
+constexpr int kLogStep = 8; // log entries per step: t1, t2, t3, v2, v3 (16-byte aligned)
+constexpr int kLogElems = 2 * kLogStep * (kWin + 1);
+
+template <class T> __device__ __forceinline__ Refl<T> ld_refl(const T* l);
+template <> __device__ __forceinline__ Refl<float> ld_refl<float>(const float* l) {
+  const float4 a = *(const float4*)l;
+  return {a.x, a.y, a.z, a.w, l[4]};
 }
-// ... from the right to row i, columns k..k+2.
-template <class T>
-__device__ __forceinline__ void right3(T* H, int k, int i, const Refl<T>& r) {
-  T& h0 = HH(i, k);
-  T& h1 = HH(i, k + 1);
-  T& h2 = HH(i, k + 2);
-  const T ss = fma(r.v3, h2, fma(r.v2, h1, h0));
-  h0 = fma(-ss, r.t1, h0);
-  h1 = fma(-ss, r.t2, h1);
-  h2 = fma(-ss, r.t3, h2);
-}
-template <class T>
-__device__ __forceinline__ void left2(T* H, int k, int j, const Refl<T>& r) {
-  T* h = &HH(k, j);
-  const T ss = fma(r.v2, h[1], h[0]);
-  h[0] = fma(-ss, r.t1, h[0]);
-  h[1] = fma(-ss, r.t2, h[1]);
-}
-template <class T>
-__device__ __forceinline__ void right2(T* H, int k, int i, const Refl<T>& r) {
-  T& h0 = HH(i, k);
-  T& h1 = HH(i, k + 1);
-  const T ss = fma(r.v2, h1, h0);
-  h0 = fma(-ss, r.t1, h0);
-  h1 = fma(-ss, r.t2, h1);
+template <> __device__ __forceinline__ Refl<double> ld_refl<double>(const double* l) {
+  const double2 a = *(const double2*)l, b = *(const double2*)(l + 2);
+  return {a.x, a.y, b.x, b.y, l[4]};
 }
 
-// Reflector of chase step k (> mx) from column k-1, writing beta and the zeros
-// back into H (GenericSchur.jl:882-895); logged for the Z pass.
+// The phase barrier: the chain warp and the far warps meet it at different places of the code.
+template <int NT> __device__ __forceinline__ void phase_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); }
+
+// One 3-element reflector on (z0, z1, z2): returns the finished first element.
 template <class T>
-__device__ __forceinline__ void make_refl(T* H, int k, int iend, Refl<T>& out, T* lg) {
-  const int nr = min(3, iend - k + 1);
-  T a = HH(k, k - 1), x1 = HH(k + 1, k - 1), x2 = (nr == 3) ? HH(k + 2, k - 1) : T(0);
-  const T t1 = reflector_fast(a, x1, x2, nr);
-  HH(k, k - 1) = a;
-  HH(k + 1, k - 1) = T(0);
-  if (k < iend - 1) HH(k + 2, k - 1) = T(0);
-  out.t1 = t1; out.v2 = x1; out.v3 = x2; out.t2 = t1 * x1; out.t3 = t1 * x2;
-  T* l = lg + 5 * (k - 1);
-  l[0] = t1; l[1] = out.t2; l[2] = out.t3; l[3] = x1; l[4] = x2;
+__device__ __forceinline__ T slide3(const Refl<T>& r, T& z0, T& z1, T z2) {
+  const T ss = fma(r.v3, z2, fma(r.v2, z1, z0));
+  const T out = fma(-ss, r.t1, z0);
+  z0 = fma(-ss, r.t2, z1);
+  z1 = fma(-ss, r.t3, z2);
+  return out;
+}
+
+// The logged reflectors of a chunk applied to one line (a column of H below row ka, a row of
+// H or Z from column ka): element e+1 follows element e at distance inc, growing by d per step.
+template <class T>
+__device__ __forceinline__ void apply_line(T* p, int inc, int d, const T* lg, int n3, int last2) {
+  T* p1 = p + inc;
+  inc += d;
+  T* p2 = p1 + inc;
+  inc += d;
+  T z0 = *p, z1 = *p1;
+  int s = 0;
+  for (; s + 4 <= n3; s += 4, lg += 4 * kLogStep) {
+    T* q1 = p2 + inc;
+    T* q2 = q1 + inc + d;
+    T* q3 = q2 + inc + 2 * d;
+    const T y0 = *p2, y1 = *q1, y2 = *q2, y3 = *q3;
+    *p = slide3(ld_refl<T>(lg), z0, z1, y0);
+    *p1 = slide3(ld_refl<T>(lg + kLogStep), z0, z1, y1);
+    *p2 = slide3(ld_refl<T>(lg + 2 * kLogStep), z0, z1, y2);
+    *q1 = slide3(ld_refl<T>(lg + 3 * kLogStep), z0, z1, y3);
+    p = q2;
+    p1 = q3;
+    p2 = q3 + inc + 3 * d;
+    inc += 4 * d;
+  }
+  for (; s < n3; ++s, lg += kLogStep) {
+    const T y0 = *p2;
+    *p = slide3(ld_refl<T>(lg), z0, z1, y0);
+    p = p1;
+    p1 = p2;
+    p2 += inc;
+    inc += d;
+  }
+  if (last2) {
+    const Refl<T> r = ld_refl<T>(lg);
+    const T ss = fma(r.v2, z1, z0);
+    z0 = fma(-ss, r.t1, z0);
+    z1 = fma(-ss, r.t2, z1);
+  }
+  *p = z0;
+  *p1 = z1;
+}
+
+// Reflector from (a, x1, x2); in FP64 the pairs x1 t, x2 t and t1 v2, t1 v3 are one
+// instruction each on two lanes (an FP64 instruction costs the pipe the same for 1 or 32 lanes).
+__device__ __forceinline__ Refl<float> chain_refl(float& a, float x1, float x2, int nr, int) {
+  const float t1 = reflector_fast(a, x1, x2, nr);
+  return {t1, t1 * x1, t1 * x2, x1, x2};
+}
+__device__ __forceinline__ Refl<double> chain_refl(double& a, double x1, double x2, int nr, int) {
+  const double t1 = reflector_fast(a, x1, x2, nr);
+  return {t1, t1 * x1, t1 * x2, x1, x2};
+}
+
+// Chain warp: steps ka..ka+nst-1 inside the window (columns ..wl, rows ka-1..).  r: the reflector of
+// step ka on entry, of step ka+nst on return.
+template <class T>
+__device__ __forceinline__ void chase_chunk(T* H, int ka, int nst, int iend, int wl, Refl<T>& r, T* lg, int lane) {
+  const int j = ka + lane;
+  const bool colok = j <= wl;
+  T* hc = H + rpk(colok ? j : ka) - 1;  // hc[i] = H(i, j)
+  const int i = ka - 1 + lane;
+  const bool rowok = i >= 1 && i <= iend;
+  T* hr = H + i - 1;  // hr[rpk(c)] = H(i, c)
+  int c0 = rpk(ka);
+  T a0 = hc[ka], a1 = hc[ka + 1], a2 = hc[ka + 2];
+  for (int s = 0; s < nst; ++s) {
+    const int k = ka + s;
+    if (lane == 0) {
+      T* l = lg + kLogStep * s;
+      l[0] = r.t1; l[1] = r.t2; l[2] = r.t3; l[3] = r.v2; l[4] = r.v3;
+    }
+    if (k <= iend - 2) {
+      if (colok && j >= k) {
+        const T ss = fma(r.v3, a2, fma(r.v2, a1, a0));
+        hc[k] = fma(-ss, r.t1, a0);
+        hc[k + 1] = fma(-ss, r.t2, a1);
+        hc[k + 2] = fma(-ss, r.t3, a2);
+      }
+      __syncwarp();
+      T x = T(0);
+      if (rowok && i <= k + 3) {
+        T* h0 = hr + c0;
+        T* h1 = h0 + k + 3;
+        T* h2 = h1 + k + 4;
+        const T b0 = *h0, b1 = *h1, b2 = *h2;
+        const T ss = fma(r.v3, b2, fma(r.v2, b1, b0));
+        x = fma(-ss, r.t1, b0);
+        *h0 = x;
+        *h1 = fma(-ss, r.t2, b1);
+        *h2 = fma(-ss, r.t3, b2);
+      }
+      // column k, rows k+1..k+3: the next reflector
+      T a = __shfl_sync(0xffffffffu, x, s + 2);
+      const T x1 = __shfl_sync(0xffffffffu, x, s + 3);
+      const T x2 = __shfl_sync(0xffffffffu, x, s + 4);
+      __syncwarp();
+      a0 = hc[k + 1]; a1 = hc[k + 2]; a2 = hc[k + 3];
+      r = chain_refl(a, x1, x2, min(3, iend - k), lane);
+      if (lane == 0) {
+        T* h = H + c0 + k;  // H(k+1, k)
+        h[0] = a;
+        h[1] = T(0);
+        if (k + 1 < iend - 1) h[2] = T(0);
+      }
+      c0 += k + 3;
+    } else {
+      // 2-element reflector at k = iend-1
+      if (colok && j >= k) {
+        const T ss = fma(r.v2, a1, a0);
+        hc[k] = fma(-ss, r.t1, a0);
+        hc[k + 1] = fma(-ss, r.t2, a1);
+      }
+      __syncwarp();
+      if (rowok) {
+        T* h0 = hr + c0;
+        T* h1 = h0 + k + 3;
+        const T b0 = *h0, b1 = *h1;
+        const T ss = fma(r.v2, b1, b0);
+        *h0 = fma(-ss, r.t1, b0);
+        *h1 = fma(-ss, r.t2, b1);
+      }
+    }
+  }
+  __syncwarp();
 }
 
 // nmax: the largest order the launch sized shared memory for.  Orders come from device
 // memory (GS_DEVICE calls are not checked on the host), so an order outside [0, nmax]
 // gets ST_BADARG before anything is read or written.
-template <class T, class W, int NT, bool HSMEM>
-__device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem, Ctl<T>& c) {
+template <class T, class W, int NT>
+__device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem, int cw) {
+  __shared__ Cmd<T> cmd[2];
+  __shared__ int s_status, s_iend, s_npair;
+  __shared__ int pairs[kSmallMax / 2];
+  __shared__ T gcs[kSmallMax / 2], gsn[kSmallMax / 2];
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const int n = bt.ns[b];
@@ -198,29 +480,13 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
     return;
   }
   T* __restrict__ Ag = bt.A + bt.offs[b];
-  T* __restrict__ Zg = bt.wantz ? bt.Z + bt.offs[b] : nullptr;
+  T* Zg = bt.wantz ? bt.Z + bt.offs[b] : nullptr;
   W* __restrict__ wr = bt.wr + bt.woffs[b];
   W* __restrict__ wi = bt.wi + bt.woffs[b];
-  const int lda = HSMEM ? (n | 1) : n;
-  const int hsz = HSMEM ? n * lda : rpk(n + 1);  // full (Hessenberg phase) or packed (QR phase)
-  const int hreg = max(hsz, rpk(n + 1));
-  T* H = smem;                      // packed H of the QR phase (and the full matrix before it, HSMEM)
-  T* tau = H + hreg;                // n-1 reflector scalars
-  T* lg = tau + n;                  // 5 per chase step: t1, t2, t3, v2, v3
-  T* red = lg + 5 * n;              // reduction scratch (32)
-  T* A = HSMEM ? smem : Ag;         // where the Hessenberg reduction runs
-
-  // ---- 1. load and scale --------------------------------------------------
-  double amax = 0.0;
-  for (int idx = tid; idx < n * n; idx += NT) {
-    const int i = idx % n, j = idx / n;
-    const T a = Ag[idx];
-    if (HSMEM) A[i + j * lda] = a;
-    const double aa = fabs((double)a);
-    amax = (aa > amax || aa != aa) ? aa : amax;
-  }
-  amax = (double)block_max<NT>((T)amax, red);
-  __syncthreads();
+  T* logs = smem;
+  T* H = smem + kLogElems;  // packed H
+  // the scale that k_hess_real applied
+  const double amax = (double)wr[0];
   const double smlnum = sqrt((double)Prec<T>::fmin) / (double)Prec<T>::eps;
   const double bignum = 1.0 / smlnum;
   bool scaled = false;
@@ -229,277 +495,273 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
     if (amax > 0.0 && amax < smlnum) { scaled = true; cscale = smlnum; }
     else if (amax > bignum) { scaled = true; cscale = bignum; }
   }
-  if (scaled) {
-    double mul[8];
-    const int nf = safescale_factors(amax, cscale, mul);
-    for (int f = 0; f < nf; ++f)
-      for (int idx = tid; idx < n * n; idx += NT) {
-        const int i = idx % n, j = idx / n;
-        A[i + j * lda] = (T)((double)A[i + j * lda] * mul[f]);
-      }
-    __syncthreads();
-  }
-
-  // ---- 2. Hessenberg reduction ------------------------------------------------
-  hessenberg_real<T, NT>(n, A, lda, tau, red);
-
-  // ---- 3. Q formation into Z (row-owner threads, no barriers) ------------------
-  if (Zg) {
-    for (int r = tid; r < n; r += NT)
-      for (int j = 0; j < n; ++j) Zg[r + (long long)j * n] = (r == j) ? T(1) : T(0);
-    for (int i = 1; i <= n - 2; ++i) {
-      const T t = tau[i - 1];
-      if (t == T(0)) continue;
-      const int m = n - i;
-      const T* col = &AA(i + 1, i);
-      for (int r = tid; r < n; r += NT) {
-        T* zr = Zg + r + (long long)i * n;  // Z[r+1, i+1]
-        T s0 = zr[0], s1 = T(0);
-        int q = 1;
-        for (; q + 1 < m; q += 2) { s0 = fma(zr[q * n], col[q], s0); s1 = fma(zr[(q + 1) * n], col[q + 1], s1); }
-        if (q < m) s0 = fma(zr[q * n], col[q], s0);
-        const T s = (s0 + s1) * t;
-        zr[0] -= s;
-        for (q = 1; q < m; ++q) zr[q * n] = fma(-s, col[q], zr[q * n]);
-      }
-    }
-  }
-  __syncthreads();
-
-  // ---- 4. pack H (Hessenberg part + bulge rows) into shared memory ----------------
-  if (HSMEM) {
-    // the full matrix occupies the same shared memory: route through the output buffer
-    for (int idx = tid; idx < n * n; idx += NT) {
-      const int i = idx % n, j = idx / n;
-      Ag[idx] = A[i + j * lda];
-    }
-    __syncthreads();
-  }
-  for (int j = 1; j <= n; ++j)
-    for (int i = 1 + tid; i <= j + 3; i += NT)
+  for (int j = 1 + warp; j <= n; j += NT / 32)
+    for (int i = 1 + lane; i <= j + 3; i += 32)
       HH(i, j) = (i <= min(j + 1, n)) ? Ag[(i - 1) + (long long)(j - 1) * n] : T(0);
   __syncthreads();
 
-  // ---- 5. Francis double-shift QR on packed H ------------------------------------------
   const T eps = Prec<T>::eps;
   const T smallnum = Prec<T>::fmin * ((T)n / eps);
-  const long long maxiter = bt.maxiter_abs > 0 ? bt.maxiter_abs : (long long)bt.maxiter_mult * n;
-  long long iter = 0;
-  int status = ST_OK;
-  int iend = n;
-  while (iend >= 1) {
-    int istart = 1;
-    int iterqr = 0;
-    bool deflate = false;
-    for (;;) {
-      ++iter;
-      if (iter > maxiter) { status = ST_UNCONVERGED; break; }
-      // deflation scan (GenericSchur.jl:563-600): largest k with a negligible H[k,k-1]
-      if (tid == 0) c.split = 0;
-      __syncthreads();
-      for (int k = istart + 1 + tid; k <= iend; k += NT) {
-        bool split = false;
-        const T hk = HH(k, k - 1);
-        if (fabs(hk) < smallnum) {
-          split = true;
-        } else {
-          const T hkk = HH(k, k), hkm1 = HH(k - 1, k - 1);
-          T t = fabs(hkm1) + fabs(hkk);
-          if (t == T(0)) {
-            if (k > 2) t += fabs(HH(k - 1, k - 2));
-            if (k + 1 <= n) t += fabs(HH(k + 1, k));
-          }
-          const T ahkkm1 = fabs(hk);
-          if (ahkkm1 <= t * eps) {
-            const T ahkm1k = fabs(HH(k - 1, k));
-            const T ab = fmax(ahkkm1, ahkm1k), ba = fmin(ahkkm1, ahkm1k);
-            const T aa = fmax(fabs(hkk), fabs(hkm1 - hkk)), bb = fmin(fabs(hkk), fabs(hkm1 - hkk));
-            const T s = aa + bb;
-            if (ba * (ab / s) <= fmax(smallnum, eps * (bb * (aa / s)))) split = true;
-          }
-        }
-        if (split) atomicMax(&c.split, k);
-      }
-      __syncthreads();
-      istart = (c.split > 0) ? c.split : 1;
-      if (istart > 1 && tid == 0) HH(istart, istart - 1) = T(0);
-      if (istart >= iend - 1) { deflate = true; break; }
-      ++iterqr;
-      __syncthreads();
-      // shifts (GenericSchur.jl:614-665)
-      if (tid == 0) {
-        T h11, h12, h21, h22;
-        if (iterqr == 10) {
-          const T s = fabs(HH(istart + 1, istart)) + fabs(HH(istart + 2, istart + 1));
-          h11 = T(0.75) * s + HH(istart, istart); h12 = T(-0.4375) * s; h21 = s; h22 = h11;
-        } else if (iterqr == 20) {
-          const T s = fabs(HH(iend, iend - 1)) + fabs(HH(iend - 1, iend - 2));
-          h11 = T(0.75) * s + HH(iend, iend); h12 = T(-0.4375) * s; h21 = s; h22 = h11;
-        } else {
-          h11 = HH(iend - 1, iend - 1); h21 = HH(iend, iend - 1);
-          h12 = HH(iend - 1, iend); h22 = HH(iend, iend);
-        }
-        const T s = fabs(h11) + fabs(h12) + fabs(h21) + fabs(h22);
-        T r1r, r2r, r1i, r2i;
-        if (s == T(0)) {
-          r1r = r2r = r1i = r2i = T(0);
-        } else {
-          h11 /= s; h12 /= s; h21 /= s; h22 /= s;
-          const T tr = (h11 + h22) / T(2);
-          const T d = (h11 - tr) * (h22 - tr) - h12 * h21;
-          const T rtd = sqrt(fabs(d));
-          if (d >= T(0)) {
-            r1r = tr * s; r2r = r1r; r1i = rtd * s; r2i = -r1i;
-          } else {
-            r1r = tr + rtd; r2r = tr - rtd;
-            if (fabs(r1r - h22) <= fabs(r2r - h22)) { r1r *= s; r2r = r1r; }
-            else { r2r *= s; r1r = r2r; }
-            r1i = r2i = T(0);
-          }
-        }
-        c.s[0] = r1r; c.s[1] = r1i; c.s[2] = r2r; c.s[3] = r2i;
-        c.mx = istart;
-      }
-      __syncthreads();
-      // start row (GenericSchur.jl:850-872): largest m with two small subdiagonals
-      {
-        const T r1r = c.s[0], r1i = c.s[1], r2r = c.s[2], r2i = c.s[3];
-        for (int m = istart + 1 + tid; m <= iend - 2; m += NT) {
-          T h21s = HH(m + 1, m);
-          T s = fabs(HH(m, m) - r2r) + fabs(r2i) + fabs(h21s);
-          h21s /= s;
-          T v0 = h21s * HH(m, m + 1) + (HH(m, m) - r1r) * ((HH(m, m) - r2r) / s) - r1i * (r2i / s);
-          T v1 = h21s * (HH(m, m) + HH(m + 1, m + 1) - r1r - r2r);
-          T v2 = h21s * HH(m + 2, m + 1);
-          s = fabs(v0) + fabs(v1) + fabs(v2);
-          v0 /= s; v1 /= s; v2 /= s;
-          if (fabs(HH(m, m - 1)) * (fabs(v1) + fabs(v2)) <=
-              eps * fabs(v0) * (fabs(HH(m - 1, m - 1)) + fabs(HH(m, m)) + fabs(HH(m + 1, m + 1))))
-            atomicMax(&c.mx, m);
-        }
-      }
-      __syncthreads();
-      const int mx = c.mx;
-      // reflector of the first step from the start vector
-      if (tid == 0) {
-        const T r1r = c.s[0], r1i = c.s[1], r2r = c.s[2], r2i = c.s[3];
-        const int m = mx;
-        T h21s = HH(m + 1, m);
-        T s = fabs(HH(m, m) - r2r) + fabs(r2i) + fabs(h21s);
-        h21s /= s;
-        T v0 = h21s * HH(m, m + 1) + (HH(m, m) - r1r) * ((HH(m, m) - r2r) / s) - r1i * (r2i / s);
-        T v1 = h21s * (HH(m, m) + HH(m + 1, m + 1) - r1r - r2r);
-        T v2 = h21s * HH(m + 2, m + 1);
-        s = fabs(v0) + fabs(v1) + fabs(v2);
-        v0 /= s; v1 /= s; v2 /= s;
-        const int nr = min(3, iend - mx + 1);
-        const T t1 = reflector_fast(v0, v1, v2, nr);
-        if (mx > istart) HH(mx, mx - 1) *= (T(1) - t1);
-        Refl<T>& r = c.r[0];
-        r.t1 = t1; r.v2 = v1; r.v3 = v2; r.t2 = t1 * v1; r.t3 = t1 * v2;
-        T* l = lg + 5 * (mx - 1);
-        l[0] = t1; l[1] = r.t2; l[2] = r.t3; l[3] = v1; l[4] = v2;
-      }
-      __syncthreads();
-      // bulge chase (GenericSchur.jl:877-949), steps with a 3-element reflector
-      int cur = 0;
-      for (int k = mx; k <= iend - 2; ++k) {
-        const Refl<T> r = c.r[cur];
-        if (warp == 0) {
-          // near block: left on columns k..k+2, then right on rows k..min(k+3, iend)
-          if (lane < 3) left3(H, k, k + lane, r);
-          __syncwarp();
-          if (lane < 4 && k + lane <= iend) right3(H, k, k + lane, r);
-          __syncwarp();
-          if (lane == 0) make_refl(H, k + 1, iend, c.r[cur ^ 1], lg);
-        } else {
-          // one task list: far columns k+3..n (left), then far rows 1..k-1 (right)
-          const int ft = tid - 32;
-          constexpr int NF = NT - 32;
-          const int nl = n - k - 2;
-          const int ntask = nl + k - 1;
-          for (int t = ft; t < ntask; t += NF) {
-            if (t < nl) left3(H, k, k + 3 + t, r);
-            else right3(H, k, t - nl + 1, r);
-          }
-        }
-        __syncthreads();
-        cur ^= 1;
-      }
-      // last step: 2-element reflector at k = iend-1 (left on columns k..n, right on rows 1..iend)
-      {
-        const int k = iend - 1;
-        const Refl<T> r = c.r[cur];
-        for (int j = k + tid; j <= n; j += NT) left2(H, k, j, r);
-        __syncthreads();
-        for (int i = 1 + tid; i <= iend; i += NT) right2(H, k, i, r);
-      }
-      __syncthreads();
-      // apply the sweep's reflectors to the Z rows each thread owns
-      if (Zg) {
-        for (int r = tid; r < n; r += NT) {
-          T* zr = Zg + r;
-          T z0 = zr[(long long)(mx - 1) * n], z1 = zr[(long long)mx * n];
-          for (int k = mx; k <= iend - 1; ++k) {
-            const T* l = lg + 5 * (k - 1);
-            if (k <= iend - 2) {
-              const T z2 = zr[(long long)(k + 1) * n];
-              const T ss = fma(l[4], z2, fma(l[3], z1, z0));
-              zr[(long long)(k - 1) * n] = fma(-ss, l[0], z0);
-              z0 = fma(-ss, l[1], z1);
-              z1 = fma(-ss, l[2], z2);
+  if (warp == cw) {
+    // ---- chain warp (all its variables are uniform over the lanes) ----
+    const long long maxiter = bt.maxiter_abs > 0 ? bt.maxiter_abs : (long long)bt.maxiter_mult * n;
+    long long iter = 0;
+    int status = ST_OK, iend = n, istart = 1, iterqr = 0, npair = 0;
+    int state = 0;             // 0: between sweeps, 1: first chunk of a sweep is next, 2: inside a sweep
+    int kn = 0;                // next step
+    int pka = 0, pn3 = 0, pwl = 0;  // previous chunk of this sweep
+    int fka = 0;               // ka of the sweep's last chunk while the far warps apply it (0: none)
+    Refl<T> r{};
+    for (int ph = 0;; ++ph) {
+      Cmd<T>& cm = cmd[ph & 1];
+      T* lg = logs + (ph & 1) * (kLogElems / 2);
+      bool done = false;
+      while (state == 0) {
+        if (iend < 1) { done = true; break; }
+        if (++iter > maxiter) { status = ST_UNCONVERGED; done = true; break; }
+        // deflation scan (GenericSchur.jl:563-600): largest k with a negligible H[k,k-1]
+        int found = 0;
+        for (int top = iend; top >= istart + 1; top -= 32) {
+          const int k = top - lane;
+          bool split = false;
+          if (k >= istart + 1) {
+            const T hk = HH(k, k - 1);
+            if (fabs(hk) < smallnum) {
+              split = true;
             } else {
-              const T ss = fma(l[3], z1, z0);
-              zr[(long long)(k - 1) * n] = fma(-ss, l[0], z0);
-              zr[(long long)k * n] = fma(-ss, l[1], z1);
+              const T hkk = HH(k, k), hkm1 = HH(k - 1, k - 1);
+              T t = fabs(hkm1) + fabs(hkk);
+              if (t == T(0)) {
+                if (k > 2) t += fabs(HH(k - 1, k - 2));
+                if (k + 1 <= n) t += fabs(HH(k + 1, k));
+              }
+              const T ahkkm1 = fabs(hk);
+              if (ahkkm1 <= t * eps) {
+                const T ahkm1k = fabs(HH(k - 1, k));
+                const T ab = fmax(ahkkm1, ahkm1k), ba = fmin(ahkkm1, ahkm1k);
+                const T aa = fmax(fabs(hkk), fabs(hkm1 - hkk)), bb = fmin(fabs(hkk), fabs(hkm1 - hkk));
+                const T s = aa + bb;
+                if (ba * (ab / s) <= fmax(smallnum, eps * (bb * (aa / s)))) split = true;
+              }
+            }
+          }
+          const unsigned bal = __ballot_sync(0xffffffffu, split);
+          if (bal) { found = top - (__ffs(bal) - 1); break; }
+        }
+        istart = found > 0 ? found : 1;
+        if (istart > 1 && lane == 0) HH(istart, istart - 1) = T(0);
+        __syncwarp();
+        if (istart >= iend - 1) {
+          if (lane == 0) {
+            if (istart >= iend) {
+              wr[iend - 1] = (W)HH(iend, iend);
+              wi[iend - 1] = W(0);
+            } else {
+              pairs[npair] = iend - 1;
+              if (iend > 2) HH(iend - 1, iend - 2) = T(0);
+            }
+          }
+          if (istart < iend) ++npair;
+          __syncwarp();
+          iend = istart - 1;
+          istart = 1;
+          iterqr = 0;
+          continue;
+        }
+        ++iterqr;
+        // shifts (GenericSchur.jl:614-665); the four quotients are one division over four lanes
+        T r1r, r1i, r2r, r2i;
+        {
+          T h11, h12, h21, h22;
+          if (iterqr == 10) {
+            const T s = fabs(HH(istart + 1, istart)) + fabs(HH(istart + 2, istart + 1));
+            h11 = T(0.75) * s + HH(istart, istart); h12 = T(-0.4375) * s; h21 = s; h22 = h11;
+          } else if (iterqr == 20) {
+            const T s = fabs(HH(iend, iend - 1)) + fabs(HH(iend - 1, iend - 2));
+            h11 = T(0.75) * s + HH(iend, iend); h12 = T(-0.4375) * s; h21 = s; h22 = h11;
+          } else {
+            h11 = HH(iend - 1, iend - 1); h21 = HH(iend, iend - 1);
+            h12 = HH(iend - 1, iend); h22 = HH(iend, iend);
+          }
+          const T s = fabs(h11) + fabs(h12) + fabs(h21) + fabs(h22);
+          if (s == T(0)) {
+            r1r = r2r = r1i = r2i = T(0);
+          } else {
+            T hq = (lane & 2) ? ((lane & 1) ? h22 : h21) : ((lane & 1) ? h12 : h11);
+            hq /= s;
+            h11 = __shfl_sync(0xffffffffu, hq, 0); h12 = __shfl_sync(0xffffffffu, hq, 1);
+            h21 = __shfl_sync(0xffffffffu, hq, 2); h22 = __shfl_sync(0xffffffffu, hq, 3);
+            const T tr = (h11 + h22) / T(2);
+            const T d = (h11 - tr) * (h22 - tr) - h12 * h21;
+            const T rtd = sqrt(fabs(d));
+            if (d >= T(0)) {
+              r1r = tr * s; r2r = r1r; r1i = rtd * s; r2i = -r1i;
+            } else {
+              r1r = tr + rtd; r2r = tr - rtd;
+              if (fabs(r1r - h22) <= fabs(r2r - h22)) { r1r *= s; r2r = r1r; }
+              else { r2r *= s; r1r = r2r; }
+              r1i = r2i = T(0);
             }
           }
         }
-      }
-    }
-    if (status != ST_OK) break;
-    __syncthreads();
-    if (deflate && istart >= iend) {
-      if (tid == 0) { wr[iend - 1] = (W)HH(iend, iend); wi[iend - 1] = W(0); }
-    } else if (deflate && istart + 1 == iend) {
-      const int p = iend - 1, q = iend;
-      if (tid == 0) {
-        double a = HH(p, p), bq = HH(p, q), cc = HH(q, p), d = HH(q, q), cs, sn, w1r, w1i, w2r, w2i;
-        gs2x2(a, bq, cc, d, cs, sn, w1r, w1i, w2r, w2i);
-        wr[q - 1] = (W)w2r; wi[q - 1] = (W)w2i; wr[p - 1] = (W)w1r; wi[p - 1] = (W)w1i;
-        c.g[0] = (T)cs; c.g[1] = (T)sn;
-        c.blk[0] = (T)a; c.blk[1] = (T)bq; c.blk[2] = (T)cc; c.blk[3] = (T)d;
-      }
-      __syncthreads();
-      const T cs = c.g[0], sn = c.g[1];
-      for (int j = q + 1 + tid; j <= n; j += NT) {  // lmul!(G, HH[:, istart:n]) beyond the block
-        const T a1 = HH(p, j), a2 = HH(q, j);
-        HH(p, j) = cs * a1 + sn * a2;
-        HH(q, j) = -sn * a1 + cs * a2;
-      }
-      for (int r = 1 + tid; r <= p - 1; r += NT) {  // rmul!(HH[1:iend, :], G') above the block
-        const T a1 = HH(r, p), a2 = HH(r, q);
-        HH(r, p) = cs * a1 + sn * a2;
-        HH(r, q) = -sn * a1 + cs * a2;
-      }
-      if (Zg)
-        for (int r = tid; r < n; r += NT) {
-          T* zp = Zg + r + (long long)(p - 1) * n;
-          const T a1 = zp[0], a2 = zp[n];
-          zp[0] = cs * a1 + sn * a2;
-          zp[n] = -sn * a1 + cs * a2;
+        // start row (GenericSchur.jl:850-872): largest m with two small subdiagonals, else
+        // istart; the start vector comes with it
+        int mx = istart;
+        T v0 = T(0), v1 = T(0), v2 = T(0);
+        for (int top = iend - 2; top >= istart; top -= 32) {
+          const int m = top - lane;
+          bool hit = false;
+          if (m >= istart) {
+            T h21s = HH(m + 1, m);
+            T s = fabs(HH(m, m) - r2r) + fabs(r2i) + fabs(h21s);
+            h21s /= s;
+            v0 = h21s * HH(m, m + 1) + (HH(m, m) - r1r) * ((HH(m, m) - r2r) / s) - r1i * (r2i / s);
+            v1 = h21s * (HH(m, m) + HH(m + 1, m + 1) - r1r - r2r);
+            v2 = h21s * HH(m + 2, m + 1);
+            s = fabs(v0) + fabs(v1) + fabs(v2);
+            v0 /= s; v1 /= s; v2 /= s;
+            hit = m == istart ||
+                  fabs(HH(m, m - 1)) * (fabs(v1) + fabs(v2)) <=
+                      eps * fabs(v0) * (fabs(HH(m - 1, m - 1)) + fabs(HH(m, m)) + fabs(HH(m + 1, m + 1)));
+          }
+          const unsigned bal = __ballot_sync(0xffffffffu, hit);
+          if (bal) {
+            const int q = __ffs(bal) - 1;
+            mx = top - q;
+            v0 = __shfl_sync(0xffffffffu, v0, q);
+            v1 = __shfl_sync(0xffffffffu, v1, q);
+            v2 = __shfl_sync(0xffffffffu, v2, q);
+            break;
+          }
         }
-      if (tid == 0) {
-        HH(p, p) = c.blk[0]; HH(p, q) = c.blk[1]; HH(q, p) = c.blk[2]; HH(q, q) = c.blk[3];
-        if (iend > 2) HH(iend - 1, iend - 2) = T(0);
+        // reflector of the first step from the start vector
+        const T t1 = reflector_fast(v0, v1, v2, min(3, iend - mx + 1));
+        if (mx > istart && lane == 0) HH(mx, mx - 1) *= (T(1) - t1);
+        r.t1 = t1; r.v2 = v1; r.v3 = v2; r.t2 = t1 * v1; r.t3 = t1 * v2;
+        __syncwarp();
+        kn = mx;
+        state = 1;
       }
+      int type = done ? 2 : 0;
+      if (!done) {
+        // the next chunk: steps kn..kn+nst-1
+        int nst = iend - kn;
+        if (nst > kWin) nst = kChunk;
+        if (state == 1 && fka > 0 && kn < fka && min(kn + nst + 2, iend) >= fka) {
+          // the far warps are still in columns fka.. above row fka-1
+          nst = min(nst, fka - kn - 3);
+          if (nst < kMinChunk) nst = 0;
+        }
+        if (nst > 0) {
+          const int kb = kn + nst - 1;
+          const int wl = min(kb + 3, iend);
+          if (state == 2) {
+            // urgent columns: the previous chunk's left updates on the columns entering the window
+            const T* pl = logs + ((ph & 1) ^ 1) * (kLogElems / 2);
+            const int j = pwl + 1 + lane;
+            if (j <= wl) apply_line(&HH(pka, j), 1, 0, pl, pn3, 0);
+            __syncwarp();
+          }
+          chase_chunk(H, kn, nst, iend, wl, r, lg, lane);
+          const bool last = kb == iend - 1;
+          int jfar = wl + 1;
+          if (!last) {
+            int nn = iend - kb - 1;
+            if (nn > kWin) nn = kChunk;
+            jfar = min(kb + nn + 3, iend) + 1;  // beyond the next chunk's window
+          }
+          if (lane == 0) {
+            cm.ka = kn;
+            cm.n3 = last ? nst - 1 : nst;
+            cm.last2 = last;
+            cm.jfar = jfar;
+          }
+          type = 1;
+          pka = kn; pn3 = nst; pwl = wl;
+          kn = kb + 1;
+          fka = last ? pka : 0;
+          state = last ? 0 : 2;
+        } else {
+          fka = 0;  // this phase's barrier ends the far work
+        }
+      }
+      if (lane == 0) cm.type = type;
+      phase_barrier<NT>();
+      if (done) break;
     }
-    iend = istart - 1;
-    __syncthreads();
+    if (lane == 0) { s_status = status; s_iend = iend; s_npair = npair; }
+  } else {
+    // ---- far warps ----
+    const int ft = tid - (warp > cw ? 32 : 0);
+    for (int ph = 0;; ++ph) {
+      if (ph > 0 && cmd[(ph - 1) & 1].type == 1) {
+        const Cmd<T> cm = cmd[(ph - 1) & 1];
+        const T* lg = logs + ((ph - 1) & 1) * (kLogElems / 2);
+        const int ka = cm.ka;
+        const int nl = n - cm.jfar + 1, nr = max(ka - 2, 0), nz = Zg ? n : 0;
+        for (int t = ft; t < nl + nr + nz; t += NT - 32) {
+          T* p;
+          int inc, d = 0;
+          if (t < nl) {
+            p = &HH(ka, cm.jfar + t);
+            inc = 1;
+          } else if (t < nl + nr) {
+            p = &HH(t - nl + 1, ka);
+            inc = ka + 3;
+            d = 1;
+          } else {
+            p = Zg + (t - nl - nr) + (long long)(ka - 1) * n;
+            inc = n;
+          }
+          apply_line(p, inc, d, lg, cm.n3, cm.last2);
+        }
+      }
+      phase_barrier<NT>();
+      if (cmd[ph & 1].type == 2) break;
+    }
+  }
+  __syncthreads();
+  const int status = s_status, npair = s_npair;
+
+  // ---- standardise the 2x2 blocks (GenericSchur.jl:667-690) ----
+  for (int q = tid; q < npair; q += NT) {
+    const int p = pairs[q];
+    double a = HH(p, p), bq = HH(p, p + 1), cc = HH(p + 1, p), d = HH(p + 1, p + 1), cs, sn, w1r, w1i, w2r, w2i;
+    gs2x2(a, bq, cc, d, cs, sn, w1r, w1i, w2r, w2i);
+    wr[p] = (W)w2r; wi[p] = (W)w2i; wr[p - 1] = (W)w1r; wi[p - 1] = (W)w1i;
+    gcs[q] = (T)cs; gsn[q] = (T)sn;
+    HH(p, p) = (T)a; HH(p, p + 1) = (T)bq; HH(p + 1, p) = (T)cc; HH(p + 1, p + 1) = (T)d;
+  }
+  __syncthreads();
+  for (int q = warp; q < npair; q += NT / 32) {  // rmul!(HH[1:p-1, :], G') and Z
+    const int p = pairs[q];
+    const T cs = gcs[q], sn = gsn[q];
+    for (int i = 1 + lane; i <= p - 1; i += 32) {
+      const T a1 = HH(i, p), a2 = HH(i, p + 1);
+      HH(i, p) = cs * a1 + sn * a2;
+      HH(i, p + 1) = -sn * a1 + cs * a2;
+    }
+    if (Zg)
+      for (int i = lane; i < n; i += 32) {
+        T* zp = Zg + i + (long long)(p - 1) * n;
+        const T a1 = zp[0], a2 = zp[n];
+        zp[0] = cs * a1 + sn * a2;
+        zp[n] = -sn * a1 + cs * a2;
+      }
+  }
+  __syncthreads();
+  for (int q = warp; q < npair; q += NT / 32) {  // lmul!(G, HH[:, p+2:n])
+    const int p = pairs[q];
+    const T cs = gcs[q], sn = gsn[q];
+    for (int j = p + 2 + lane; j <= n; j += 32) {
+      const T a1 = HH(p, j), a2 = HH(p + 1, j);
+      HH(p, j) = cs * a1 + sn * a2;
+      HH(p + 1, j) = -sn * a1 + cs * a2;
+    }
   }
   __syncthreads();
 
-  // ---- 6. write back -----------------------------------------------------------
+  // ---- write back ----
   double mul[8];
   int nf = 0;
   if (scaled) nf = safescale_factors(cscale, amax, mul);
@@ -518,70 +780,88 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
   if (tid == 0) bt.status[b] = status;
   __syncthreads();
 }
-#undef AA
 #undef HH
 
-template <class T, class W, int NT, bool HSMEM>
+template <class T, class W, int NT>
 __global__ void __launch_bounds__(NT) k_schur_real(RealBatchT<T, W> bt, const int* __restrict__ order,
-                                                   int* __restrict__ sched, int bin, int nmax) {
+                                                   int* __restrict__ sched, int bin, int nmax, int num_sms) {
   extern __shared__ double smem_raw[];
   T* smem = (T*)smem_raw;
-  __shared__ Ctl<T> c;
   __shared__ int s_job;
   const int start = sched[3 * bin], end = sched[3 * bin + 1];
+  // the chain warps of an SM's CTAs sit on different sub-partitions (warps are dealt to the
+  // four in turn): NW = 4, 8 warps shift by CTA, 2, 6 by pairs of CTAs, odd NW shift by themselves
+  constexpr int NW = NT / 32;
+  const int slot = blockIdx.x / num_sms;
+  const int cw = NW % 4 == 0 ? slot % 4 : (NW % 2 == 0 ? (slot >> 1) & 1 : 0);
   for (;;) {
     if (threadIdx.x == 0) s_job = start + atomicAdd(&sched[3 * bin + 2], 1);
     __syncthreads();
     const int job = s_job;
     __syncthreads();
     if (job >= end) break;
-    solve_real<T, W, NT, HSMEM>(bt, order[job], nmax, smem, c);
+    solve_real<T, W, NT>(bt, order[job], nmax, smem, cw);
   }
 }
 
-// Dynamic shared memory of one CTA for orders up to nmax: the packed H of the QR phase
-// (or the full matrix of the Hessenberg phase, hsmem), tau, the reflector log and the
-// reduction scratch.
-size_t bin_smem_elems(int nmax, bool hsmem) {
-  const size_t full = hsmem ? (size_t)nmax * (nmax | 1) : 0;
-  const size_t hreg = full > (size_t)rpk(nmax + 1) ? full : (size_t)rpk(nmax + 1);
-  return hreg + 6 * (size_t)nmax + 32;
+// Dynamic shared memory of one CTA of the iteration for orders up to nmax: the reflector
+// log and the packed H.
+size_t bin_smem_elems(int nmax) { return kLogElems + (size_t)rpk(nmax + 1); }
+// ... of the reduction: the matrix, and Z where both fit.
+size_t hess_smem_elems(int nmax, size_t tsize) {
+  const size_t one = (size_t)nmax * (nmax | 1), most = (kMaxDynSmem - 8 * 1024) / tsize;
+  return 2 * one <= most ? 2 * one : (one > most ? one : most);
 }
 
-template <class T, class W, int NT, bool HSMEM>
-cudaError_t launch_bin(const RealBatchT<T, W>& bt, const int* order, int* sched, int bin, int nmax, int ctas,
-                       int num_sms, cudaStream_t s) {
-  const size_t smem = sizeof(T) * bin_smem_elems(nmax, HSMEM);
-  cudaError_t e = cudaFuncSetAttribute(k_schur_real<T, W, NT, HSMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <class T, class W, int NC>
+cudaError_t launch_hess(const RealBatchT<T, W>& bt, const int* order, const int* sched, int bin, int nmax,
+                        int num_sms, cudaStream_t s) {
+  const size_t elems = hess_smem_elems(nmax, sizeof(T)), smem = sizeof(T) * elems;
+  cudaError_t e = cudaFuncSetAttribute(k_hess_real<T, W, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_real<T, W, NT, HSMEM>, NT, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hess_real<T, W, NC>, 4 * NC, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
-  if (ctas > 0 && per_sm > ctas) per_sm = ctas;
-  k_schur_real<T, W, NT, HSMEM><<<num_sms * per_sm, NT, smem, s>>>(bt, order, sched, bin, nmax);
+  const int ctas = num_sms * per_sm < bt.count ? num_sms * per_sm : bt.count;
+  k_hess_real<T, W, NC><<<ctas, 4 * NC, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
   return cudaGetLastError();
 }
 
-// One bin with the requested shape.  FP64 compiles every shape of kTuneThreads with
-// and without the shared-memory Hessenberg phase, the FP32 kernel with FP32 eigenvalues
-// (Float32 batches and the FP32 stage of the mixed form) the same but 160 threads, the
-// FP32 kernel with FP64 eigenvalues (the large path's small solves) the default shapes.
+template <class T, class W, int NT>
+cudaError_t launch_bin(const RealBatchT<T, W>& bt, const int* order, int* sched, int bin, int nmax, int ctas,
+                       int num_sms, cudaStream_t s) {
+  cudaError_t e = nmax <= 32 ? launch_hess<T, W, 32>(bt, order, sched, bin, nmax, num_sms, s)
+                             : (nmax <= 64 ? launch_hess<T, W, 64>(bt, order, sched, bin, nmax, num_sms, s)
+                                           : launch_hess<T, W, 128>(bt, order, sched, bin, nmax, num_sms, s));
+  if (e != cudaSuccess) return e;
+  const size_t smem = sizeof(T) * bin_smem_elems(nmax);
+  e = cudaFuncSetAttribute(k_schur_real<T, W, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_real<T, W, NT>, NT, smem);
+  if (e != cudaSuccess) return e;
+  if (per_sm < 1) per_sm = 1;
+  if (ctas > 0 && per_sm > ctas) per_sm = ctas;
+  const int grid = num_sms * per_sm < bt.count ? num_sms * per_sm : bt.count;
+  k_schur_real<T, W, NT><<<grid, NT, smem, s>>>(bt, order, sched, bin, nmax, num_sms);
+  return cudaGetLastError();
+}
+
+// One bin with the requested shape: FP64 compiles every thread count of kTuneThreads, the FP32
+// kernel with FP32 eigenvalues (Float32 batches and the FP32 stage of the mixed form) all but
+// 160, the FP32 kernel with FP64 eigenvalues (the large path's small solves) the default ones.
 template <class T, class W>
 cudaError_t launch_shape(const RealBatchT<T, W>& bt, const int* order, int* sched, int bin, int nmax, int nt,
-                         int hsmem, int ctas, int num_sms, cudaStream_t s) {
-#define GS_SHAPE(NTV, HS) \
-  if (nt == NTV && (hsmem != 0) == HS) return launch_bin<T, W, NTV, HS>(bt, order, sched, bin, nmax, ctas, num_sms, s);
+                         int ctas, int num_sms, cudaStream_t s) {
+#define GS_SHAPE(NTV) \
+  if (nt == NTV) return launch_bin<T, W, NTV>(bt, order, sched, bin, nmax, ctas, num_sms, s);
   if constexpr (sizeof(T) == 8) {
-    GS_SHAPE(64, true) GS_SHAPE(64, false) GS_SHAPE(96, true) GS_SHAPE(96, false)
-    GS_SHAPE(128, true) GS_SHAPE(128, false) GS_SHAPE(160, true) GS_SHAPE(160, false)
-    GS_SHAPE(192, true) GS_SHAPE(192, false) GS_SHAPE(256, true) GS_SHAPE(256, false)
+    GS_SHAPE(64) GS_SHAPE(96) GS_SHAPE(128) GS_SHAPE(160) GS_SHAPE(192) GS_SHAPE(256)
   } else if constexpr (std::is_same_v<W, float>) {
-    GS_SHAPE(64, true) GS_SHAPE(64, false) GS_SHAPE(96, true) GS_SHAPE(96, false)
-    GS_SHAPE(128, true) GS_SHAPE(128, false) GS_SHAPE(192, true) GS_SHAPE(192, false)
-    GS_SHAPE(256, true) GS_SHAPE(256, false)
+    GS_SHAPE(64) GS_SHAPE(96) GS_SHAPE(128) GS_SHAPE(192) GS_SHAPE(256)
   } else {
-    GS_SHAPE(64, true) GS_SHAPE(128, false)
+    GS_SHAPE(64) GS_SHAPE(128)
   }
 #undef GS_SHAPE
   return cudaErrorInvalidValue;
@@ -593,7 +873,7 @@ cudaError_t launch_all_bins(const RealBatchT<T, W>& bt, const int* order, int* s
   // largest bin first: it carries most of the work
   for (int i = 0; i < kNumBins; ++i) {
     const int bin = kNumBins - 1 - i;
-    cudaError_t e = launch_shape(bt, order, sched, bin, t.bounds[bin], t.nt[bin], t.hsmem[bin], t.ctas[bin], num_sms,
+    cudaError_t e = launch_shape(bt, order, sched, bin, t.bounds[bin], t.nt[bin], t.ctas[bin], num_sms,
                                  streams[i % nstreams]);
     if (e != cudaSuccess) return e;
   }
@@ -602,8 +882,14 @@ cudaError_t launch_all_bins(const RealBatchT<T, W>& bt, const int* order, int* s
 
 }  // namespace
 
-size_t real_bin_smem_bytes(int nmax, int hsmem) { return sizeof(double) * bin_smem_elems(nmax, hsmem != 0); }
-size_t real32_bin_smem_bytes(int nmax, int hsmem) { return sizeof(float) * bin_smem_elems(nmax, hsmem != 0); }
+// A tuning row's hsmem flag (the Hessenberg phase in shared memory) selects nothing here any
+// more: the reduction always runs in shared memory.
+size_t real_bin_smem_bytes(int nmax, int) {
+  return sizeof(double) * (bin_smem_elems(nmax) > hess_smem_elems(nmax, 8) ? bin_smem_elems(nmax) : hess_smem_elems(nmax, 8));
+}
+size_t real32_bin_smem_bytes(int nmax, int) {
+  return sizeof(float) * (bin_smem_elems(nmax) > hess_smem_elems(nmax, 4) ? bin_smem_elems(nmax) : hess_smem_elems(nmax, 4));
+}
 
 template <class T, class W>
 cudaError_t launch_schur_batched_real(const RealBatchT<T, W>& bt, const int* order, int* sched, int num_sms,
@@ -621,7 +907,7 @@ template <class T, class W>
 cudaError_t launch_schur_real_one(const RealBatchT<T, W>& bt, int m, const int* order, int* sched, cudaStream_t s) {
   const BinTuning t = default_tuning_real();
   const int bin = default_bin_of(m);
-  return launch_shape(bt, order, sched, bin, t.bounds[bin], t.nt[bin], t.hsmem[bin], 1, 1, s);
+  return launch_shape(bt, order, sched, bin, t.bounds[bin], t.nt[bin], 1, 1, s);
 }
 template cudaError_t launch_schur_real_one<double, double>(const RealBatchT<double, double>&, int, const int*, int*,
                                                            cudaStream_t);
