@@ -317,15 +317,19 @@ __device__ inline double2 zreflector2(double2& a, double2& x1) {
 // which square the relative error per step (23 -> 46 -> past 53 bits).  Inputs are
 // kept inside [1e-290, 1e290] by the callers; extreme values take the scaled path.
 namespace gsk {
+// y / 2 for a normal y well inside the range: the exponent's last bit, off the FP64 pipe
+__device__ __forceinline__ double half_normal(double y) {
+  return __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));
+}
 __device__ __forceinline__ double rsqrt_nr(double s) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
   double h = s * y;
   double e = fma(-h, y, 1.0);
-  y = fma(0.5 * y, e, y);
+  y = fma(half_normal(y), e, y);
   h = s * y;
   e = fma(-h, y, 1.0);
-  return fma(0.5 * y, e, y);
+  return fma(half_normal(y), e, y);
 }
 __device__ __forceinline__ double rcp_nr(double d) {
   double r;

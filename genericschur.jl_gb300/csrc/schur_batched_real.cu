@@ -379,85 +379,133 @@ __device__ __forceinline__ void apply_line(T* p, int inc, int d, const T* lg, in
   *p1 = z1;
 }
 
-// Reflector from (a, x1, x2); in FP64 the pairs x1 t, x2 t and t1 v2, t1 v3 are one
-// instruction each on two lanes (an FP64 instruction costs the pipe the same for 1 or 32 lanes).
+// Reflector (householder.jl:12-54, as reflector_fast) of (a, x1, x2), x2 = 0 for a 2-element one;
+// a <- beta.  One test sends every case off the plain path to reflector_fast.
 __device__ __forceinline__ Refl<float> chain_refl(float& a, float x1, float x2, int nr, int) {
-  const float t1 = reflector_fast(a, x1, x2, nr);
-  return {t1, t1 * x1, t1 * x2, x1, x2};
+  const float ss = fmaf(a, a, fmaf(x1, x1, x2 * x2));
+  if (!(ss > 1.0e-30f && ss < 1.0e30f) || ((__float_as_uint(x1) | __float_as_uint(x2)) << 1) == 0) {
+    const float t1 = reflector_fast(a, x1, x2, nr);
+    return {t1, t1 * x1, t1 * x2, x1, x2};
+  }
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(ss));
+  const float s = ss * y;
+  const float aa = fabsf(a);
+  const float tau = fmaf(aa, y, 1.0f);
+  const float t = copysignf(__frcp_rn(aa + s), a);
+  x1 *= t;
+  x2 *= t;
+  a = -copysignf(s, a);
+  return {tau, tau * x1, tau * x2, x1, x2};
 }
-__device__ __forceinline__ Refl<double> chain_refl(double& a, double x1, double x2, int nr, int) {
-  const double t1 = reflector_fast(a, x1, x2, nr);
-  return {t1, t1 * x1, t1 * x2, x1, x2};
+// FP64: every FP64 instruction holds the sub-partition's pipe for 64 cycles whether 1 or 32 lanes are
+// active, so a step of the chase costs its number of FP64 instructions: 5 for the left update (a column
+// per lane), 5 for the right update (a row per lane) and 17 here: independent pairs (tau and s,
+// v2 and v3, t2 and t3) are one instruction on two lanes each, the range tests are on the bits.
+__device__ __forceinline__ Refl<double> chain_refl(double& a, double x1, double x2, int nr, int lane) {
+  const double xs = fma(x1, x1, x2 * x2);
+  const double ss = fma(a, a, xs);
+  // xs != 0 and 1e-290 < ss < 1e290 (nonnegative values; NaN is above all)
+  const long long sb = __double_as_longlong(ss);
+  if (__double_as_longlong(xs) == 0 || sb <= __double_as_longlong(1.0e-290) || sb >= __double_as_longlong(1.0e290)) {
+    const double t1 = reflector_fast(a, x1, x2, nr);
+    return {t1, t1 * x1, t1 * x2, x1, x2};
+  }
+  const double y = rsqrt_nr(ss);
+  const double aa = fabs(a);
+  // even lanes tau = |a| y + 1, odd lanes s = ss y
+  const double ts = fma((lane & 1) ? ss : aa, y, (lane & 1) ? 0.0 : 1.0);
+  const double tau = __shfl_sync(0xffffffffu, ts, 0), s = __shfl_sync(0xffffffffu, ts, 1);
+  const double t = copysign(rcp_nr(aa + s), a);
+  // even lanes v2, t2; odd lanes v3, t3
+  const double v = ((lane & 1) ? x2 : x1) * t;
+  const double tv = tau * v;
+  a = -copysign(s, a);
+  return {tau, __shfl_sync(0xffffffffu, tv, 0), __shfl_sync(0xffffffffu, tv, 1), __shfl_sync(0xffffffffu, v, 0),
+          __shfl_sync(0xffffffffu, v, 1)};
+}
+
+__device__ __forceinline__ void st_refl(float* l, const Refl<float>& r) {
+  *(float4*)l = make_float4(r.t1, r.t2, r.t3, r.v2);
+  l[4] = r.v3;
+}
+__device__ __forceinline__ void st_refl(double* l, const Refl<double>& r) {
+  *(double2*)l = make_double2(r.t1, r.t2);
+  *(double2*)(l + 2) = make_double2(r.t3, r.v2);
+  l[4] = r.v3;
 }
 
 // Chain warp: steps ka..ka+nst-1 inside the window (columns ..wl, rows ka-1..).  r: the reflector of
-// step ka on entry, of step ka+nst on return.
+// step ka on entry, of step ka+nst on return.  The loop is written for few instructions and no
+// branches: one warp runs it alone, so each costs about four cycles.  Lanes outside the window
+// compute on clamped addresses and store nothing.
 template <class T>
 __device__ __forceinline__ void chase_chunk(T* H, int ka, int nst, int iend, int wl, Refl<T>& r, T* lg, int lane) {
-  const int j = ka + lane;
-  const bool colok = j <= wl;
-  T* hc = H + rpk(colok ? j : ka) - 1;  // hc[i] = H(i, j)
-  const int i = ka - 1 + lane;
+  const unsigned all = 0xffffffffu;
+  const int n3 = min(nst, iend - 1 - ka);     // steps with a 3-element reflector
+  const int j = min(ka + lane, wl);           // left updates: a column per lane
+  const bool colok = ka + lane <= wl;
+  T* hc = H + rpk(j) + ka - 1;                // H(k, j)
+  const int i = ka - 1 + lane;                // right updates: a row per lane
   const bool rowok = i >= 1 && i <= iend;
-  T* hr = H + i - 1;  // hr[rpk(c)] = H(i, c)
+  const int ic = min(max(i, 1), iend) - 1;
   int c0 = rpk(ka);
-  T a0 = hc[ka], a1 = hc[ka + 1], a2 = hc[ka + 2];
-  for (int s = 0; s < nst; ++s) {
+  T* p0 = H + c0 + ic;                        // H(i, k), H(i, k+1), H(i, k+2)
+  T* p1 = p0 + ka + 3;
+  T* p2 = p1 + ka + 4;
+  T* hb = H + c0 + ka;                        // H(k+1, k)
+  T a0 = hc[0], a1 = hc[1], a2 = hc[2];
+  for (int s = 0; s < n3; ++s) {
     const int k = ka + s;
-    if (lane == 0) {
-      T* l = lg + kLogStep * s;
-      l[0] = r.t1; l[1] = r.t2; l[2] = r.t3; l[3] = r.v2; l[4] = r.v3;
+    if (lane == 0) st_refl(lg, r);
+    lg += kLogStep;
+    {
+      const T ss = fma(r.v3, a2, fma(r.v2, a1, a0));
+      a0 = fma(-ss, r.t1, a0);
+      a1 = fma(-ss, r.t2, a1);
+      a2 = fma(-ss, r.t3, a2);
     }
-    if (k <= iend - 2) {
-      if (colok && j >= k) {
-        const T ss = fma(r.v3, a2, fma(r.v2, a1, a0));
-        hc[k] = fma(-ss, r.t1, a0);
-        hc[k + 1] = fma(-ss, r.t2, a1);
-        hc[k + 2] = fma(-ss, r.t3, a2);
-      }
-      __syncwarp();
-      T x = T(0);
-      if (rowok && i <= k + 3) {
-        T* h0 = hr + c0;
-        T* h1 = h0 + k + 3;
-        T* h2 = h1 + k + 4;
-        const T b0 = *h0, b1 = *h1, b2 = *h2;
-        const T ss = fma(r.v3, b2, fma(r.v2, b1, b0));
-        x = fma(-ss, r.t1, b0);
-        *h0 = x;
-        *h1 = fma(-ss, r.t2, b1);
-        *h2 = fma(-ss, r.t3, b2);
-      }
-      // column k, rows k+1..k+3: the next reflector
-      T a = __shfl_sync(0xffffffffu, x, s + 2);
-      const T x1 = __shfl_sync(0xffffffffu, x, s + 3);
-      const T x2 = __shfl_sync(0xffffffffu, x, s + 4);
-      __syncwarp();
-      a0 = hc[k + 1]; a1 = hc[k + 2]; a2 = hc[k + 3];
-      r = chain_refl(a, x1, x2, min(3, iend - k), lane);
-      if (lane == 0) {
-        T* h = H + c0 + k;  // H(k+1, k)
-        h[0] = a;
-        h[1] = T(0);
-        if (k + 1 < iend - 1) h[2] = T(0);
-      }
-      c0 += k + 3;
-    } else {
-      // 2-element reflector at k = iend-1
-      if (colok && j >= k) {
-        const T ss = fma(r.v2, a1, a0);
-        hc[k] = fma(-ss, r.t1, a0);
-        hc[k + 1] = fma(-ss, r.t2, a1);
-      }
-      __syncwarp();
-      if (rowok) {
-        T* h0 = hr + c0;
-        T* h1 = h0 + k + 3;
-        const T b0 = *h0, b1 = *h1;
-        const T ss = fma(r.v2, b1, b0);
-        *h0 = fma(-ss, r.t1, b0);
-        *h1 = fma(-ss, r.t2, b1);
-      }
+    if (colok && j >= k) { hc[0] = a0; hc[1] = a1; hc[2] = a2; }
+    __syncwarp();
+    T b0 = *p0, b1 = *p1, b2 = *p2;
+    {
+      const T ss = fma(r.v3, b2, fma(r.v2, b1, b0));
+      b0 = fma(-ss, r.t1, b0);
+      b1 = fma(-ss, r.t2, b1);
+      b2 = fma(-ss, r.t3, b2);
+    }
+    // column k, rows k+1..k+3: the next reflector
+    T a = __shfl_sync(all, b0, s + 2);
+    const T x1 = __shfl_sync(all, b0, s + 3);
+    T x2 = __shfl_sync(all, b0, s + 4);
+    if (rowok && i <= k + 3) { *p0 = b0; *p1 = b1; *p2 = b2; }
+    __syncwarp();
+    ++hc;
+    a0 = hc[0]; a1 = hc[1]; a2 = hc[2];
+    const int nr = min(3, iend - k);
+    if (nr < 3) x2 = T(0);
+    r = chain_refl(a, x1, x2, nr, lane);
+    if (lane == 0) { hb[0] = a; hb[1] = T(0); hb[2] = T(0); }
+    hb += k + 4;
+    p0 = p1;
+    p1 = p2;
+    p2 += k + 5;
+  }
+  if (n3 < nst) {
+    // 2-element reflector at k = iend-1
+    const int k = iend - 1;
+    if (lane == 0) st_refl(lg, r);
+    if (colok && j >= k) {
+      const T ss = fma(r.v2, a1, a0);
+      hc[0] = fma(-ss, r.t1, a0);
+      hc[1] = fma(-ss, r.t2, a1);
+    }
+    __syncwarp();
+    if (rowok) {
+      const T b0 = *p0, b1 = *p1;
+      const T ss = fma(r.v2, b1, b0);
+      *p0 = fma(-ss, r.t1, b0);
+      *p1 = fma(-ss, r.t2, b1);
     }
   }
   __syncwarp();
@@ -782,8 +830,9 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
 }
 #undef HH
 
+// 768 threads per SM: at most 80 registers
 template <class T, class W, int NT>
-__global__ void __launch_bounds__(NT) k_schur_real(RealBatchT<T, W> bt, const int* __restrict__ order,
+__global__ void __launch_bounds__(NT, 768 / NT) k_schur_real(RealBatchT<T, W> bt, const int* __restrict__ order,
                                                    int* __restrict__ sched, int bin, int nmax, int num_sms) {
   extern __shared__ double smem_raw[];
   T* smem = (T*)smem_raw;
