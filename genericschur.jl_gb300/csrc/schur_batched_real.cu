@@ -2,7 +2,7 @@
 // instance of the same code for Float32 batches and the FP32 stage of the mixed form).
 //
 // Per size bin two launches over the bin's queue of matrices (largest first):
-//   k_hess_real   load + _scale! (util.jl:14-29), Householder Hessenberg reduction
+//   k_hess_real64 / k_hess_real32, k_formq_real32   load + _scale! (util.jl:14-29), Householder Hessenberg reduction
 //                 (hessenberg.jl:3-17; reflector as in householder.jl:12-54, lmul!/rmul!
 //                 as householder.jl:140-172) and Q formation (hessenberg.jl:150-166);
 //   k_schur_real  the real double-shift Francis iteration of gschur!(H::Hessenberg{<:Real}, Z)
@@ -42,9 +42,10 @@ __host__ __device__ __forceinline__ int rpk(int j) { return ((j - 1) * (j + 6)) 
 // FP32, the latency of the seven barrier-separated steps per column.  With the matrix read
 // from the L2-resident output buffer, one column per thread (32 lines per warp load), this phase
 // took 31M cycles of an FP32 matrix of order 128 (57% of its time) and 17M of an FP64 one.
+template <class T>
 struct HessCtl {
-  double tau, t, beta;  // of the current column (exact for T = float too)
-  int mode;             // 0: zero column, 1: reflector ready, 2: underflow guard needed
+  T tau, t, beta;  // of the current column
+  int mode;        // 0: zero column, 1: reflector ready, 2: underflow guard needed
 };
 
 // max |.| over nonnegative values by their bit patterns: NaN compares largest, as block_max
@@ -59,17 +60,133 @@ template <class T> __device__ __forceinline__ T bits_abs(unsigned long long b);
 template <> __device__ __forceinline__ double bits_abs<double>(unsigned long long b) { return __longlong_as_double((long long)b); }
 template <> __device__ __forceinline__ float bits_abs<float>(unsigned long long b) { return __uint_as_float((unsigned)b); }
 
-template <class T, class W, int NC>
-__global__ void __launch_bounds__(4 * NC) k_hess_real(RealBatchT<T, W> bt, const int* __restrict__ order,
-                                                      const int* __restrict__ sched, int bin, int nmax, int cap) {
+template <class T>
+struct HessShared {
+  T red[32];
+  unsigned long long gmax[4];
+  T gssq[4];
+  HessCtl<T> c;
+};
+
+// Entries outside the range where squaring is safe, or the underflow guard
+// (householder.jl:25-42): rescale x, alpha and beta.  All NT threads; ends behind a barrier.
+template <class T, int NT>
+__device__ __noinline__ void hess_reflector_guarded(T* col, int m, HessShared<T>& sh, T& tau, T& t, T& beta) {
+  const int tid = threadIdx.x;
+  const T sfmin = T(2) * Prec<T>::fmin / Prec<T>::eps;
+  T big = T(0);
+  for (int w = 0; w < 4; ++w) { const T v = bits_abs<T>(sh.gmax[w]); big = (v > big || v != v) ? v : big; }
+  const bool safe = (big < Prec<T>::safe_hi && big > Prec<T>::safe_lo);
+  const T sc = safe ? T(1) : T(1) / big;
+  T ls = T(0);
+  for (int r = 1 + tid; r < m; r += NT) { const T v = col[r] * sc; ls = fma(v, v, ls); }
+  const T ssq = block_sum<NT>(ls, sh.red);
+  T xnorm = safe ? sqrt(ssq) : big * sqrt(ssq);
+  T alpha = col[0];
+  beta = -copysign(hypot(alpha, xnorm), alpha);
+  int kount = 0;
+  if (fabs(beta) < sfmin) {
+    const T rsfmin = T(1) / sfmin;
+    T bb = beta;
+    do { ++kount; bb *= rsfmin; alpha *= rsfmin; } while (fabs(bb) < sfmin && kount < 20);
+    __syncthreads();
+    for (int r = 1 + tid; r < m; r += NT) {
+      T v = col[r];
+      for (int q = 0; q < kount; ++q) v *= rsfmin;
+      col[r] = v;
+    }
+    __syncthreads();
+    T lm2 = T(0);
+    for (int r = 1 + tid; r < m; r += NT) lm2 = fmax(lm2, fabs(col[r]));
+    const T big2 = block_max<NT>(lm2, sh.red);
+    const T sc2 = (big2 > T(0)) ? T(1) / big2 : T(0);
+    T ls2 = T(0);
+    for (int r = 1 + tid; r < m; r += NT) { const T v = col[r] * sc2; ls2 = fma(v, v, ls2); }
+    const T ssq2 = block_sum<NT>(ls2, sh.red);
+    xnorm = big2 * sqrt(ssq2);
+    beta = -copysign(hypot(alpha, xnorm), alpha);
+  }
+  tau = (beta - alpha) / beta;
+  t = T(1) / (alpha - beta);
+  for (int q = 0; q < kount; ++q) beta *= sfmin;
+  __syncthreads();
+}
+
+// Scalars of the reflector from the warps' maxima and sums: the mode as in HessCtl.
+template <class T>
+__device__ __forceinline__ int hess_scalars(const HessShared<T>& sh, T alpha, T& tau, T& t, T& beta) {
+  const T sfmin = T(2) * Prec<T>::fmin / Prec<T>::eps;
+  unsigned long long mb = sh.gmax[0];
+  for (int w = 1; w < 4; ++w) mb = sh.gmax[w] > mb ? sh.gmax[w] : mb;
+  const T big = bits_abs<T>(mb);
+  tau = t = beta = T(0);
+  if (big == T(0)) return 0;
+  if (!(big < Prec<T>::safe_hi && big > Prec<T>::safe_lo)) return 2;
+  T ssq = sh.gssq[0];
+  for (int w = 1; w < 4; ++w) ssq += sh.gssq[w];
+  const T xnorm = sqrt(ssq);
+  beta = -copysign(hypot(alpha, xnorm), alpha);
+  if (fabs(beta) < sfmin) return 2;
+  tau = (beta - alpha) / beta;
+  t = T(1) / (alpha - beta);
+  return 1;
+}
+
+// Reflector of col[0..m): tau, the scale t of the tail and beta (householder.jl:12-54); false when
+// the tail is zero.  All 4*NC threads call it; it ends behind a barrier.
+template <class T, int NT>
+__device__ __forceinline__ bool hess_reflector(T* col, int m, HessShared<T>& sh, T& tau, T& t, T& beta) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // norm of the tail: elements 1+32w..32+32w are warp w's, summed by a tree, the warps' sums in order
+  if (warp < 4) {
+    const T x = (1 + tid < m) ? col[1 + tid] : T(0);
+    unsigned long long mb = abs_bits<T>(x);
+    T q = fma(x, x, T(0));
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long w = __shfl_xor_sync(0xffffffffu, mb, o);
+      mb = w > mb ? w : mb;
+      q += __shfl_xor_sync(0xffffffffu, q, o);
+    }
+    if (lane == 0) { sh.gmax[warp] = mb; sh.gssq[warp] = q; }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    T tau_, t_, beta_;
+    const int mode = hess_scalars(sh, col[0], tau_, t_, beta_);
+    if (lane == 0) { sh.c.mode = mode; sh.c.tau = tau_; sh.c.t = t_; sh.c.beta = beta_; }
+  }
+  __syncthreads();
+  const int mode = sh.c.mode;
+  if (mode == 0) return false;
+  tau = sh.c.tau; t = sh.c.t; beta = sh.c.beta;
+  if (mode == 2) hess_reflector_guarded<T, NT>(col, m, sh, tau, t, beta);
+  return true;
+}
+
+// _scale! factors (util.jl:14-29) on element-wise access; returns whether the matrix was scaled.
+template <class T, class F>
+__device__ __forceinline__ void hess_scale(double amax, F each) {
+  const double smlnum = sqrt((double)Prec<T>::fmin) / (double)Prec<T>::eps;
+  const double bignum = 1.0 / smlnum;
+  double cscale = 0.0;
+  if (amax > 0.0 && amax < smlnum) cscale = smlnum;
+  else if (amax > bignum) cscale = bignum;
+  if (cscale == 0.0) return;
+  double mul[8];
+  const int nf = safescale_factors(amax, cscale, mul);
+  for (int f = 0; f < nf; ++f) each(mul[f]);
+  __syncthreads();
+}
+
+template <class W, int NC>
+__global__ void __launch_bounds__(4 * NC) k_hess_real64(RealBatchT<double, W> bt, const int* __restrict__ order,
+                                                        const int* __restrict__ sched, int bin, int nmax, int cap) {
+  typedef double T;
   constexpr int NT = 4 * NC;
   extern __shared__ double smem_raw[];
   __shared__ T part[4][NC];
-  __shared__ T red[32];
-  __shared__ unsigned long long gmax[4];
-  __shared__ T gssq[4];
-  __shared__ HessCtl hc;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ HessShared<T> sh;
+  const int tid = threadIdx.x;
   const int start = sched[3 * bin], end = sched[3 * bin + 1];
   const bool isz = tid >= 2 * NC;
   const int c = tid % NC, par = (tid / NC) & 1;
@@ -80,7 +197,7 @@ __global__ void __launch_bounds__(4 * NC) k_hess_real(RealBatchT<T, W> bt, const
     T* __restrict__ Ag = bt.A + bt.offs[b];
     T* __restrict__ Zg = bt.wantz ? bt.Z + bt.offs[b] : nullptr;
     const int ld = n | 1;
-    T* A = (T*)smem_raw;
+    T* A = smem_raw;
     // Z in shared memory beside A where the launch left room for it
     const bool zs = Zg && 2 * n * ld <= cap;
     T* Z = zs ? A + n * ld : Zg;
@@ -92,111 +209,20 @@ __global__ void __launch_bounds__(4 * NC) k_hess_real(RealBatchT<T, W> bt, const
       const T a = Ag[idx];
       A[i + j * ld] = a;
       if (Zg) Z[i + j * ldz] = (i == j) ? T(1) : T(0);
-      const double aa = fabs((double)a);
+      const double aa = fabs(a);
       amax = (aa > amax || aa != aa) ? aa : amax;
     }
-    amax = (double)block_max<NT>((T)amax, red);
+    amax = block_max<NT>(amax, sh.red);
     __syncthreads();
-    if (bt.scale) {
-      const double smlnum = sqrt((double)Prec<T>::fmin) / (double)Prec<T>::eps;
-      const double bignum = 1.0 / smlnum;
-      double cscale = 0.0;
-      if (amax > 0.0 && amax < smlnum) cscale = smlnum;
-      else if (amax > bignum) cscale = bignum;
-      if (cscale != 0.0) {
-        double mul[8];
-        const int nf = safescale_factors(amax, cscale, mul);
-        for (int f = 0; f < nf; ++f)
-          for (int idx = tid; idx < n * n; idx += NT) {
-            const int i = idx % n, j = idx / n;
-            A[i + j * ld] = (T)((double)A[i + j * ld] * mul[f]);
-          }
-        __syncthreads();
-      }
-    }
-    const T sfmin = T(2) * Prec<T>::fmin / Prec<T>::eps;
+    if (bt.scale)
+      hess_scale<T>(amax, [&](double f) {
+        for (int idx = tid; idx < n * n; idx += NT) A[idx % n + idx / n * ld] *= f;
+      });
     for (int i = 1; i <= n - 2; ++i) {
       const int m = n - i;                     // reflector length: rows i+1..n
       T* col = A + i + (size_t)(i - 1) * ld;   // col[0] = alpha, col[1..m-1] = x
-      // norm of x: elements 1+32w..32+32w are warp w's, summed by a tree, the warps' sums in order
-      if (warp < 4) {
-        const T x = (1 + tid < m) ? col[1 + tid] : T(0);
-        unsigned long long mb = abs_bits<T>(x);
-        T q = fma(x, x, T(0));
-        for (int o = 16; o > 0; o >>= 1) {
-          const unsigned long long w = __shfl_xor_sync(0xffffffffu, mb, o);
-          mb = w > mb ? w : mb;
-          q += __shfl_xor_sync(0xffffffffu, q, o);
-        }
-        if (lane == 0) { gmax[warp] = mb; gssq[warp] = q; }
-      }
-      __syncthreads();
-      if (warp == 0) {
-        unsigned long long mb = gmax[0];
-        for (int w = 1; w < 4; ++w) mb = gmax[w] > mb ? gmax[w] : mb;
-        const T big = bits_abs<T>(mb);
-        int mode = 0;
-        T tau = T(0), t = T(0), beta = T(0);
-        if (big != T(0)) {
-          mode = 2;
-          if (big < Prec<T>::safe_hi && big > Prec<T>::safe_lo) {
-            T ssq = gssq[0];
-            for (int w = 1; w < 4; ++w) ssq += gssq[w];
-            const T xnorm = sqrt(ssq);
-            const T alpha = col[0];
-            beta = -copysign(hypot(alpha, xnorm), alpha);
-            if (!(fabs(beta) < sfmin)) {
-              mode = 1;
-              tau = (beta - alpha) / beta;
-              t = T(1) / (alpha - beta);
-            }
-          }
-        }
-        if (lane == 0) { hc.mode = mode; hc.tau = (double)tau; hc.t = (double)t; hc.beta = (double)beta; }
-      }
-      __syncthreads();
-      const int mode = hc.mode;
-      if (mode == 0) continue;
-      T tau = (T)hc.tau, t = (T)hc.t, beta = (T)hc.beta;
-      if (mode == 2) {
-        // entries outside the range where squaring is safe, or the underflow guard
-        // (householder.jl:25-42): rescale x, alpha and beta
-        T big = T(0);
-        for (int w = 0; w < 4; ++w) { const T v = bits_abs<T>(gmax[w]); big = (v > big || v != v) ? v : big; }
-        const bool safe = (big < Prec<T>::safe_hi && big > Prec<T>::safe_lo);
-        const T sc = safe ? T(1) : T(1) / big;
-        T ls = T(0);
-        for (int r = 1 + tid; r < m; r += NT) { const T v = col[r] * sc; ls = fma(v, v, ls); }
-        const T ssq = block_sum<NT>(ls, red);
-        T xnorm = safe ? sqrt(ssq) : big * sqrt(ssq);
-        T alpha = col[0];
-        beta = -copysign(hypot(alpha, xnorm), alpha);
-        int kount = 0;
-        if (fabs(beta) < sfmin) {
-          const T rsfmin = T(1) / sfmin;
-          T bb = beta;
-          do { ++kount; bb *= rsfmin; alpha *= rsfmin; } while (fabs(bb) < sfmin && kount < 20);
-          __syncthreads();
-          for (int r = 1 + tid; r < m; r += NT) {
-            T v = col[r];
-            for (int q = 0; q < kount; ++q) v *= rsfmin;
-            col[r] = v;
-          }
-          __syncthreads();
-          T lm2 = T(0);
-          for (int r = 1 + tid; r < m; r += NT) lm2 = fmax(lm2, fabs(col[r]));
-          const T big2 = block_max<NT>(lm2, red);
-          const T sc2 = (big2 > T(0)) ? T(1) / big2 : T(0);
-          T ls2 = T(0);
-          for (int r = 1 + tid; r < m; r += NT) { const T v = col[r] * sc2; ls2 = fma(v, v, ls2); }
-          const T ssq2 = block_sum<NT>(ls2, red);
-          xnorm = big2 * sqrt(ssq2);
-          beta = -copysign(hypot(alpha, xnorm), alpha);
-        }
-        tau = (beta - alpha) / beta;
-        t = T(1) / (alpha - beta);
-        for (int q = 0; q < kount; ++q) beta *= sfmin;
-      }
+      T tau, t, beta;
+      if (!hess_reflector<T, NT>(col, m, sh, tau, t, beta)) continue;
       if (1 + tid < m) col[1 + tid] *= t;
       __syncthreads();
       if (tid == 0) col[0] = beta;
@@ -210,28 +236,18 @@ __global__ void __launch_bounds__(4 * NC) k_hess_real(RealBatchT<T, W> bt, const
         else if (Zg && c < n) { x = Z + c + (size_t)i * ldz; st = ldz; }
         T a = T(0);
         if (x) {
-          if (par == 0) {
-            a = x[0];
+          if (par == 0) a = x[0];
 #pragma unroll 4
-            for (int r = 1; r < m; r += 2) a = fma(col[r], x[r * st], a);
-          } else {
-#pragma unroll 4
-            for (int r = 2; r < m; r += 2) a = fma(col[r], x[r * st], a);
-          }
+          for (int r = 1 + par; r < m; r += 2) a = fma(col[r], x[r * st], a);
         }
         part[tid / NC][c] = a;
         __syncthreads();
         if (x) {
           const int g = isz ? 2 : 0;
           const T va = (part[g][c] + part[g + 1][c]) * tau;
-          if (par == 0) {
-            x[0] -= va;
+          if (par == 0) x[0] -= va;
 #pragma unroll 4
-            for (int r = 1; r < m; r += 2) x[r * st] = fma(-va, col[r], x[r * st]);
-          } else {
-#pragma unroll 4
-            for (int r = 2; r < m; r += 2) x[r * st] = fma(-va, col[r], x[r * st]);
-          }
+          for (int r = 1 + par; r < m; r += 2) x[r * st] = fma(-va, col[r], x[r * st]);
         }
       }
       __syncthreads();
@@ -240,27 +256,17 @@ __global__ void __launch_bounds__(4 * NC) k_hess_real(RealBatchT<T, W> bt, const
         T* x = (!isz && c < n) ? A + c + (size_t)i * ld : nullptr;
         T a = T(0);
         if (x) {
-          if (par == 0) {
-            a = x[0];
+          if (par == 0) a = x[0];
 #pragma unroll 4
-            for (int q = 1; q < m; q += 2) a = fma(x[q * ld], col[q], a);
-          } else {
-#pragma unroll 4
-            for (int q = 2; q < m; q += 2) a = fma(x[q * ld], col[q], a);
-          }
+          for (int q = 1 + par; q < m; q += 2) a = fma(x[q * ld], col[q], a);
           part[par][c] = a;
         }
         __syncthreads();
         if (x) {
           const T va = (part[0][c] + part[1][c]) * tau;
-          if (par == 0) {
-            x[0] -= va;
+          if (par == 0) x[0] -= va;
 #pragma unroll 4
-            for (int q = 1; q < m; q += 2) x[q * ld] = fma(-va, col[q], x[q * ld]);
-          } else {
-#pragma unroll 4
-            for (int q = 2; q < m; q += 2) x[q * ld] = fma(-va, col[q], x[q * ld]);
-          }
+          for (int q = 1 + par; q < m; q += 2) x[q * ld] = fma(-va, col[q], x[q * ld]);
         }
       }
       __syncthreads();
@@ -272,6 +278,230 @@ __global__ void __launch_bounds__(4 * NC) k_hess_real(RealBatchT<T, W> bt, const
       if (zs) Zg[idx] = Z[i + j * ld];
     }
     if (tid == 0) bt.wr[bt.woffs[b]] = (W)amax;  // for the unscaling; k_schur_real overwrites it
+  }
+}
+
+// FP32: bound by latency (a line's sum is a serial chain; about seven cycles per instruction and warp,
+// four barriers per column), so many CTAs per SM matter: the reduction of A and the formation of Z
+// are kernels of their own.  A pair of neighbouring lanes holds a column or row of A.  A line's entries
+// stay in registers between its dot product and its update, in blocks of eight (A is padded by 16
+// zero rows and columns so that a block needs no bounds), and the reflector is read four entries at a
+// time.  The essential parts of the reflectors stay below the subdiagonal of A and their scalars
+// in the (not yet computed) imaginary parts of the eigenvalues, for k_formq_real32.
+constexpr int kHessPad = 16;
+// leading dimension = 18 mod 32: sixteen columns' pairs of neighbouring rows fall into 32 banks,
+// and sixteen rows' pairs of neighbouring columns into 30
+__host__ __device__ __forceinline__ int hess_ld32(int n) { return ((n + kHessPad + 13) & ~31) + 18; }
+
+// dst[8 k + e], e = 0..7, for the blocks k < nb: f(k, u) with u the coefficients of block k
+template <int NB, class F>
+__device__ __forceinline__ void coef_blocks(const float* co, int k0, int k1, F f) {
+#pragma unroll
+  for (int k = 0; k < NB; ++k)
+    if (k >= k0 && k < k1) {
+      const float4 u0 = *(const float4*)(co + 8 * k), u1 = *(const float4*)(co + 8 * k + 4);
+      const float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+      f(k, u);
+    }
+}
+
+// One line p[0], p[st], p[2 st], ... of A against 1, co: p -= tau (p . v) v.  x: registers.  All
+// lanes of the warp call it, those without a line of their own (on = false) with another's.
+template <int NB>
+__device__ __forceinline__ void hess_line32(float* p, int st, int par, int nb, const float* co, float tau, bool on,
+                                            float (&x)[8 * NB]) {
+  const float x0 = p[0];
+  float a = par == 0 ? x0 : 0.f;
+  float* q = p + (1 + par) * st;
+#pragma unroll
+  for (int k = 0; k <= NB; ++k) {
+    // the loads of block k are in flight during the sums of block k-1
+    if (k < NB && k < nb) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[(8 * k + e) % (8 * NB)] = q[2 * (8 * k + e) * st];
+    }
+    if (k > 0 && k - 1 < nb) {
+      const float4 u0 = *(const float4*)(co + 8 * (k - 1)), u1 = *(const float4*)(co + 8 * (k - 1) + 4);
+      const float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a = fmaf(u[e], x[8 * (k > 0 ? k - 1 : 0) + e], a);
+    }
+  }
+  const float va = (a + __shfl_xor_sync(0xffffffffu, a, 1)) * tau;
+  if (!on) return;
+  if (par == 0) p[0] = x0 - va;
+  coef_blocks<NB>(co, 0, nb, [&](int k, const float* u) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) q[2 * (8 * k + e) * st] = fmaf(-va, u[e], x[8 * k + e]);
+  });
+}
+
+template <class W, int NC>
+__global__ void __launch_bounds__(NC == 32 ? 128 : 2 * NC, NC == 128 ? 2 : (NC == 64 ? 6 : 8))
+    k_hess_real32(RealBatchT<float, W> bt, const int* __restrict__ order, const int* __restrict__ sched, int bin,
+                  int nmax) {
+  typedef float T;
+  // at least the four warps of the norm
+  constexpr int NT = 2 * NC < 128 ? 128 : 2 * NC, HC = NC / 2, NB = HC / 8;
+  extern __shared__ double smem_raw[];
+  __shared__ __align__(16) T ca[2][HC + 4];  // the reflector's odd and even entries, in different banks
+  __shared__ HessShared<T> sh;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int start = sched[3 * bin], end = sched[3 * bin + 1];
+  const int c = tid >> 1, par = tid & 1;
+  const int cw = c & ~15;  // the warp's first line
+  for (int job = start + blockIdx.x; job < end; job += gridDim.x) {
+    const int b = order[job];
+    const int n = bt.ns[b];
+    if (n <= 0 || n > nmax) continue;  // k_schur_real reports it
+    T* __restrict__ Ag = bt.A + bt.offs[b];
+    W* __restrict__ taus = bt.wi + bt.woffs[b];
+    const int ld = hess_ld32(n);
+    T* A = (T*)smem_raw;
+    __syncthreads();  // the previous matrix is out of shared memory
+    T amaxt = T(0);
+    for (int j = warp; j < n + kHessPad; j += NT / 32)
+      for (int i = lane; i < n + kHessPad; i += 32) {
+        const T a = (i < n && j < n) ? Ag[i + j * n] : T(0);
+        A[i + j * ld] = a;
+        const T aa = fabsf(a);
+        amaxt = (aa > amaxt || aa != aa) ? aa : amaxt;
+      }
+    const double amax = (double)block_max<NT>(amaxt, sh.red);
+    __syncthreads();
+    if (bt.scale)
+      hess_scale<T>(amax, [&](double f) {
+        for (int idx = tid; idx < n * n; idx += NT) {
+          T& a = A[idx % n + idx / n * ld];
+          a = (T)((double)a * f);
+        }
+      });
+    T x[HC];
+    for (int i = 1; i <= n - 2; ++i) {
+      const int m = n - i;                     // reflector length: rows i+1..n
+      T* col = A + i + (i - 1) * ld;           // col[0] = alpha, col[1..m-1] = x
+      // the first four warps: norm of the tail, the scalars (each for itself), the reflector
+      const T alpha = col[0];
+      const T xt = (tid < 128 && 1 + tid < m) ? col[1 + tid] : T(0);
+      if (warp < 4) {
+        T q = fmaf(xt, xt, T(0));
+        for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+        const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(xt)));
+        if (lane == 0) { sh.gmax[warp] = mb; sh.gssq[warp] = q; }
+      }
+      __syncthreads();
+      if (warp < 4) {
+        T tau, t, beta;
+        const int mode = hess_scalars(sh, alpha, tau, t, beta);
+        if (tid == 0) {
+          sh.c.mode = mode;
+          sh.c.tau = tau;
+          taus[i - 1] = (W)tau;
+          if (mode == 1) col[0] = beta;
+        }
+        if (mode == 1 && tid < NC) {
+          const T v = xt * t;
+          if (1 + tid < m) col[1 + tid] = v;
+          ca[tid & 1][tid >> 1] = v;
+        }
+      }
+      __syncthreads();
+      const int mode = sh.c.mode;
+      if (mode == 0) continue;
+      T tau = sh.c.tau;
+      if (mode == 2) {
+        T t, beta;
+        hess_reflector_guarded<T, NT>(col, m, sh, tau, t, beta);
+        if (tid < NC) {
+          const T v = (1 + tid < m) ? col[1 + tid] * t : T(0);
+          if (1 + tid < m) col[1 + tid] = v;
+          ca[tid & 1][tid >> 1] = v;
+        }
+        if (tid == 0) { col[0] = beta; taus[i - 1] = (W)tau; }
+        __syncthreads();
+      }
+      if (tau == T(0)) continue;
+      const int nb = (m / 2 + 7) / 8;  // of either parity: zeros beyond
+      // lmul!(H', A[i+1:n, i+1:n]): a column of A per pair of lanes
+      if (cw < m) hess_line32<NB>(A + i + (i + min(c, m - 1)) * ld, 1, par, nb, ca[par], tau, c < m, x);
+      __syncthreads();
+      // rmul!(A[:, i+1:n], H): a row of A per pair of lanes
+      if (cw < n) hess_line32<NB>(A + min(c, n - 1) + i * ld, ld, par, nb, ca[par], tau, c < n, x);
+      __syncthreads();
+    }
+    __syncthreads();
+    for (int j = warp; j < n; j += NT / 32)
+      for (int i = lane; i < n; i += 32) Ag[i + j * n] = A[i + j * ld];
+    if (tid == 0) bt.wr[bt.woffs[b]] = (W)amax;  // for the unscaling; k_schur_real overwrites it
+  }
+}
+
+// FP32 formation of Z (hessenberg.jl:150-166) from the reflectors that k_hess_real32 left in A and wi.
+// Z stays in registers from the identity to the end: a pair of neighbouring lanes holds a row, one lane
+// the even columns, the other the odd ones.  Two reflectors are staged in shared memory ahead, by
+// absolute column: cd with 0, cu with 1 at column i.
+template <class W, int NC>
+__global__ void __launch_bounds__(2 * NC, NC == 128 ? 2 : (NC == 64 ? 6 : 16))
+    k_formq_real32(RealBatchT<float, W> bt, const int* __restrict__ order, const int* __restrict__ sched, int bin,
+                   int nmax) {
+  typedef float T;
+  constexpr int HC = NC / 2, NB = HC / 8;
+  __shared__ __align__(16) T cd[2][2][HC + 4], cu[2][2][HC + 4];
+  __shared__ T taus[NC];
+  const int tid = threadIdx.x;
+  const int start = sched[3 * bin], end = sched[3 * bin + 1];
+  const int c = tid >> 1, par = tid & 1;
+  for (int job = start + blockIdx.x; job < end; job += gridDim.x) {
+    const int b = order[job];
+    const int n = bt.ns[b];
+    if (n <= 0 || n > nmax) continue;
+    const T* __restrict__ Ag = bt.A + bt.offs[b];
+    T* __restrict__ Zg = bt.Z + bt.offs[b];
+    if (tid < n) taus[tid] = (T)bt.wi[bt.woffs[b] + tid];
+    const bool zrow = (c & ~15) < n;
+    const int bz = ((n + 1) / 2 + 7) / 8;
+    T z[HC];  // Z(c, par + 2 e)
+#pragma unroll
+    for (int e = 0; e < HC; ++e) z[e] = (2 * e + par == c) ? T(1) : T(0);
+    T next = (tid < n && tid > 1 && n > 2) ? Ag[tid] : T(0);  // entry at absolute column tid of reflector 1
+    for (int i = 1; i <= n - 2; ++i) {
+      const int buf = i & 1;
+      if (tid < NC) {
+        const T v = tid > i ? next : T(0);
+        cd[buf][tid & 1][tid >> 1] = v;
+        cu[buf][tid & 1][tid >> 1] = tid == i ? T(1) : v;
+        next = (tid < n && tid > i + 1) ? Ag[tid + i * n] : T(0);
+      }
+      __syncthreads();  // the buffer of step i - 1 is rewritten after the next one
+      const T tau = taus[i - 1];
+      if (tau == T(0) || !zrow) continue;
+      const int b0 = i >> 4;         // of either parity
+      const bool own = par == (i & 1);  // this lane holds column i
+      T x0 = T(0);  // Z(c, i): cu - cd is 1 at column i, 0 elsewhere
+#pragma unroll
+      for (int k = 0; k < NB; ++k)
+        if (k == b0) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x0 = fmaf(cu[buf][par][8 * k + e] - cd[buf][par][8 * k + e], z[8 * k + e], x0);
+        }
+      x0 = __shfl_xor_sync(0xffffffffu, x0, 1);
+      T a = own ? T(0) : x0;
+      coef_blocks<NB>(cd[buf][par], b0, bz, [&](int k, const T* u) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a = fmaf(u[e], z[8 * k + e], a);
+      });
+      const T va = (a + __shfl_xor_sync(0xffffffffu, a, 1)) * tau;
+      coef_blocks<NB>(cu[buf][par], b0, bz, [&](int k, const T* u) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) z[8 * k + e] = fmaf(-va, u[e], z[8 * k + e]);
+      });
+    }
+    if (c < n) {
+#pragma unroll
+      for (int e = 0; e < HC; ++e)
+        if (2 * e + par < n) Zg[c + (2 * e + par) * n] = z[e];
+    }
+    __syncthreads();  // before the next matrix's reflectors
   }
 }
 
@@ -379,6 +609,16 @@ __device__ __forceinline__ void apply_line(T* p, int inc, int d, const T* lg, in
   *p1 = z1;
 }
 
+// Correctly rounded 1/d of a normal d whose reciprocal is normal: one Newton step on a seed within one
+// ulp, exact for every significand but all ones (P. Markstein, IBM J. Res. Dev. 34, 1990); the seed
+// of that one is exact enough too (all 2^23 significands compared with __frcp_rn).  28 cycles
+// against 79 for __frcp_rn with its range test.
+__device__ __forceinline__ float rcp_markstein(float d) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return fmaf(y, fmaf(-d, y, 1.0f), y);
+}
+
 // Reflector (householder.jl:12-54, as reflector_fast) of (a, x1, x2), x2 = 0 for a 2-element one;
 // a <- beta.  One test sends every case off the plain path to reflector_fast.
 __device__ __forceinline__ Refl<float> chain_refl(float& a, float x1, float x2, int nr, int) {
@@ -392,7 +632,7 @@ __device__ __forceinline__ Refl<float> chain_refl(float& a, float x1, float x2, 
   const float s = ss * y;
   const float aa = fabsf(a);
   const float tau = fmaf(aa, y, 1.0f);
-  const float t = copysignf(__frcp_rn(aa + s), a);
+  const float t = copysignf(rcp_markstein(aa + s), a);
   x1 *= t;
   x2 *= t;
   a = -copysignf(s, a);
@@ -533,7 +773,7 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
   W* __restrict__ wi = bt.wi + bt.woffs[b];
   T* logs = smem;
   T* H = smem + kLogElems;  // packed H
-  // the scale that k_hess_real applied
+  // the scale that the reduction applied
   const double amax = (double)wr[0];
   const double smlnum = sqrt((double)Prec<T>::fmin) / (double)Prec<T>::eps;
   const double bignum = 1.0 / smlnum;
@@ -856,8 +1096,9 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_schur_real(RealBatchT<T, W> bt
 // Dynamic shared memory of one CTA of the iteration for orders up to nmax: the reflector
 // log and the packed H.
 size_t bin_smem_elems(int nmax) { return kLogElems + (size_t)rpk(nmax + 1); }
-// ... of the reduction: the matrix, and Z where both fit.
+// ... of the reduction: FP64 the matrix, and Z where both fit; FP32 the padded matrix.
 size_t hess_smem_elems(int nmax, size_t tsize) {
+  if (tsize == 4) return (size_t)(nmax + kHessPad) * hess_ld32(nmax);
   const size_t one = (size_t)nmax * (nmax | 1), most = (kMaxDynSmem - 8 * 1024) / tsize;
   return 2 * one <= most ? 2 * one : (one > most ? one : most);
 }
@@ -866,14 +1107,30 @@ template <class T, class W, int NC>
 cudaError_t launch_hess(const RealBatchT<T, W>& bt, const int* order, const int* sched, int bin, int nmax,
                         int num_sms, cudaStream_t s) {
   const size_t elems = hess_smem_elems(nmax, sizeof(T)), smem = sizeof(T) * elems;
-  cudaError_t e = cudaFuncSetAttribute(k_hess_real<T, W, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr int NT = sizeof(T) == 8 ? 4 * NC : (2 * NC < 128 ? 128 : 2 * NC);
+  const void* f;
+  if constexpr (sizeof(T) == 8) f = (const void*)k_hess_real64<W, NC>;
+  else f = (const void*)k_hess_real32<W, NC>;
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hess_real<T, W, NC>, 4 * NC, smem);
+  auto grid = [&](const void* k, int nt, size_t sm) -> int {
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, sm)) != cudaSuccess) return 0;
+    const int ctas = num_sms * (per_sm < 1 ? 1 : per_sm);
+    return ctas < bt.count ? ctas : bt.count;
+  };
+  int ctas = grid(f, NT, smem);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
-  const int ctas = num_sms * per_sm < bt.count ? num_sms * per_sm : bt.count;
-  k_hess_real<T, W, NC><<<ctas, 4 * NC, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
+  if constexpr (sizeof(T) == 8) {
+    k_hess_real64<W, NC><<<ctas, NT, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
+  } else {
+    k_hess_real32<W, NC><<<ctas, NT, smem, s>>>(bt, order, sched, bin, nmax);
+    if (bt.wantz) {
+      ctas = grid((const void*)k_formq_real32<W, NC>, 2 * NC, 0);
+      if (e != cudaSuccess) return e;
+      k_formq_real32<W, NC><<<ctas, 2 * NC, 0, s>>>(bt, order, sched, bin, nmax);
+    }
+  }
   return cudaGetLastError();
 }
 
