@@ -524,7 +524,9 @@ __global__ void __launch_bounds__(2 * NC, NC == 128 ? 2 : (NC == 64 ? 6 : 16))
 //     rows: its first chunk is shortened, or the chain warp skips a phase.
 // The 2x2 blocks are standardised together at the end, a block per thread (GenericSchur.jl
 // standardises each as it deflates; the block, its eigenvalues and Z see the same operations,
-// entries above a block see its rotation after instead of before later sweeps' reflectors).
+// entries above a block see its rotation after instead of before later sweeps' reflectors).  The
+// windows of the FP32 large path (kInOrder), where such a rounding difference could change a later
+// decision, have the far warps standardise and rotate before the next chunk.
 //
 // Why: with one CTA barrier per chase step (the near block and the next reflector on one
 // warp, far updates on the others, the Z pass after each sweep), a step of an order-128 matrix took
@@ -536,6 +538,7 @@ struct Cmd {
   int n3;    // steps with a 3-element reflector
   int last2; // then a 2-element one
   int jfar;  // first column of the far left updates
+  int giv0, giv1;  // kInOrder: the pairs to standardise before the chunk
 };
 
 constexpr int kWin = 28;    // most steps of a chunk (kWin + 3 columns, kWin + 3 rows in a warp's lanes)
@@ -556,6 +559,8 @@ template <> __device__ __forceinline__ Refl<double> ld_refl<double>(const double
 
 // The phase barrier: the chain warp and the far warps meet it at different places of the code.
 template <int NT> __device__ __forceinline__ void phase_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); }
+
+template <int NT> __device__ __forceinline__ void far_barrier() { asm volatile("bar.sync 2, %0;" ::"n"(NT - 32) : "memory"); }
 
 // One 3-element reflector on (z0, z1, z2): returns the finished first element.
 template <class T>
@@ -751,15 +756,44 @@ __device__ __forceinline__ void chase_chunk(T* H, int ka, int nst, int iend, int
   __syncwarp();
 }
 
+// Rotation of a standardised block at (p, p+1): rmul!(HH[1:p-1, :], G') and Z, lmul!(G, HH[:, p+2:n]),
+// thread t of nt.
+template <class T>
+__device__ __forceinline__ void rotate_cols(T* H, int n, int p, T cs, T sn, int t, int nt, T* Zg) {
+  for (int i = 1 + t; i <= p - 1; i += nt) {
+    const T a1 = HH(i, p), a2 = HH(i, p + 1);
+    HH(i, p) = cs * a1 + sn * a2;
+    HH(i, p + 1) = -sn * a1 + cs * a2;
+  }
+  if (Zg)
+    for (int i = t; i < n; i += nt) {
+      T* zp = Zg + i + (long long)(p - 1) * n;
+      const T a1 = zp[0], a2 = zp[n];
+      zp[0] = cs * a1 + sn * a2;
+      zp[n] = -sn * a1 + cs * a2;
+    }
+}
+template <class T>
+__device__ __forceinline__ void rotate_rows(T* H, int n, int p, T cs, T sn, int t, int nt) {
+  for (int j = p + 2 + t; j <= n; j += nt) {
+    const T a1 = HH(p, j), a2 = HH(p + 1, j);
+    HH(p, j) = cs * a1 + sn * a2;
+    HH(p + 1, j) = -sn * a1 + cs * a2;
+  }
+}
+
 // nmax: the largest order the launch sized shared memory for.  Orders come from device
 // memory (GS_DEVICE calls are not checked on the host), so an order outside [0, nmax]
 // gets ST_BADARG before anything is read or written.
 template <class T, class W, int NT>
 __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem, int cw) {
   __shared__ Cmd<T> cmd[2];
-  __shared__ int s_status, s_iend, s_npair;
+  __shared__ int s_status, s_npair;
   __shared__ int pairs[kSmallMax / 2];
   __shared__ T gcs[kSmallMax / 2], gsn[kSmallMax / 2];
+  __shared__ T blks[kSmallMax * 2];  // kInOrder: the standardised blocks
+  constexpr bool kInOrder = sizeof(T) == 4 && sizeof(W) == 8;
+  __shared__ int s_giv;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const int n = bt.ns[b];
@@ -794,7 +828,7 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
     // ---- chain warp (all its variables are uniform over the lanes) ----
     const long long maxiter = bt.maxiter_abs > 0 ? bt.maxiter_abs : (long long)bt.maxiter_mult * n;
     long long iter = 0;
-    int status = ST_OK, iend = n, istart = 1, iterqr = 0, npair = 0;
+    int status = ST_OK, iend = n, istart = 1, iterqr = 0, npair = 0, ngiv = 0;
     int state = 0;             // 0: between sweeps, 1: first chunk of a sweep is next, 2: inside a sweep
     int kn = 0;                // next step
     int pka = 0, pn3 = 0, pwl = 0;  // previous chunk of this sweep
@@ -963,7 +997,10 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
             cm.n3 = last ? nst - 1 : nst;
             cm.last2 = last;
             cm.jfar = jfar;
+            cm.giv0 = ngiv;
+            cm.giv1 = npair;
           }
+          ngiv = npair;
           type = 1;
           pka = kn; pn3 = nst; pwl = wl;
           kn = kb + 1;
@@ -977,7 +1014,7 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
       phase_barrier<NT>();
       if (done) break;
     }
-    if (lane == 0) { s_status = status; s_iend = iend; s_npair = npair; }
+    if (lane == 0) { s_status = status; s_giv = kInOrder ? ngiv : 0; s_npair = npair; }
   } else {
     // ---- far warps ----
     const int ft = tid - (warp > cw ? 32 : 0);
@@ -986,6 +1023,20 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
         const Cmd<T> cm = cmd[(ph - 1) & 1];
         const T* lg = logs + ((ph - 1) & 1) * (kLogElems / 2);
         const int ka = cm.ka;
+        if constexpr (kInOrder) {
+          for (int q = cm.giv0; q < cm.giv1; ++q) {
+            const int p = pairs[q];
+            double a = HH(p, p), bq = HH(p, p + 1), cc = HH(p + 1, p), d = HH(p + 1, p + 1), cs, sn, w1r, w1i, w2r, w2i;
+            gs2x2(a, bq, cc, d, cs, sn, w1r, w1i, w2r, w2i);
+            rotate_cols(H, n, p, (T)cs, (T)sn, ft, NT - 32, Zg);
+            rotate_rows(H, n, p, (T)cs, (T)sn, ft, NT - 32);
+            if (ft == 0) {
+              wr[p] = (W)w2r; wi[p] = (W)w2i; wr[p - 1] = (W)w1r; wi[p - 1] = (W)w1i;
+              blks[4 * q] = (T)a; blks[4 * q + 1] = (T)bq; blks[4 * q + 2] = (T)cc; blks[4 * q + 3] = (T)d;
+            }
+            far_barrier<NT>();
+          }
+        }
         const int nl = n - cm.jfar + 1, nr = max(ka - 2, 0), nz = Zg ? n : 0;
         for (int t = ft; t < nl + nr + nz; t += NT - 32) {
           T* p;
@@ -1011,8 +1062,15 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
   __syncthreads();
   const int status = s_status, npair = s_npair;
 
-  // ---- standardise the 2x2 blocks (GenericSchur.jl:667-690) ----
-  for (int q = tid; q < npair; q += NT) {
+  // ---- standardise the (remaining) 2x2 blocks (GenericSchur.jl:667-690) ----
+  const int g0 = s_giv;
+  if constexpr (kInOrder)
+    for (int q = tid; q < g0; q += NT) {
+      const int p = pairs[q];
+      HH(p, p) = blks[4 * q]; HH(p, p + 1) = blks[4 * q + 1];
+      HH(p + 1, p) = blks[4 * q + 2]; HH(p + 1, p + 1) = blks[4 * q + 3];
+    }
+  for (int q = g0 + tid; q < npair; q += NT) {
     const int p = pairs[q];
     double a = HH(p, p), bq = HH(p, p + 1), cc = HH(p + 1, p), d = HH(p + 1, p + 1), cs, sn, w1r, w1i, w2r, w2i;
     gs2x2(a, bq, cc, d, cs, sn, w1r, w1i, w2r, w2i);
@@ -1021,32 +1079,9 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
     HH(p, p) = (T)a; HH(p, p + 1) = (T)bq; HH(p + 1, p) = (T)cc; HH(p + 1, p + 1) = (T)d;
   }
   __syncthreads();
-  for (int q = warp; q < npair; q += NT / 32) {  // rmul!(HH[1:p-1, :], G') and Z
-    const int p = pairs[q];
-    const T cs = gcs[q], sn = gsn[q];
-    for (int i = 1 + lane; i <= p - 1; i += 32) {
-      const T a1 = HH(i, p), a2 = HH(i, p + 1);
-      HH(i, p) = cs * a1 + sn * a2;
-      HH(i, p + 1) = -sn * a1 + cs * a2;
-    }
-    if (Zg)
-      for (int i = lane; i < n; i += 32) {
-        T* zp = Zg + i + (long long)(p - 1) * n;
-        const T a1 = zp[0], a2 = zp[n];
-        zp[0] = cs * a1 + sn * a2;
-        zp[n] = -sn * a1 + cs * a2;
-      }
-  }
+  for (int q = g0 + warp; q < npair; q += NT / 32) rotate_cols(H, n, pairs[q], gcs[q], gsn[q], lane, 32, Zg);
   __syncthreads();
-  for (int q = warp; q < npair; q += NT / 32) {  // lmul!(G, HH[:, p+2:n])
-    const int p = pairs[q];
-    const T cs = gcs[q], sn = gsn[q];
-    for (int j = p + 2 + lane; j <= n; j += 32) {
-      const T a1 = HH(p, j), a2 = HH(p + 1, j);
-      HH(p, j) = cs * a1 + sn * a2;
-      HH(p + 1, j) = -sn * a1 + cs * a2;
-    }
-  }
+  for (int q = g0 + warp; q < npair; q += NT / 32) rotate_rows(H, n, pairs[q], gcs[q], gsn[q], lane, 32);
   __syncthreads();
 
   // ---- write back ----
