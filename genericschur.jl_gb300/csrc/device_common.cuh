@@ -12,6 +12,15 @@ constexpr double kEps = 2.220446049250313e-16;       // eps(Float64) = 2^-52
 constexpr double kFmin = 2.2250738585072014e-308;    // floatmin(Float64)
 constexpr double kSafemin = 2.2250738585072014e-308; // safemin(Float64) (util.jl:5-12)
 
+// One element from global to shared memory without waiting (4, 8 or 16 bytes); async_wait before use.
+template <class T>
+__device__ __forceinline__ void async_load(T* sm, const T* g) {
+  static_assert(sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16, "cp.async sizes");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(sm)), "l"(g),
+               "n"((int)sizeof(T)));
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Block reductions over the whole CTA.  `red` is shared scratch of >= 32 entries.
 template <int NT, class V>
 __device__ __forceinline__ V block_max(V v, V* red) {

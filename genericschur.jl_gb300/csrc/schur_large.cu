@@ -61,7 +61,8 @@ __global__ void __launch_bounds__(32 * kChaseWarps) k_chase_chunk(ChaseArgs<T> c
   const int n = ca.n, B = ca.B;
   T* H = ca.H;
   for (int j = warp; j < nw; j += kChaseWarps)
-    for (int i = lane; i < nw; i += 32) W[i + j * ldw] = H[(size_t)(ca.wlo - 1 + j) * n + (ca.wlo - 1 + i)];
+    for (int i = lane; i < nw; i += 32) async_load(&W[i + j * ldw], &H[(size_t)(ca.wlo - 1 + j) * n + (ca.wlo - 1 + i)]);
+  async_wait();
   __syncthreads();
 #define WW(i, j) W[((i) - ca.wlo) + ((j) - ca.wlo) * ldw]
   // reflector of bulge `lane` at sweep step ca.t0 + s (warp 0)
@@ -181,17 +182,18 @@ __global__ void __launch_bounds__(256) k_chase_far(ChaseArgs<T> ca, int nleft, i
   T* seg = (T*)(lk + (((size_t)steps * ca.B + 1) & ~size_t(1)));  // segment
   const int tid = threadIdx.x;
   const int n = ca.n;
-  for (int idx = tid; idx < steps * ca.B * 5; idx += blockDim.x) lr[idx] = ca.logr[idx];
-  for (int idx = tid; idx < steps * ca.B; idx += blockDim.x) lk[idx] = ca.logk[idx];
+  const int lane = tid & 31, warp = tid >> 5;  // 8 warps
+  static_assert(kFarTile == 32, "a tile's rows are a warp's lanes");
+  for (int idx = tid; idx < steps * ca.B * 5; idx += blockDim.x) async_load(&lr[idx], &ca.logr[idx]);
+  for (int idx = tid; idx < steps * ca.B; idx += blockDim.x) async_load(&lk[idx], &ca.logk[idx]);
   int tile = blockIdx.x;
   if (tile < nleft) {
     // columns c0.. c0+kFarTile-1 right of the window, rows wlo..whi: segment[nw][kFarTile]
     const int c0 = ca.whi + 1 + tile * kFarTile;
     const int nc = min(kFarTile, n - c0 + 1);
-    for (int idx = tid; idx < nw * kFarTile; idx += blockDim.x) {
-      const int i = idx % nw, c = idx / nw;
-      seg[i + c * nw] = (c < nc) ? ca.H[(size_t)(c0 - 1 + c) * n + (ca.wlo - 1 + i)] : T(0);
-    }
+    for (int c = warp; c < nc; c += 8)
+      for (int i = lane; i < nw; i += 32) async_load(&seg[i + c * nw], &ca.H[(size_t)(c0 - 1 + c) * n + (ca.wlo - 1 + i)]);
+    async_wait();
     __syncthreads();
     for (int s = 0; s < steps; ++s) {
       for (int idx = tid; idx < ca.B * kFarTile; idx += blockDim.x) {
@@ -208,10 +210,8 @@ __global__ void __launch_bounds__(256) k_chase_far(ChaseArgs<T> ca, int nleft, i
       }
       __syncthreads();
     }
-    for (int idx = tid; idx < nw * kFarTile; idx += blockDim.x) {
-      const int i = idx % nw, c = idx / nw;
-      if (c < nc) ca.H[(size_t)(c0 - 1 + c) * n + (ca.wlo - 1 + i)] = seg[i + c * nw];
-    }
+    for (int c = warp; c < nc; c += 8)
+      for (int i = lane; i < nw; i += 32) ca.H[(size_t)(c0 - 1 + c) * n + (ca.wlo - 1 + i)] = seg[i + c * nw];
     return;
   }
   tile -= nleft;
@@ -228,10 +228,9 @@ __global__ void __launch_bounds__(256) k_chase_far(ChaseArgs<T> ca, int nleft, i
     nrw = min(kFarTile, n - r0 + 1);
   }
   // rows r0..r0+nrw-1, columns wlo..whi: segment[kFarTile][nw] (row index fastest)
-  for (int idx = tid; idx < kFarTile * nw; idx += blockDim.x) {
-    const int i = idx % kFarTile, j = idx / kFarTile;
-    seg[i + j * kFarTile] = (i < nrw) ? M[(size_t)(ca.wlo - 1 + j) * n + (r0 - 1 + i)] : T(0);
-  }
+  if (lane < nrw)
+    for (int j = warp; j < nw; j += 8) async_load(&seg[lane + j * kFarTile], &M[(size_t)(ca.wlo - 1 + j) * n + (r0 - 1 + lane)]);
+  async_wait();
   __syncthreads();
   for (int s = 0; s < steps; ++s) {
     for (int idx = tid; idx < ca.B * kFarTile; idx += blockDim.x) {

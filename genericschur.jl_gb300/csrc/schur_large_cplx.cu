@@ -202,84 +202,104 @@ struct ZChase {
 // One chunk of the chain's chase inside the window [wlo, whi] (shared memory).  At sweep
 // step t bulge b sits at k = ilo + t - 2b.
 __global__ void __launch_bounds__(256) k_zchase_chunk(ZChase ca) {
+  // the pairing of bulges and the overlap as in k_chase_chunk (schur_large.cu)
   extern __shared__ double2 W[];
+  constexpr int kWarps = 8;
   const int nw = ca.whi - ca.wlo + 1;
   const int ldw = nw;
-  __shared__ double2 rf[kZMaxB][3];
-  __shared__ int rk[kZMaxB];
-  const int tid = threadIdx.x;
-  const int n = ca.n;
-  for (int idx = tid; idx < nw * nw; idx += blockDim.x) {
-    const int i = idx % nw, j = idx / nw;
-    W[i + j * ldw] = ca.H[(size_t)(ca.wlo - 1 + j) * n + (ca.wlo - 1 + i)];
-  }
+  struct Rf {
+    double2 tau, v2, t2;
+    int k;  // position (0: inactive)
+  };
+  __shared__ Rf rf[2][kZMaxB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = ca.n, B = ca.B;
+  for (int j = warp; j < nw; j += kWarps)
+    for (int i = lane; i < nw; i += 32) async_load(&W[i + j * ldw], &ca.H[(size_t)(ca.wlo - 1 + j) * n + (ca.wlo - 1 + i)]);
+  async_wait();
   __syncthreads();
 #define WW(i, j) W[((i) - ca.wlo) + ((j) - ca.wlo) * ldw]
-  for (int s = 0; s < ca.w; ++s) {
-    const int t = ca.t0 + s;
-    if (tid < ca.B) {
-      const int b = tid;
-      const int k = ca.ilo + t - 2 * b;
-      double2 tau = zc(0.0), v2 = zc(0.0);
-      const bool on = k >= ca.ilo && k <= ca.ihi - 1;
-      if (on) {
-        double2 a, x1;
-        if (k == ca.ilo) {
-          // start vector of the shift (GenericSchur.jl:409-414 at m = istart), scaled
-          a = zsub(WW(k, k), ca.shifts[b]);
-          x1 = WW(k + 1, k);
-          const double sn = zabs1(a) + zabs1(x1);
-          if (sn != 0.0) { a = zscal(a, 1.0 / sn); x1 = zscal(x1, 1.0 / sn); }
-        } else {
-          a = WW(k, k - 1);
-          x1 = WW(k + 1, k - 1);
-        }
-        tau = zreflector2_fast(a, x1);
-        v2 = x1;
-        if (k > ca.ilo) {
-          WW(k, k - 1) = a;
-          WW(k + 1, k - 1) = zc(0.0);
-        }
+  // reflector of bulge `lane` at sweep step ca.t0 + s (warp 0)
+  auto reflectors = [&](int s) {
+    const int b = lane, k = ca.ilo + ca.t0 + s - 2 * b;
+    if (b >= B) return;
+    double2 tau = zc(0.0), v2 = zc(0.0);
+    const bool on = k >= ca.ilo && k <= ca.ihi - 1;
+    if (on) {
+      double2 a, x1;
+      if (k == ca.ilo) {
+        // start vector of the shift (GenericSchur.jl:409-414 at m = istart), scaled
+        a = zsub(WW(k, k), ca.shifts[b]);
+        x1 = WW(k + 1, k);
+        const double sn = zabs1(a) + zabs1(x1);
+        if (sn != 0.0) { a = zscal(a, 1.0 / sn); x1 = zscal(x1, 1.0 / sn); }
+      } else {
+        a = WW(k, k - 1);
+        x1 = WW(k + 1, k - 1);
       }
-      rk[b] = on ? k : 0;
-      rf[b][0] = tau;
-      rf[b][1] = v2;
-      rf[b][2] = zmul(tau, v2);
-      const size_t li = (size_t)s * ca.B + b;
-      ca.logk[li] = on ? k : 0;
-      ca.logr[3 * li + 0] = tau;
-      ca.logr[3 * li + 1] = v2;
-      ca.logr[3 * li + 2] = rf[b][2];
+      tau = zreflector2_fast(a, x1);
+      v2 = x1;
+      if (k > ca.ilo) {
+        WW(k, k - 1) = a;
+        WW(k + 1, k - 1) = zc(0.0);
+      }
     }
-    __syncthreads();
+    const double2 t2 = zmul(tau, v2);
+    rf[s & 1][b] = Rf{tau, v2, t2, on ? k : 0};
+    const size_t li = (size_t)s * B + b;
+    ca.logk[li] = on ? k : 0;
+    ca.logr[3 * li + 0] = tau;
+    ca.logr[3 * li + 1] = v2;
+    ca.logr[3 * li + 2] = t2;
+  };
+  auto right = [&](const Rf& r, int i) {
+    const double2 h0 = WW(i, r.k), h1 = WW(i, r.k + 1);
+    const double2 ss = zadd(zmul(r.tau, h0), zmul(r.t2, h1));
+    WW(i, r.k) = zsub(h0, ss);
+    WW(i, r.k + 1) = zfms(ss, zconj(r.v2), h1);
+  };
+  if (warp == 0) reflectors(0);
+  __syncthreads();
+  const int npair = (B + 1) / 2;
+  for (int s = 0; s < ca.w; ++s) {
+    const Rf* rs = rf[s & 1];
     // left (P^H from the left) inside the window: bulge b, columns j >= k_b
-    for (int idx = tid; idx < ca.B * nw; idx += blockDim.x) {
-      const int b = idx / nw, j = ca.wlo + idx % nw;
-      const int k = rk[b];
-      if (!k || j < k) continue;
-      const double2 h0 = WW(k, j), h1 = WW(k + 1, j);
-      const double2 ss = zadd(zmul(zconj(rf[b][0]), h0), zmul(zconj(rf[b][2]), h1));
-      WW(k, j) = zsub(h0, ss);
-      WW(k + 1, j) = zfms(ss, rf[b][1], h1);
+    for (int p = warp; p < npair; p += kWarps) {
+      const int q = B - 1 - p;
+      const int kp = rs[p].k, kq = rs[q].k;
+      const int np = kp ? ca.whi - kp + 1 : 0, nq = (q != p && kq) ? ca.whi - kq + 1 : 0;
+      for (int t = lane; t < np + nq; t += 32) {
+        const Rf& r = rs[t < np ? p : q];
+        const int j = r.k + (t < np ? t : t - np);
+        const double2 h0 = WW(r.k, j), h1 = WW(r.k + 1, j);
+        const double2 ss = zadd(zmul(zconj(r.tau), h0), zmul(zconj(r.t2), h1));
+        WW(r.k, j) = zsub(h0, ss);
+        WW(r.k + 1, j) = zfms(ss, r.v2, h1);
+      }
     }
     __syncthreads();
     // right (P from the right) inside the window: bulge b, rows i <= min(k_b + 2, ihi)
-    for (int idx = tid; idx < ca.B * nw; idx += blockDim.x) {
-      const int b = idx / nw, i = ca.wlo + idx % nw;
-      const int k = rk[b];
-      if (!k || i > min(k + 2, ca.ihi)) continue;
-      const double2 h0 = WW(i, k), h1 = WW(i, k + 1);
-      const double2 ss = zadd(zmul(rf[b][0], h0), zmul(rf[b][2], h1));
-      WW(i, k) = zsub(h0, ss);
-      WW(i, k + 1) = zfms(ss, zconj(rf[b][1]), h1);
+    if (warp == 0) {
+      for (int t = lane; t < 4 * B; t += 32) {
+        const Rf& r = rs[t >> 2];
+        const int i = r.k + (t & 3);
+        if (r.k && (t & 3) < 3 && i <= ca.ihi) right(r, i);
+      }
+      __syncwarp();
+      if (s + 1 < ca.w) reflectors(s + 1);
+    } else {
+      for (int p = warp - 1; p < npair; p += kWarps - 1) {
+        const int q = B - 1 - p;
+        const int kp = rs[p].k, kq = rs[q].k;
+        const int np = kp ? kp - ca.wlo : 0, nq = (q != p && kq) ? kq - ca.wlo : 0;
+        for (int t = lane; t < np + nq; t += 32) right(rs[t < np ? p : q], ca.wlo + (t < np ? t : t - np));
+      }
     }
     __syncthreads();
   }
 #undef WW
-  for (int idx = tid; idx < nw * nw; idx += blockDim.x) {
-    const int i = idx % nw, j = idx / nw;
-    ca.H[(size_t)(ca.wlo - 1 + j) * n + (ca.wlo - 1 + i)] = W[i + j * ldw];
-  }
+  for (int j = warp; j < nw; j += kWarps)
+    for (int i = lane; i < nw; i += 32) ca.H[(size_t)(ca.wlo - 1 + j) * n + (ca.wlo - 1 + i)] = W[i + j * ldw];
 }
 
 // Far updates of one chunk: tiles of columns right of the window (left updates on rows
@@ -294,16 +314,16 @@ __global__ void __launch_bounds__(256) k_zchase_far(ZChase ca, int nleft, int nr
   int* lk = (int*)(seg + (size_t)nw * kZFarTile);      // steps*B
   const int tid = threadIdx.x;
   const int n = ca.n;
-  for (int idx = tid; idx < steps * B * 3; idx += blockDim.x) lr[idx] = ca.logr[idx];
-  for (int idx = tid; idx < steps * B; idx += blockDim.x) lk[idx] = ca.logk[idx];
+  const int lane = tid & 31, warp = tid >> 5;  // 8 warps
+  for (int idx = tid; idx < steps * B * 3; idx += blockDim.x) async_load(&lr[idx], &ca.logr[idx]);
+  for (int idx = tid; idx < steps * B; idx += blockDim.x) async_load(&lk[idx], &ca.logk[idx]);
   int tile = blockIdx.x;
   if (tile < nleft) {
     const int c0 = ca.whi + 1 + tile * kZFarTile;
     const int nc = min(kZFarTile, n - c0 + 1);
-    for (int idx = tid; idx < nw * kZFarTile; idx += blockDim.x) {
-      const int i = idx % nw, c = idx / nw;
-      seg[i + c * nw] = (c < nc) ? ca.H[(size_t)(c0 - 1 + c) * n + (ca.wlo - 1 + i)] : zc(0.0);
-    }
+    for (int c = warp; c < nc; c += 8)
+      for (int i = lane; i < nw; i += 32) async_load(&seg[i + c * nw], &ca.H[(size_t)(c0 - 1 + c) * n + (ca.wlo - 1 + i)]);
+    async_wait();
     __syncthreads();
     for (int s = 0; s < steps; ++s) {
       for (int idx = tid; idx < B * kZFarTile; idx += blockDim.x) {
@@ -318,10 +338,8 @@ __global__ void __launch_bounds__(256) k_zchase_far(ZChase ca, int nleft, int nr
       }
       __syncthreads();
     }
-    for (int idx = tid; idx < nw * kZFarTile; idx += blockDim.x) {
-      const int i = idx % nw, c = idx / nw;
-      if (c < nc) ca.H[(size_t)(c0 - 1 + c) * n + (ca.wlo - 1 + i)] = seg[i + c * nw];
-    }
+    for (int c = warp; c < nc; c += 8)
+      for (int i = lane; i < nw; i += 32) ca.H[(size_t)(c0 - 1 + c) * n + (ca.wlo - 1 + i)] = seg[i + c * nw];
     return;
   }
   tile -= nleft;
@@ -339,8 +357,9 @@ __global__ void __launch_bounds__(256) k_zchase_far(ZChase ca, int nleft, int nr
   }
   for (int idx = tid; idx < kZFarTile * nw; idx += blockDim.x) {
     const int i = idx % kZFarTile, j = idx / kZFarTile;
-    seg[i + j * kZFarTile] = (i < nrw) ? M[(size_t)(ca.wlo - 1 + j) * n + (r0 - 1 + i)] : zc(0.0);
+    if (i < nrw) async_load(&seg[i + j * kZFarTile], &M[(size_t)(ca.wlo - 1 + j) * n + (r0 - 1 + i)]);
   }
+  async_wait();
   __syncthreads();
   for (int s = 0; s < steps; ++s) {
     for (int idx = tid; idx < B * kZFarTile; idx += blockDim.x) {
