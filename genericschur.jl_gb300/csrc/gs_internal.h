@@ -178,6 +178,7 @@ struct QzrBatch {
   int* status;
   int scale;
   int n1;
+  int nmax;                // the largest order (0: unknown)
 };
 cudaError_t launch_ggschur_real(const QzrBatch& bt, int num_sms, cudaStream_t s);
 

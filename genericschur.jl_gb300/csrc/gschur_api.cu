@@ -3327,6 +3327,9 @@ int ggschur_real_impl(gs_context* ctx, int64_t count, const int32_t* ns, const i
   bt.count = (int)count;
   bt.scale = (flags & GS_SCALE) ? 1 : 0;
   bt.n1 = single;
+  bt.nmax = single;
+  if (!single && !dev)
+    for (int64_t b = 0; b < count; ++b) bt.nmax = std::max(bt.nmax, (int)ns[b]);
   if (dev) {
     bt.ns = single ? nullptr : ns;
     bt.offs = (const long long*)offs;

@@ -5,11 +5,18 @@
 // _gsvd_2x2 / dlasv2 and evaluated with _ggs_2x2 / dlag2).  S = Q^T A Z is quasi-triangular,
 // T = Q^T B Z upper triangular with a non-negative diagonal.
 //
-// One CTA per pencil (a ragged batch or a batch of one), the matrices in global memory
-// (L2-resident at the orders this path serves).  Every thread runs the reference's scalar
-// control flow on the same data -- shift, Givens and reflector computations, deflation
-// tests -- so all threads take the same branches; thread 0 alone writes scalar entries
-// (between barriers), and the row / column updates of H, B, Q, Z are split over the CTA.
+// One CTA per pencil (a ragged batch or a batch of one), H, B, Q, Z in shared memory up to order 82, H
+// and B up to 117, in global memory (L2-resident at the orders this path serves) above.  Between
+// the sweeps every thread runs the reference's scalar control flow on the same data --
+// shifts, deflation tests -- so all threads take the same branches; thread 0 alone writes scalar
+// entries (between barriers).  In the sweeps and in the Hessenberg-triangular reduction warp 0 (the
+// chain warp) computes the rotations and reflectors, one after the other, from the few entries
+// around the diagonal that they depend on, while the other warps apply the left transformation of this
+// step and the right one of the step before to the rest of H, B and to Q, Z: one barrier per step.
+// Bound: the FP64 latency of the chain (about 5,000 cycles for a double-shift step: two square
+// roots, a hypotenuse, nine dependent quotients and products); independent quotients share an
+// instruction on different lanes.  With the matrices in global memory and the scalars on
+// all warps, then all updates, behind four to six barriers, 64 pencils of orders 9..65 took 43.9 ms.
 #include <algorithm>
 
 #include "device_common.cuh"
@@ -20,8 +27,8 @@ namespace {
 
 constexpr int kQrT = 128;
 
-#define HH(i, j) H[((i) - 1) + (size_t)((j) - 1) * n]
-#define BB(i, j) B[((i) - 1) + (size_t)((j) - 1) * n]
+#define HH(i, j) H[((i) - 1) + (size_t)((j) - 1) * ld]
+#define BB(i, j) B[((i) - 1) + (size_t)((j) - 1) * ld]
 #define SYNC() __syncthreads()
 
 // Julia's Givens(i1, i2, c, s) on the CTA: lmul! rows (columns j0..j1), rmul!(M, G) and
@@ -33,15 +40,6 @@ __device__ void crows(double* M, int n, int i1, int i2, double c, double s, int 
     const double x = *p1, y = *p2;
     *p1 = c * x + s * y;
     *p2 = c * y - s * x;
-  }
-}
-__device__ void ccols(double* M, int n, int i1, int i2, double c, double s, int r0, int r1) {
-  double* c1 = M + (size_t)(i1 - 1) * n;
-  double* c2 = M + (size_t)(i2 - 1) * n;
-  for (int r = r0 - 1 + (int)threadIdx.x; r <= r1 - 1; r += kQrT) {
-    const double x = c1[r], y = c2[r];
-    c1[r] = x * c - y * s;
-    c2[r] = x * s + y * c;
   }
 }
 __device__ void ccols_adj(double* M, int n, int i1, int i2, double c, double s, int r0, int r1) {
@@ -111,7 +109,7 @@ __device__ double refl3(double& a, double& x1, double& x2) {
 }
 
 // dlag2 (rgeneralized.jl:810-948) on the 2 x 2 pencil at (i, i) of H, B.
-__device__ void ggs2x2(const double* H, const double* B, int n, int i, double safmin, double& scale1, double& scale2,
+__device__ void ggs2x2(const double* H, const double* B, int ld, int i, double safmin, double& scale1, double& scale2,
                        double& wr1, double& wr2, double& wi) {
   const double rtmin = sqrt(safmin), rtmax = 1.0 / rtmin, safmax = 1.0 / safmin;
   const double fuzzy1 = 1.0 + sqrt(sqrt(Prec<double>::eps)) / 10.0;
@@ -280,18 +278,158 @@ __device__ void gsvd2x2(double f0, double g0, double h0, double& ssmin, double& 
   ssmin = copysign(ssmin, tsgn * copysign(1.0, f0) * copysign(1.0, h0));
 }
 
-// 2-norm of all n x n entries (Frobenius) without overflow.
-__device__ double cta_fro_real(const double* M, int n, double* red) {
-  return cta_norm2<double, kQrT>(M, n * n, red);
+// 2-norm of all n x n entries (Frobenius) without overflow: cta_norm2 of the packed entries.
+__device__ double cta_fro_real(const double* M, int n, int ld, double* red) {
+  double mx = 0.0;
+  for (int k = threadIdx.x; k < n * n; k += kQrT) mx = fmax(mx, fabs(M[k % n + (size_t)(k / n) * ld]));
+  mx = block_max<kQrT>(mx, red);
+  if (!(mx > 0.0) || !isfinite(mx)) return mx;
+  const double inv = 1.0 / mx;
+  double ss = 0.0;
+  for (int k = threadIdx.x; k < n * n; k += kQrT) ss += comp_ssq(M[k % n + (size_t)(k / n) * ld], inv);
+  ss = block_sum<kQrT>(ss, red);
+  return mx * sqrt(ss);
 }
 
-// _gqz! (rgeneralized.jl:68-808), ilo = 1, ihi = n, wantSchur; returns 0 or 1.
-__device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, double2* alpha, double* beta,
+// Quotients of a warp's lanes 0, 1, 2: one division.
+__device__ __forceinline__ double lane_get(double v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+
+// givens_alg for two problems at once: lanes with an even number hold one (f, g), those with an odd
+// number the other; all lanes of a warp call it.
+__device__ __forceinline__ void givens_lanes(double f, double g, double& cs, double& sn, double& r) {
+  const int lane = threadIdx.x & 31;
+  const double scale = fmax(fabs(f), fabs(g));
+  const bool plain = f != 0.0 && g != 0.0 && scale < 0x1p485 && scale > 0x1p-485;
+  if (!__all_sync(0xffffffffu, plain)) {
+    givens_alg(f, g, cs, sn, r);
+    return;
+  }
+  double rr = sqrt(f * f + g * g);
+  const double v = ((lane & 2) ? g : f) / rr;
+  cs = lane_get(v, lane & 1);
+  sn = lane_get(v, (lane & 1) | 2);
+  if (fabs(f) > fabs(g) && cs < 0.0) { cs = -cs; sn = -sn; rr = -rr; }
+  r = rr;
+}
+
+// refl3 with its quotients on different lanes; all lanes of a warp call it with the same values.
+__device__ __forceinline__ double refl3_lanes(double& a, double& x1, double& x2) {
+  const int lane = threadIdx.x & 31;
+  const double m = fmax(fabs(x1), fabs(x2));
+  const double sfmin = 2.0 * Prec<double>::fmin / Prec<double>::eps;
+  if (!(m > 0.0) || !isfinite(m)) return refl3(a, x1, x2);
+  const double pq = ((lane & 1) ? x2 : x1) / m;
+  const double p = lane_get(pq, 0), q = lane_get(pq, 1);
+  const double xnorm = m * sqrt(p * p + q * q);
+  const double beta = -copysign(hypot(a, xnorm), a);
+  if (xnorm == 0.0 || !(fabs(beta) >= sfmin)) return refl3(a, x1, x2);
+  const double v = ((lane & 1) ? 1.0 : (beta - a)) / ((lane & 1) ? (a - beta) : beta);
+  const double t = lane_get(v, 1);
+  x1 *= t;
+  x2 *= t;
+  a = beta;
+  return lane_get(v, 0);
+}
+
+// A left (rows j, j+1[, j+2]) and a right (columns j, j+1[, j+2]) transformation of a step.
+struct QzrStep {
+  double l0, l1, l2;  // left: tau, v1, v2 or c, s
+  double r0, r1, r2;  // right
+};
+
+// Three rows / columns against the reflector 1, v1, v2 with tau, at distance st.
+__device__ __forceinline__ void qz_left3(double* p, double tau, double v1, double v2) {
+  const double t2 = tau * v1, t3 = tau * v2;
+  const double t1 = p[0] + v1 * p[1] + v2 * p[2];
+  p[0] -= t1 * tau;
+  p[1] -= t1 * t2;
+  p[2] -= t1 * t3;
+}
+__device__ __forceinline__ void qz_right3(double* p, size_t st, double tau, double v1, double v2) {
+  const double t2 = tau * v1, t3 = tau * v2;
+  const double t1 = p[0] + v1 * p[st] + v2 * p[2 * st];
+  p[0] -= t1 * tau;
+  p[st] -= t2 * t1;
+  p[2 * st] -= t3 * t1;
+}
+// Rotations of one line: rmul!(M, G) on columns is qz_rot_cols.
+__device__ __forceinline__ void qz_rot_rows(double* p, double c, double s) {
+  const double x = p[0], y = p[1];
+  p[0] = c * x + s * y;
+  p[1] = c * y - s * x;
+}
+__device__ __forceinline__ void qz_rot_cols(double* p1, double* p2, double c, double s) {
+  const double x = *p1, y = *p2;
+  *p1 = x * c - y * s;
+  *p2 = x * s + y * c;
+}
+__device__ __forceinline__ void qz_rot_cols_adj(double* p1, double* p2, double c, double s) {
+  const double x = *p1, y = *p2;
+  *p1 = x * c + y * s;
+  *p2 = y * c - x * s;
+}
+
+// Far work of a double-shift step, thread t of nt: left on the columns from j+3 and Q, right on the
+// rows above j and Z.
+__device__ __forceinline__ void qz_far_left3(double* H, double* B, int ld, double* Q, int lq, int n, int j, double tau,
+                                             double v1, double v2, int t, int nt) {
+  const int nc = max(n - j - 2, 0), tot = 2 * nc + (Q ? n : 0);
+  for (; t < tot; t += nt) {
+    if (t < 2 * nc) {
+      double* M = t < nc ? H : B;
+      qz_left3(&M[(j - 1) + (size_t)(j + 2 + (t < nc ? t : t - nc)) * ld], tau, v1, v2);
+    } else {
+      const double t2 = tau * v1, t3 = tau * v2;
+      double* q = Q + (t - 2 * nc) + (size_t)(j - 1) * lq;
+      const double t1 = q[0] + v1 * q[lq] + v2 * q[2 * lq];
+      q[0] -= t1 * tau;
+      q[lq] -= t1 * t2;
+      q[2 * lq] -= t1 * t3;
+    }
+  }
+}
+__device__ __forceinline__ void qz_far_right3(double* H, double* B, int ld, double* Z, int lq, int n, int j, double tau,
+                                              double v1, double v2, int t, int nt) {
+  const int nr = j - 1, tot = 2 * nr + (Z ? n : 0);
+  for (; t < tot; t += nt) {
+    double* p = t < nr ? H + t : (t < 2 * nr ? B + (t - nr) : Z + (t - 2 * nr));
+    const size_t st = t < 2 * nr ? ld : lq;
+    qz_right3(p + (j - 1) * st, st, tau, v1, v2);
+  }
+}
+// ... of a single-shift step.
+__device__ __forceinline__ void qz_far_left2(double* H, double* B, int ld, double* Q, int lq, int n, int j, double c,
+                                             double s, int t, int nt) {
+  const int nc = max(n - j - 1, 0), tot = 2 * nc + (Q ? n : 0);
+  for (; t < tot; t += nt) {
+    if (t < 2 * nc) {
+      double* M = t < nc ? H : B;
+      qz_rot_rows(&M[(j - 1) + (size_t)(j + 1 + (t < nc ? t : t - nc)) * ld], c, s);
+    } else {
+      double* q = Q + (t - 2 * nc) + (size_t)(j - 1) * lq;
+      qz_rot_cols_adj(q, q + lq, c, s);
+    }
+  }
+}
+__device__ __forceinline__ void qz_far_right2(double* H, double* B, int ld, double* Z, int lq, int n, int j, double c,
+                                              double s, int t, int nt) {
+  const int nr = j - 1, tot = 2 * nr + (Z ? n : 0);
+  for (; t < tot; t += nt) {
+    double* p = t < nr ? H + t : (t < 2 * nr ? B + (t - nr) : Z + (t - 2 * nr));
+    const size_t st = t < 2 * nr ? ld : lq;
+    qz_rot_cols(p + (j - 1) * st, p + j * st, c, s);
+  }
+}
+
+// _gqz! (rgeneralized.jl:68-808), ilo = 1, ihi = n, wantSchur; returns 0 or 1.  H, B with
+// leading dimension ld, Q, Z with lq.
+__device__ int gqz_real(double* H, double* B, int ld, double* Q, double* Z, int lq, int n, double2* alpha, double* beta,
                         long long maxiter, double* red) {
-  const int tid = threadIdx.x;
+  __shared__ QzrStep steps[2];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int ilo = 1;
   const double ulp = Prec<double>::eps, safmin = Prec<double>::fmin, safmax = 1.0 / safmin, safety = 100.0;
-  const double anorm = cta_fro_real(H, n, red), bnorm = cta_fro_real(B, n, red);
+  const double anorm = cta_fro_real(H, n, ld, red), bnorm = cta_fro_real(B, n, ld, red);
   const double atol = fmax(safmin, ulp * anorm), btol = fmax(safmin, ulp * bnorm);
   const double ascale = 1.0 / fmax(safmin, anorm), bscale = 1.0 / fmax(safmin, bnorm);
   int ifirst = ilo, ilast = n;
@@ -317,7 +455,16 @@ __device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, doubl
         SYNC();
         br = INF;
       } else {
-        for (int j = ilast - 1; j >= ilo; --j) {
+        // the largest j with a negligible H[j, j-1] (or the first row) or B[j, j]; every case below leaves
+        // the loop
+        int jf = ilo;
+        for (int top = ilast - 1; top >= ilo; top -= 32) {
+          const int q = top - lane;
+          const bool hit = q >= ilo && (q == ilo || fabs(HH(q, q - 1)) <= atol || fabs(BB(q, q)) < btol);
+          const unsigned bal = __ballot_sync(0xffffffffu, hit);
+          if (bal) { jf = top - (__ffs(bal) - 1); break; }
+        }
+        for (int j = jf; j >= ilo; --j) {
           bool h0 = false;
           if (j == ilo) {
             h0 = true;
@@ -344,9 +491,9 @@ __device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, doubl
                 givens_alg(HH(jch, jch), HH(jch + 1, jch), c, s, r);
                 SYNC();
                 if (tid == 0) { HH(jch, jch) = r; HH(jch + 1, jch) = 0.0; }
-                crows(H, n, jch, jch + 1, c, s, jch + 1, ilastm);
-                crows(B, n, jch, jch + 1, c, s, jch + 1, ilastm);
-                if (Q) ccols_adj(Q, n, jch, jch + 1, c, s, 1, n);
+                crows(H, ld, jch, jch + 1, c, s, jch + 1, ilastm);
+                crows(B, ld, jch, jch + 1, c, s, jch + 1, ilastm);
+                if (Q) ccols_adj(Q, lq, jch, jch + 1, c, s, 1, n);
                 SYNC();
                 if (have2) {
                   if (tid == 0) HH(jch, jch - 1) *= c;
@@ -370,17 +517,17 @@ __device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, doubl
                 givens_alg(BB(jch, jch + 1), BB(jch + 1, jch + 1), c, s, r);
                 SYNC();
                 if (tid == 0) { BB(jch, jch + 1) = r; BB(jch + 1, jch + 1) = 0.0; }
-                if (jch < ilastm - 1) crows(B, n, jch, jch + 1, c, s, jch + 2, ilastm);
-                crows(H, n, jch, jch + 1, c, s, jch - 1, ilastm);
-                if (Q) ccols_adj(Q, n, jch, jch + 1, c, s, 1, n);
+                if (jch < ilastm - 1) crows(B, ld, jch, jch + 1, c, s, jch + 2, ilastm);
+                crows(H, ld, jch, jch + 1, c, s, jch - 1, ilastm);
+                if (Q) ccols_adj(Q, lq, jch, jch + 1, c, s, 1, n);
                 SYNC();
                 givens_alg(HH(jch + 1, jch), HH(jch + 1, jch - 1), c, s, r);
                 SYNC();
                 if (tid == 0) { HH(jch + 1, jch) = r; HH(jch + 1, jch - 1) = 0.0; }
                 SYNC();
-                ccols_adj(H, n, jch, jch - 1, c, s, ifirstm, jch);
-                ccols_adj(B, n, jch, jch - 1, c, s, ifirstm, jch - 1);
-                if (Z) ccols_adj(Z, n, jch, jch - 1, c, s, 1, n);
+                ccols_adj(H, ld, jch, jch - 1, c, s, ifirstm, jch);
+                ccols_adj(B, ld, jch, jch - 1, c, s, ifirstm, jch - 1);
+                if (Z) ccols_adj(Z, lq, jch, jch - 1, c, s, 1, n);
                 SYNC();
               }
               br = INF;
@@ -399,9 +546,9 @@ __device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, doubl
         SYNC();
         if (tid == 0) { HH(ilast, ilast) = r; HH(ilast, ilast - 1) = 0.0; }
         SYNC();
-        ccols_adj(H, n, ilast, ilast - 1, c, s, ifirstm, ilast - 1);
-        ccols_adj(B, n, ilast, ilast - 1, c, s, ifirstm, ilast - 1);
-        if (Z) ccols_adj(Z, n, ilast, ilast - 1, c, s, 1, n);
+        ccols_adj(H, ld, ilast, ilast - 1, c, s, ifirstm, ilast - 1);
+        ccols_adj(B, ld, ilast, ilast - 1, c, s, ifirstm, ilast - 1);
+        if (Z) ccols_adj(Z, lq, ilast, ilast - 1, c, s, 1, n);
         SYNC();
         br = NORMAL;
       }
@@ -409,9 +556,9 @@ __device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, doubl
     if (br == NORMAL) {
       if (BB(ilast, ilast) < 0.0) {
         SYNC();
-        cnegcol(H, n, ilast, ifirstm, ilast);
-        cnegcol(B, n, ilast, ifirstm, ilast);
-        if (Z) cnegcol(Z, n, ilast, 1, n);
+        cnegcol(H, ld, ilast, ifirstm, ilast);
+        cnegcol(B, ld, ilast, ifirstm, ilast);
+        if (Z) cnegcol(Z, lq, ilast, 1, n);
         SYNC();
       }
       if (tid == 0) {
@@ -428,7 +575,7 @@ __device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, doubl
     ++shiftcount;
     double s1, s2, wr, wr2, wi;
     if (shiftcount % 10 != 0) {
-      ggs2x2(H, B, n, ilast - 1, safmin * safety, s1, s2, wr, wr2, wi);
+      ggs2x2(H, B, ld, ilast - 1, safmin * safety, s1, s2, wr, wr2, wi);
       if (fabs((wr / s1) * BB(ilast, ilast) - HH(ilast, ilast)) > fabs((wr2 / s2) * BB(ilast, ilast) - HH(ilast, ilast))) {
         double t = wr; wr = wr2; wr2 = t;
         t = s1; s1 = s2; s2 = t;
@@ -450,56 +597,85 @@ __device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, doubl
       if (fabs(wr) > t) scale = fmin(scale, t / fabs(wr));
       s1 *= scale;
       wr *= scale;
-      int istart = -1;
-      bool gotit = false;
-      for (int j = ilast - 1; j >= ifirst + 1; --j) {
-        istart = j;
-        double t1 = fabs(s1 * HH(j, j - 1));
-        double t2 = fabs(s1 * HH(j, j) - wr * BB(j, j));
-        const double tr = fmax(t1, t2);
-        if (tr < 1.0 && tr != 0.0) { t1 /= tr; t2 /= tr; }
-        if (fabs((ascale * HH(j + 1, j)) * t1) <= ascale * atol * t2) { gotit = true; break; }
+      int istart = ifirst;
+      for (int top = ilast - 1; top >= ifirst + 1; top -= 32) {
+        const int j = top - lane;
+        bool hit = false;
+        if (j >= ifirst + 1) {
+          double t1 = fabs(s1 * HH(j, j - 1));
+          double t2 = fabs(s1 * HH(j, j) - wr * BB(j, j));
+          const double tr = fmax(t1, t2);
+          if (tr < 1.0 && tr != 0.0) { t1 /= tr; t2 /= tr; }
+          hit = fabs((ascale * HH(j + 1, j)) * t1) <= ascale * atol * t2;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, hit);
+        if (bal) { istart = top - (__ffs(bal) - 1); break; }
       }
-      if (!gotit) istart = ifirst;
       const double f1 = s1 * HH(istart, istart) - wr * BB(istart, istart);
       const double g2 = s1 * HH(istart + 1, istart);
-      double c, s, t3;
-      givens_alg(f1, g2, c, s, t3);
-      for (int j = istart; j <= ilast - 1; ++j) {
-        if (j > istart) {
-          double r;
-          givens_alg(HH(j, j - 1), HH(j + 1, j - 1), c, s, r);
-          SYNC();
-          if (tid == 0) { HH(j, j - 1) = r; HH(j + 1, j - 1) = 0.0; }
-        }
+      {
+        double c, s, t3;
+        givens_alg(f1, g2, c, s, t3);
         SYNC();
-        crows(H, n, j, j + 1, c, s, j, ilastm);
-        crows(B, n, j, j + 1, c, s, j, ilastm);
-        if (Q) ccols_adj(Q, n, j, j + 1, c, s, 1, n);
-        SYNC();
-        double r;
-        givens_alg(BB(j + 1, j + 1), BB(j + 1, j), c, s, r);
-        SYNC();
-        if (tid == 0) { BB(j + 1, j + 1) = r; BB(j + 1, j) = 0.0; }
-        SYNC();
-        ccols(H, n, j, j + 1, c, s, ifirstm, min(j + 2, ilast));
-        ccols(B, n, j, j + 1, c, s, ifirstm, j);
-        if (Z) ccols(Z, n, j, j + 1, c, s, 1, n);
+        if (tid == 0) { steps[istart & 1].l0 = c; steps[istart & 1].l1 = s; }
         SYNC();
       }
+      for (int j = istart; j <= ilast - 1; ++j) {
+        QzrStep& st = steps[j & 1];
+        if (wid == 0) {
+          // left on columns j, j+1 of H and B
+          double c = st.l0, s = st.l1, r;
+          if (lane < 4) {
+            double* M = lane < 2 ? H : B;
+            qz_rot_rows(&M[(j - 1) + (size_t)(j - 1 + (lane & 1)) * ld], c, s);
+          }
+          __syncwarp();
+          givens_lanes(BB(j + 1, j + 1), BB(j + 1, j), c, s, r);
+          __syncwarp();
+          // right on rows j..min(j+2, ilast) of H and j of B
+          if (lane < 3 && j + lane <= ilast) qz_rot_cols(&HH(j + lane, j), &HH(j + lane, j + 1), c, s);
+          if (lane == 3) qz_rot_cols(&BB(j, j), &BB(j, j + 1), c, s);
+          if (lane == 4) { BB(j + 1, j + 1) = r; BB(j + 1, j) = 0.0; }
+          if (lane == 0) { st.r0 = c; st.r1 = s; }
+          __syncwarp();
+          if (j + 1 <= ilast - 1) {
+            double f = HH(j + 1, j), g = HH(j + 2, j);
+            givens_lanes(f, g, c, s, r);
+            __syncwarp();
+            if (lane == 0) {
+              HH(j + 1, j) = r;
+              HH(j + 2, j) = 0.0;
+              steps[(j + 1) & 1].l0 = c;
+              steps[(j + 1) & 1].l1 = s;
+            }
+          }
+        } else {
+          qz_far_left2(H, B, ld, Q, lq, n, j, st.l0, st.l1, tid - 32, kQrT - 32);
+          if (j > istart) {
+            const QzrStep& pv = steps[(j - 1) & 1];
+            qz_far_right2(H, B, ld, Z, lq, n, j - 1, pv.r0, pv.r1, tid - 32, kQrT - 32);
+          }
+        }
+        SYNC();
+      }
+      if (ilast - 1 >= istart) {
+        const QzrStep& pv = steps[(ilast - 1) & 1];
+        qz_far_right2(H, B, ld, Z, lq, n, ilast - 1, pv.r0, pv.r1, tid, kQrT);
+      }
+      SYNC();
     } else if (ilast == ifirst + 1) {
       // 2 x 2 block with complex eigenvalues: diagonalise the B block, then alpha, beta
       double b22, b11, sr, cr, sl, cl;
       gsvd2x2(BB(ifirst, ifirst), BB(ifirst, ilast), BB(ilast, ilast), b22, b11, sr, cr, sl, cl);
       if (b11 < 0.0) { cr = -cr; sr = -sr; b11 = -b11; b22 = -b22; }
       SYNC();
-      crows(H, n, ifirst, ilast, cl, sl, ifirst, ilastm);
+      crows(H, ld, ifirst, ilast, cl, sl, ifirst, ilastm);
       SYNC();
-      ccols_adj(H, n, ifirst, ilast, cr, sr, ifirstm, ilast);
-      if (ilast < ilastm) crows(B, n, ifirst, ilast, cl, sl, ilast + 1, ilastm);
-      if (ifirstm < ifirst) ccols_adj(B, n, ifirst, ilast, cr, sr, ifirstm, ifirst - 1);
-      if (Q) ccols_adj(Q, n, ifirst, ilast, cl, sl, 1, n);
-      if (Z) ccols_adj(Z, n, ifirst, ilast, cr, sr, 1, n);
+      ccols_adj(H, ld, ifirst, ilast, cr, sr, ifirstm, ilast);
+      if (ilast < ilastm) crows(B, ld, ifirst, ilast, cl, sl, ilast + 1, ilastm);
+      if (ifirstm < ifirst) ccols_adj(B, ld, ifirst, ilast, cr, sr, ifirstm, ifirst - 1);
+      if (Q) ccols_adj(Q, lq, ifirst, ilast, cl, sl, 1, n);
+      if (Z) ccols_adj(Z, lq, ifirst, ilast, cr, sr, 1, n);
       SYNC();
       if (tid == 0) {
         BB(ilast - 1, ilast - 1) = b11;
@@ -509,14 +685,14 @@ __device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, doubl
       }
       SYNC();
       if (b22 < 0.0) {
-        cnegcol(H, n, ilast, ifirstm, ilast);
-        cnegcol(B, n, ilast, ifirstm, ilast);
-        if (Z) cnegcol(Z, n, ilast, 1, n);
+        cnegcol(H, ld, ilast, ifirstm, ilast);
+        cnegcol(B, ld, ilast, ifirstm, ilast);
+        if (Z) cnegcol(Z, lq, ilast, 1, n);
         SYNC();
         b22 = -b22;
       }
       double d2, d3;
-      ggs2x2(H, B, n, ilast - 1, safmin * safety, s1, d2, wr, d3, wi);
+      ggs2x2(H, B, ld, ilast - 1, safmin * safety, s1, d2, wr, d3, wi);
       if (wi == 0.0) continue;  // back to a single shift
       const double s1inv = 1.0 / s1;
       const double a11 = HH(ilast - 1, ilast - 1), a21 = HH(ilast, ilast - 1), a12 = HH(ilast - 1, ilast),
@@ -595,128 +771,127 @@ __device__ int gqz_real(double* H, double* B, double* Q, double* Z, int n, doubl
       double v1 = (((ad22l - ad11l) - ad21l * u12l - (ad11 - ad11l) - (ad22 - ad11l) + ad21 * u12)) * ad21l;
       double v2 = ad32l * ad21l;
       const int istart = ifirst;
-      double tau = refl3(v0, v1, v2);
-      for (int j = istart; j <= ilast - 2; ++j) {
-        if (j > istart) {
-          v0 = HH(j, j - 1);
-          v1 = HH(j + 1, j - 1);
-          v2 = HH(j + 2, j - 1);
-          tau = refl3(v0, v1, v2);
-          SYNC();
-          if (tid == 0) { HH(j, j - 1) = v0; HH(j + 1, j - 1) = 0.0; HH(j + 2, j - 1) = 0.0; }
-        }
+      {
+        const double tau = refl3(v0, v1, v2);
         SYNC();
-        {
-          const double t2 = tau * v1, t3 = tau * v2;
-          for (int jc = j + tid; jc <= ilastm; jc += kQrT) {
-            double t1 = HH(j, jc) + v1 * HH(j + 1, jc) + v2 * HH(j + 2, jc);
-            HH(j, jc) -= t1 * tau;
-            HH(j + 1, jc) -= t1 * t2;
-            HH(j + 2, jc) -= t1 * t3;
-            t1 = BB(j, jc) + v1 * BB(j + 1, jc) + v2 * BB(j + 2, jc);
-            BB(j, jc) -= t1 * tau;
-            BB(j + 1, jc) -= t1 * t2;
-            BB(j + 2, jc) -= t1 * t3;
-          }
-          if (Q)
-            for (int jr = 1 + tid; jr <= n; jr += kQrT) {
-              double* qr = Q + (jr - 1);
-              const double t1 = qr[(size_t)(j - 1) * n] + v1 * qr[(size_t)j * n] + v2 * qr[(size_t)(j + 1) * n];
-              qr[(size_t)(j - 1) * n] -= t1 * tau;
-              qr[(size_t)j * n] -= t1 * t2;
-              qr[(size_t)(j + 1) * n] -= t1 * t3;
-            }
-        }
-        SYNC();
-        // zero the j-th column of B: 2 x 2 solve with pivoting
-        bool pivot = false;
-        double scale, u1, u2;
-        {
-          double t1 = fmax(fabs(BB(j + 1, j + 1)), fabs(BB(j + 1, j + 2)));
-          const double tt2 = fmax(fabs(BB(j + 2, j + 1)), fabs(BB(j + 2, j + 2)));
-          if (fmax(t1, tt2) < safmin) {
-            scale = 0.0; u1 = 1.0; u2 = 0.0;
-          } else {
-            double w11, w21, w12, w22;
-            if (t1 >= tt2) {
-              w11 = BB(j + 1, j + 1); w21 = BB(j + 2, j + 1); w12 = BB(j + 1, j + 2); w22 = BB(j + 2, j + 2);
-              u1 = BB(j + 1, j); u2 = BB(j + 2, j);
-            } else {
-              w21 = BB(j + 1, j + 1); w11 = BB(j + 2, j + 1); w22 = BB(j + 1, j + 2); w12 = BB(j + 2, j + 2);
-              u2 = BB(j + 1, j); u1 = BB(j + 2, j);
-            }
-            if (fabs(w12) > fabs(w11)) {
-              pivot = true;
-              double t = w11; w11 = w12; w12 = t;
-              t = w21; w21 = w22; w22 = t;
-            }
-            t1 = w21 / w11;
-            u2 -= t1 * u1;
-            w22 -= t1 * w12;
-            scale = 1.0;
-            if (fabs(w22) < safmin) {
-              scale = 0.0;
-            } else {
-              if (fabs(w22) < fabs(u2)) scale = fabs(w22 / u2);
-              if (fabs(w11) < fabs(u1)) scale = fmin(scale, fabs(w11 / u1));
-              u2 = (scale * u2) / w22;
-              u1 = (scale * u1 - w12 * u2) / w11;
-            }
-          }
-        }
-        if (pivot) { const double t = u1; u1 = u2; u2 = t; }
-        {
-          const double t1 = bhypot3(scale, u1, u2);
-          tau = 1.0 + scale / t1;
-          const double vs = -1.0 / (scale + t1);
-          v1 = vs * u1;
-          v2 = vs * u2;
-        }
-        {
-          const double t2 = tau * v1, t3 = tau * v2;
-          const int rh = min(j + 3, ilast);
-          for (int jr = ifirstm + tid; jr <= rh; jr += kQrT) {
-            const double t1 = HH(jr, j) + v1 * HH(jr, j + 1) + v2 * HH(jr, j + 2);
-            HH(jr, j) -= t1 * tau;
-            HH(jr, j + 1) -= t2 * t1;
-            HH(jr, j + 2) -= t3 * t1;
-          }
-          for (int jr = ifirstm + tid; jr <= j + 2; jr += kQrT) {
-            const double t1 = BB(jr, j) + v1 * BB(jr, j + 1) + v2 * BB(jr, j + 2);
-            BB(jr, j) -= t1 * tau;
-            BB(jr, j + 1) -= t2 * t1;
-            BB(jr, j + 2) -= t3 * t1;
-          }
-          if (Z)
-            for (int jr = 1 + tid; jr <= n; jr += kQrT) {
-              double* zr = Z + (jr - 1);
-              const double t1 = zr[(size_t)(j - 1) * n] + v1 * zr[(size_t)j * n] + v2 * zr[(size_t)(j + 1) * n];
-              zr[(size_t)(j - 1) * n] -= t1 * tau;
-              zr[(size_t)j * n] -= t2 * t1;
-              zr[(size_t)(j + 1) * n] -= t3 * t1;
-            }
-        }
-        SYNC();
-        if (tid == 0) { BB(j + 1, j) = 0.0; BB(j + 2, j) = 0.0; }
+        if (tid == 0) { QzrStep& st = steps[istart & 1]; st.l0 = tau; st.l1 = v1; st.l2 = v2; }
         SYNC();
       }
+      for (int j = istart; j <= ilast - 2; ++j) {
+        QzrStep& st = steps[j & 1];
+        if (wid == 0) {
+          // left on columns j..j+2 of H and B
+          if (lane < 6) {
+            double* M = lane < 3 ? H : B;
+            qz_left3(&M[(j - 1) + (size_t)(j - 1 + (lane < 3 ? lane : lane - 3)) * ld], st.l0, st.l1, st.l2);
+          }
+          __syncwarp();
+          // zero the j-th column of B: 2 x 2 solve with pivoting
+          bool pivot = false;
+          double scale, u1, u2;
+          {
+            double t1 = fmax(fabs(BB(j + 1, j + 1)), fabs(BB(j + 1, j + 2)));
+            const double tt2 = fmax(fabs(BB(j + 2, j + 1)), fabs(BB(j + 2, j + 2)));
+            if (fmax(t1, tt2) < safmin) {
+              scale = 0.0; u1 = 1.0; u2 = 0.0;
+            } else {
+              double w11, w21, w12, w22;
+              if (t1 >= tt2) {
+                w11 = BB(j + 1, j + 1); w21 = BB(j + 2, j + 1); w12 = BB(j + 1, j + 2); w22 = BB(j + 2, j + 2);
+                u1 = BB(j + 1, j); u2 = BB(j + 2, j);
+              } else {
+                w21 = BB(j + 1, j + 1); w11 = BB(j + 2, j + 1); w22 = BB(j + 1, j + 2); w12 = BB(j + 2, j + 2);
+                u2 = BB(j + 1, j); u1 = BB(j + 2, j);
+              }
+              if (fabs(w12) > fabs(w11)) {
+                pivot = true;
+                double t = w11; w11 = w12; w12 = t;
+                t = w21; w21 = w22; w22 = t;
+              }
+              t1 = w21 / w11;
+              u2 -= t1 * u1;
+              w22 -= t1 * w12;
+              scale = 1.0;
+              if (fabs(w22) < safmin) {
+                scale = 0.0;
+              } else {
+                if (fabs(w22) < fabs(u2)) scale = fabs(w22 / u2);
+                if (fabs(w11) < fabs(u1)) scale = fmin(scale, fabs(w11 / u1));
+                u2 = (scale * u2) / w22;
+                u1 = (scale * u1 - w12 * u2) / w11;
+              }
+            }
+          }
+          if (pivot) { const double t = u1; u1 = u2; u2 = t; }
+          double tau, v1, v2;
+          {
+            // bhypot3(scale, u1, u2) with its quotients on lanes 0, 1, 2
+            double t1;
+            const double m = fmax(fmax(fabs(scale), fabs(u1)), fabs(u2));
+            if (m > 0.0 && !isinf(m)) {
+              const double w = (lane == 1 ? u1 : (lane == 2 ? u2 : scale)) / m;
+              const double a = lane_get(w, 0), b = lane_get(w, 1), c = lane_get(w, 2);
+              t1 = m * sqrt(a * a + b * b + c * c);
+            } else {
+              t1 = bhypot3(scale, u1, u2);
+            }
+            const double w = ((lane & 1) ? -1.0 : scale) / ((lane & 1) ? (scale + t1) : t1);
+            tau = 1.0 + lane_get(w, 0);
+            const double vs = lane_get(w, 1);
+            v1 = vs * u1;
+            v2 = vs * u2;
+          }
+          __syncwarp();
+          // right on rows j..min(j+3, ilast) of H and j..j+2 of B
+          if (lane < 4 && j + lane <= ilast) qz_right3(&HH(j + lane, j), ld, tau, v1, v2);
+          if (lane >= 4 && lane < 7) {
+            const int jr = j + lane - 4;
+            qz_right3(&BB(jr, j), ld, tau, v1, v2);
+            if (jr > j) BB(jr, j) = 0.0;
+          }
+          if (lane == 0) { st.r0 = tau; st.r1 = v1; st.r2 = v2; }
+          __syncwarp();
+          if (j + 1 <= ilast - 2) {
+            double w0 = HH(j + 1, j), w1 = HH(j + 2, j), w2 = HH(j + 3, j);
+            const double tl = refl3_lanes(w0, w1, w2);
+            __syncwarp();
+            if (lane == 0) {
+              HH(j + 1, j) = w0; HH(j + 2, j) = 0.0; HH(j + 3, j) = 0.0;
+              QzrStep& nx = steps[(j + 1) & 1];
+              nx.l0 = tl; nx.l1 = w1; nx.l2 = w2;
+            }
+          }
+        } else {
+          qz_far_left3(H, B, ld, Q, lq, n, j, st.l0, st.l1, st.l2, tid - 32, kQrT - 32);
+          if (j > istart) {
+            const QzrStep& pv = steps[(j - 1) & 1];
+            qz_far_right3(H, B, ld, Z, lq, n, j - 1, pv.r0, pv.r1, pv.r2, tid - 32, kQrT - 32);
+          }
+        }
+        SYNC();
+      }
+      {
+        const QzrStep& pv = steps[(ilast - 2) & 1];
+        qz_far_right3(H, B, ld, Z, lq, n, ilast - 2, pv.r0, pv.r1, pv.r2, tid, kQrT);
+      }
+      SYNC();
       // the last two rotations
       const int j = ilast - 1;
       double c, s, r;
       givens_alg(HH(j, j - 1), HH(j + 1, j - 1), c, s, r);
       SYNC();
       if (tid == 0) { HH(j, j - 1) = r; HH(j + 1, j - 1) = 0.0; }
-      crows(H, n, j, j + 1, c, s, j, ilastm);
-      crows(B, n, j, j + 1, c, s, j, ilastm);
-      if (Q) ccols_adj(Q, n, j, j + 1, c, s, 1, n);
+      crows(H, ld, j, j + 1, c, s, j, ilastm);
+      crows(B, ld, j, j + 1, c, s, j, ilastm);
+      if (Q) ccols_adj(Q, lq, j, j + 1, c, s, 1, n);
       SYNC();
       givens_alg(BB(j + 1, j + 1), BB(j + 1, j), c, s, r);
       SYNC();
       if (tid == 0) { BB(j + 1, j + 1) = r; BB(j + 1, j) = 0.0; }
       SYNC();
-      ccols_adj(H, n, j + 1, j, c, s, ifirstm, ilast);
-      ccols_adj(B, n, j + 1, j, c, s, ifirstm, ilast - 1);
-      if (Z) ccols_adj(Z, n, j + 1, j, c, s, 1, n);
+      ccols_adj(H, ld, j + 1, j, c, s, ifirstm, ilast);
+      ccols_adj(B, ld, j + 1, j, c, s, ifirstm, ilast - 1);
+      if (Z) ccols_adj(Z, lq, j + 1, j, c, s, 1, n);
       SYNC();
     }
     if (it >= maxiter) return 1;
@@ -757,16 +932,82 @@ __device__ bool cta_scale_real(double* M, int n, double* red, double& cscale, do
   return sc;
 }
 
-__global__ void __launch_bounds__(kQrT) k_ggschur_real(QzrBatch bt) {
+template <int NT> __device__ __forceinline__ void qz_far_barrier() { asm volatile("bar.sync 2, %0;" ::"n"(NT - 32) : "memory"); }
+
+// _hessenberg!(A, B, Q, Z) (generalized.jl:84-113).  In phase jr of column jc the chain warp rotates
+// A[jr-1:jr, jc] and B[jr-1:jr, jr-1:jr], computes the right rotation of jr and the left rotation of
+// jr-1 (on even and odd lanes) and applies the right one to rows jr-2..jr of B; the others apply the right
+// rotation of jr+1 and then the left one of jr.  Row jr-2 of B needs the right rotation of jr+1 before
+// that of jr, so the chain warp does that one too.
+__device__ void ht_real(double* H, double* B, int ld, double* Q, double* Z, int lq, int n) {
+  __shared__ QzrStep steps[2];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  constexpr int NF = kQrT - 32;
+  // right rotation of jq on all rows of A, the rows of B outside [x0, x1], Z: thread t of nt
+  auto far_right = [&](int jq, double c, double s, int x0, int x1, int t, int nt) {
+    for (; t < 2 * n + (Z ? n : 0); t += nt) {
+      const int r = t % n;
+      if (t < n) qz_rot_cols_adj(&HH(r + 1, jq), &HH(r + 1, jq - 1), c, s);
+      else if (t < 2 * n) { if (r + 1 < x0 || r + 1 > x1) qz_rot_cols_adj(&BB(r + 1, jq), &BB(r + 1, jq - 1), c, s); }
+      else qz_rot_cols_adj(Z + r + (size_t)(jq - 1) * lq, Z + r + (size_t)(jq - 2) * lq, c, s);
+    }
+  };
+  for (int jc = 1; jc <= n - 2; ++jc) {
+    if (wid == 0) {
+      double c, s, r;
+      givens_lanes(HH(n - 1, jc), HH(n, jc), c, s, r);
+      if (lane == 0) { steps[n & 1].l0 = c; steps[n & 1].l1 = s; }
+    }
+    SYNC();
+    for (int jr = n; jr >= jc + 2; --jr) {
+      QzrStep& st = steps[jr & 1];
+      const QzrStep& pv = steps[(jr + 1) & 1];
+      if (wid == 0) {
+        const double cl = st.l0, sl = st.l1;
+        if (lane == 3 && jr < n) qz_rot_cols_adj(&BB(jr - 2, jr + 1), &BB(jr - 2, jr), pv.r0, pv.r1);
+        if (lane == 0) qz_rot_rows(&HH(jr - 1, jc), cl, sl);
+        if (lane == 1 || lane == 2) qz_rot_rows(&BB(jr - 1, jr - 2 + lane), cl, sl);
+        __syncwarp();
+        const bool more = jr - 1 >= jc + 2;
+        double f = BB(jr, jr), g = BB(jr, jr - 1), c, s, r;
+        if ((lane & 1) && more) { f = HH(jr - 2, jc); g = HH(jr - 1, jc); }
+        givens_lanes(f, g, c, s, r);
+        const double cr = lane_get(c, 0), sr = lane_get(s, 0);
+        __syncwarp();
+        if (lane < 3 && jr - 2 + lane >= 1) qz_rot_cols_adj(&BB(jr - 2 + lane, jr), &BB(jr - 2 + lane, jr - 1), cr, sr);
+        if (lane == 0) { st.r0 = cr; st.r1 = sr; }
+        const double cn = lane_get(c, 1), sn = lane_get(s, 1);
+        if (lane == 0 && more) { steps[(jr - 1) & 1].l0 = cn; steps[(jr - 1) & 1].l1 = sn; }
+      } else {
+        if (jr < n) far_right(jr + 1, pv.r0, pv.r1, jr - 2, jr + 1, tid - 32, NF);
+        qz_far_barrier<kQrT>();
+        const double c = st.l0, s = st.l1;
+        for (int t = tid - 32; t < 2 * n + (Q ? n : 0); t += NF) {
+          const int q = t % n;
+          if (t < n) { if (q + 1 != jc) qz_rot_rows(&HH(jr - 1, q + 1), c, s); }
+          else if (t < 2 * n) { if (q + 1 != jr - 1 && q + 1 != jr) qz_rot_rows(&BB(jr - 1, q + 1), c, s); }
+          else qz_rot_cols_adj(Q + q + (size_t)(jr - 2) * lq, Q + q + (size_t)(jr - 1) * lq, c, s);
+        }
+      }
+      SYNC();
+    }
+    // the last right rotation (jr = jc + 2): the rows of B above jc have not seen it
+    far_right(jc + 2, steps[(jc + 2) & 1].r0, steps[(jc + 2) & 1].r1, jc, jc + 2, tid, kQrT);
+    SYNC();
+  }
+}
+
+__global__ void __launch_bounds__(kQrT, 3) k_ggschur_real(QzrBatch bt, int cap) {
+  extern __shared__ double smq[];
   __shared__ double red[kQrT / 32];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int b = blockIdx.x; b < bt.count; b += gridDim.x) {
     const int n = bt.ns ? bt.ns[b] : bt.n1;
     const long long off = bt.ns ? bt.offs[b] : 0, woff = bt.ns ? bt.woffs[b] : 0;
-    double* A = bt.A + off;
-    double* B = bt.B + off;
-    double* Q = bt.Q ? bt.Q + off : nullptr;
-    double* Z = bt.Z ? bt.Z + off : nullptr;
+    double* Ag = bt.A + off;
+    double* Bg = bt.B + off;
+    double* Qg = bt.Q ? bt.Q + off : nullptr;
+    double* Zg = bt.Z ? bt.Z + off : nullptr;
     double2* alpha = bt.alpha + woff;
     double* beta = bt.beta + woff;
     if (n == 0) {
@@ -776,19 +1017,35 @@ __global__ void __launch_bounds__(kQrT) k_ggschur_real(QzrBatch bt) {
     double cscale = 1.0, anrm = 1.0, cscaleb = 1.0, bnrm = 1.0;
     bool scA = false, scB = false;
     if (bt.scale) {
-      scA = cta_scale_real(A, n, red, cscale, anrm);
-      scB = cta_scale_real(B, n, red, cscaleb, bnrm);
+      scA = cta_scale_real(Ag, n, red, cscale, anrm);
+      scB = cta_scale_real(Bg, n, red, cscaleb, bnrm);
+    }
+    // where the matrices live: shared memory as far as it reaches
+    const long long one = (long long)n * (n | 1);
+    const bool hs = 2 * one <= cap, qs = 4 * one <= cap;
+    const int ld = hs ? (n | 1) : n, lq = qs ? (n | 1) : n;
+    double* A = hs ? smq : Ag;
+    double* B = hs ? smq + one : Bg;
+    double* Q = Qg ? (qs ? smq + 2 * one : Qg) : nullptr;
+    double* Z = Zg ? (qs ? smq + 3 * one : Zg) : nullptr;
+    if (hs) {
+      __syncthreads();
+      for (int e = tid; e < n * n; e += kQrT) {
+        A[e % n + e / n * ld] = Ag[e];
+        B[e % n + e / n * ld] = Bg[e];
+      }
+      __syncthreads();
     }
     // qr!(B), A <- Q^T A; tau in beta (scratch until the iteration)
     for (int j = 1; j <= n; ++j) {
       const int len = n - j + 1;
-      double* v = B + (j - 1) + (size_t)(j - 1) * n;
+      double* v = B + (j - 1) + (size_t)(j - 1) * ld;
       const double t = cta_reflector<kQrT>(v, len, red);
       if (tid == 0) beta[j - 1] = t;
       __syncthreads();
       if (t != 0.0) {
         for (int col = wid; col < (n - j) + n; col += kQrT / 32) {
-          double* x = col < n - j ? B + (j - 1) + (size_t)(j + col) * n : A + (j - 1) + (size_t)(col - (n - j)) * n;
+          double* x = col < n - j ? B + (j - 1) + (size_t)(j + col) * ld : A + (j - 1) + (size_t)(col - (n - j)) * ld;
           double sacc = 0.0;
           for (int r = lane; r < len; r += 32) sacc = fma(r == 0 ? 1.0 : v[r], x[r], sacc);
           for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
@@ -799,15 +1056,15 @@ __global__ void __launch_bounds__(kQrT) k_ggschur_real(QzrBatch bt) {
       __syncthreads();
     }
     if (Q) {
-      for (size_t e = tid; e < (size_t)n * n; e += kQrT) Q[e] = ((e % n) == (e / n)) ? 1.0 : 0.0;
+      for (int e = tid; e < n * n; e += kQrT) Q[e % n + (size_t)(e / n) * lq] = ((e % n) == (e / n)) ? 1.0 : 0.0;
       __syncthreads();
       for (int j = n; j >= 1; --j) {
         const double t = beta[j - 1];
         const int len = n - j + 1;
-        const double* v = B + (j - 1) + (size_t)(j - 1) * n;
+        const double* v = B + (j - 1) + (size_t)(j - 1) * ld;
         if (t != 0.0) {
           for (int col = j + wid; col <= n; col += kQrT / 32) {
-            double* x = Q + (j - 1) + (size_t)(col - 1) * n;
+            double* x = Q + (j - 1) + (size_t)(col - 1) * lq;
             double sacc = 0.0;
             for (int r = lane; r < len; r += 32) sacc = fma(r == 0 ? 1.0 : v[r], x[r], sacc);
             for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
@@ -818,45 +1075,38 @@ __global__ void __launch_bounds__(kQrT) k_ggschur_real(QzrBatch bt) {
         __syncthreads();
       }
     }
-    for (size_t e = tid; e < (size_t)n * n; e += kQrT) {
-      if ((e % n) > (e / n)) B[e] = 0.0;
-      if (Z) Z[e] = ((e % n) == (e / n)) ? 1.0 : 0.0;
+    for (int e = tid; e < n * n; e += kQrT) {
+      const int i = e % n, j = e / n;
+      if (i > j) B[i + (size_t)j * ld] = 0.0;
+      if (Z) Z[i + (size_t)j * lq] = i == j ? 1.0 : 0.0;
     }
     __syncthreads();
-    // _hessenberg!(A, B, Q, Z) (generalized.jl:84-113)
-    for (int jc = 1; jc <= n - 2; ++jc)
-      for (int jr = n; jr >= jc + 2; --jr) {
-        double c, s, r;
-        {
-          const double* H = A;
-          givens_alg(HH(jr - 1, jc), HH(jr, jc), c, s, r);
-        }
-        __syncthreads();
-        crows(A, n, jr - 1, jr, c, s, 1, n);
-        crows(B, n, jr - 1, jr, c, s, 1, n);
-        if (Q) ccols_adj(Q, n, jr - 1, jr, c, s, 1, n);
-        __syncthreads();
-        givens_alg(BB(jr, jr), BB(jr, jr - 1), c, s, r);
-        __syncthreads();
-        ccols_adj(A, n, jr, jr - 1, c, s, 1, n);
-        ccols_adj(B, n, jr, jr - 1, c, s, 1, n);
-        if (Z) ccols_adj(Z, n, jr, jr - 1, c, s, 1, n);
-        __syncthreads();
+    ht_real(A, B, ld, Q, Z, lq, n);
+    for (int e = tid; e < n * n; e += kQrT) {
+      const int i = e % n, j = e / n;
+      if (i > j + 1) A[i + (size_t)j * ld] = 0.0;
+      if (i > j) B[i + (size_t)j * ld] = 0.0;
+    }
+    __syncthreads();
+    const int st = gqz_real(A, B, ld, Q, Z, lq, n, alpha, beta, 100LL * n, red);
+    __syncthreads();
+    if (hs)
+      for (int e = tid; e < n * n; e += kQrT) {
+        Ag[e] = A[e % n + e / n * ld];
+        Bg[e] = B[e % n + e / n * ld];
       }
-    for (size_t e = tid; e < (size_t)n * n; e += kQrT) {
-      const int i = (int)(e % n), j = (int)(e / n);
-      if (i > j + 1) A[e] = 0.0;
-      if (i > j) B[e] = 0.0;
-    }
-    __syncthreads();
-    const int st = gqz_real(A, B, Q, Z, n, alpha, beta, 100LL * n, red);
+    if (qs)
+      for (int e = tid; e < n * n; e += kQrT) {
+        if (Qg) Qg[e] = Q[e % n + e / n * lq];
+        if (Zg) Zg[e] = Z[e % n + e / n * lq];
+      }
     __syncthreads();
     if (scA) {
-      cta_safescale_real(A, (size_t)n * n, cscale, anrm);
+      cta_safescale_real(Ag, (size_t)n * n, cscale, anrm);
       cta_safescale_real(reinterpret_cast<double*>(alpha), 2 * (size_t)n, cscale, anrm);
     }
     if (scB) {
-      cta_safescale_real(B, (size_t)n * n, cscaleb, bnrm);
+      cta_safescale_real(Bg, (size_t)n * n, cscaleb, bnrm);
       cta_safescale_real(beta, (size_t)n, cscaleb, bnrm);
     }
     if (tid == 0 && bt.status) bt.status[b] = st;
@@ -1513,8 +1763,21 @@ cudaError_t launch_ggordschur_real(int n, double* S, double* T, double* Q, doubl
 
 cudaError_t launch_ggschur_real(const QzrBatch& bt, int num_sms, cudaStream_t s) {
   if (bt.count <= 0) return cudaSuccess;
+  // shared memory for the largest pencil's four matrices, or two, as far as it reaches (bt.nmax, 0:
+  // not known, two CTAs per SM)
+  const size_t most = (kMaxDynSmem - 4 * 1024) / sizeof(double);
+  const long long one = (long long)bt.nmax * (bt.nmax | 1);
+  size_t cap = most / 2;
+  if (bt.nmax > 0) {
+    cap = 4 * one <= (long long)most ? (size_t)(4 * one) : (2 * one <= (long long)most ? (size_t)(2 * one) : 0);
+    // smaller pencils of the batch: keep at least what holds all four of theirs at two CTAs per SM
+    if (bt.ns && cap < most / 2) cap = std::max(cap, std::min((size_t)(4 * one), most / 2));
+  }
+  const size_t smem = sizeof(double) * cap;
+  cudaError_t e = cudaFuncSetAttribute(k_ggschur_real, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
   const int grid = std::min(bt.count, 8 * num_sms);
-  k_ggschur_real<<<grid, kQrT, 0, s>>>(bt);
+  k_ggschur_real<<<grid, kQrT, smem, s>>>(bt, (int)cap);
   return cudaGetLastError();
 }
 
