@@ -27,26 +27,20 @@ __global__ void __launch_bounds__(1024) k_bin_sort(const int* __restrict__ ns, i
     atomicAdd(&hist[n], 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  // the matrices of larger order come first: pos[n] = sum of hist over m > n
+  for (int n = threadIdx.x; n <= kSmallMax; n += blockDim.x) {
     int run = 0;
-    int bin = kNumBins - 1;
-    sched[3 * bin] = 0;
-    for (int n = kSmallMax; n >= 0; --n) {
-      while (bin > 0 && n <= bounds.b[bin - 1]) {
-        sched[3 * bin + 1] = run;
-        --bin;
-        sched[3 * bin] = run;
-      }
-      pos[n] = run;
-      run += hist[n];
-    }
-    sched[3 * bin + 1] = run;
-    while (bin > 0) {  // empty low bins
-      --bin;
-      sched[3 * bin] = run;
-      sched[3 * bin + 1] = run;
-    }
-    for (int i = 0; i < kNumBins; ++i) sched[3 * i + 2] = 0;
+#pragma unroll 8
+    for (int m = kSmallMax; m > n; --m) run += hist[m];
+    pos[n] = run;
+  }
+  __syncthreads();
+  if (threadIdx.x < kNumBins) {
+    // bin i holds the orders in (bounds[i-1], bounds[i]], bin 0 those from 0
+    const int i = threadIdx.x, hi = i == kNumBins - 1 ? kSmallMax : bounds.b[i];
+    sched[3 * i] = pos[hi];
+    sched[3 * i + 1] = i > 0 ? pos[bounds.b[i - 1]] : pos[0] + hist[0];
+    sched[3 * i + 2] = 0;
   }
   __syncthreads();
   for (int b = threadIdx.x; b < count; b += blockDim.x) {

@@ -466,6 +466,12 @@ cudaError_t launch_schur_batched_cplx(const CplxBatch& bt, const int* order, int
                                       int num_sms, cudaStream_t* streams, int nstreams);
 cudaError_t launch_schur_batched_cplx_tuned(const CplxBatch& bt, const int* order, int* sched, int num_sms,
                                             cudaStream_t* streams, int nstreams, const BinTuning& tun);
+// One bin's kernels (the queue prepared, shapes from `tun`).
+template <class T, class W>
+cudaError_t launch_schur_real_bin(const RealBatchT<T, W>& bt, const int* order, int* sched, int bin,
+                                  const BinTuning& tun, int num_sms, cudaStream_t s);
+cudaError_t launch_schur_cplx_bin(const CplxBatch& bt, const int* order, int* sched, int bin, const BinTuning& tun,
+                                  int num_sms, cudaStream_t s);
 // One matrix of order m (<= kSmallMax) by one CTA of the default shape of its bin, without
 // the bin sort: launch_single_queue fills order/sched for that bin (default_bin_of(m));
 // launch_single_meta writes iota[0..kSmallMax] and two zero offsets once, so that a batch

@@ -356,6 +356,21 @@ static int run_batched_real(gs_context* ctx, const RealBatchT<T, W>& bt, int* or
   return run_graph_or_direct(ctx, use_graph, key, enqueue);
 }
 
+// One matrix of order n (a batch of one, n known here): only its bin's kernels, on the context stream
+// itself.  The bin sort and the three empty bins of the batched sequence took 30 us of a call.
+template <class F>
+static int run_single(gs_context* ctx, int n, const BinTuning& t, int* order, int* sched, F launch) {
+  int bin = 0;
+  while (bin < kNumBins - 1 && n > t.bounds[bin]) ++bin;
+  cudaStream_t s = ctx->stream;
+  CK(cudaEventRecord(ctx->t0, s));
+  CK(launch_single_queue(bin, order, sched, s));
+  CK(launch(bin, s));
+  CK(cudaEventRecord(ctx->t1, s));
+  ctx->timed = true;
+  return GS_OK;
+}
+
 static int pipe_setup(gs_context* ctx) {
   if (ctx->pipe_ready) return GS_OK;
   for (int c = 0; c < kPipeChunks; ++c) {
@@ -875,7 +890,12 @@ static int schur_real_impl(gs_context* ctx, int64_t n, T* A, int64_t lda, T* Z, 
   long long mi = maxiter > 0 ? maxiter : 100 * n;
   bt.maxiter_mult = 100;
   bt.maxiter_abs = mi;
-  rc = run_batched_real(ctx, bt, (int*)(base + o_order), (int*)(base + o_sched), flags, false, {});
+  int* order = (int*)(base + o_order);
+  int* sched = (int*)(base + o_sched);
+  const BinTuning tun = sizeof(T) == 8 ? ctx->tun_real : default_tuning_real();
+  rc = run_single(ctx, (int)n, tun, order, sched, [&](int bin, cudaStream_t st) {
+    return launch_schur_real_bin(bt, order, sched, bin, tun, ctx->num_sms, st);
+  });
   if (rc) return rc;
   CK(cudaMemcpy2DAsync(A, lda * sizeof(T), dA, n * sizeof(T), n * sizeof(T), n, out, s));
   if (wantz) CK(cudaMemcpy2DAsync(Z, ldz * sizeof(T), dZ, n * sizeof(T), n * sizeof(T), n, out, s));
@@ -1082,7 +1102,11 @@ int gs_schur_c64(gs_context* ctx, int64_t n, double* A, int64_t lda, double* Z, 
     CK(cudaEventRecord(ctx->t1, s));
     ctx->timed = true;
   } else {
-    rc = run_batched_cplx(ctx, bt, (int*)(base + o_order), (int*)(base + o_sched), false, {});
+    int* order = (int*)(base + o_order);
+    int* sched = (int*)(base + o_sched);
+    rc = run_single(ctx, (int)n, ctx->tun_cplx, order, sched, [&](int bin, cudaStream_t st) {
+      return launch_schur_cplx_bin(bt, order, sched, bin, ctx->tun_cplx, ctx->num_sms, st);
+    });
     if (rc) return rc;
   }
   CK(cudaMemcpy2DAsync(A, lda * es, dA, n * es, n * es, n, out, s));

@@ -384,6 +384,24 @@ __device__ __forceinline__ ZR chain_zrefl(double2& a, double2 x1, int lane) {
   return {tau, v2, fma(tau.x, v2.x, -tau.y * v2.y)};
 }
 
+// Exponent field of a double: 2^(e - 1023) <= |x| < 2^(e - 1022) for a normal x (0 and denormals: 0).
+__device__ __forceinline__ int zfield(const double& x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+__device__ __forceinline__ int zfield(const double2& x) { return max(zfield(x.x), zfield(x.y)); }
+
+// Whether the deflation test at row k certainly fails: |Re sd| > ulp (|hkk|_1 + |hk1|_1), all of moderate size.
+__device__ __forceinline__ bool no_zsplit(const double2& sd, const double2& hkk, const double2& hk1) {
+  const int e = zfield(sd.x), m = max(zfield(hkk), zfield(hk1));
+  return e > 923 && m > 0 && e > m + 3 - 52;
+}
+// Whether the start-row test at row mm certainly fails: |h10| |h21| > ulp |h11 - shift|_1 (|h11|_1 + |h22|_1).
+__device__ __forceinline__ bool no_zstart(const double& h10, const double& h21, const double2& h11, const double2& h22,
+                                          double2 shift) {
+  const int e10 = zfield(h10), e21 = zfield(h21), x = max(zfield(h11), zfield(shift)), d = max(zfield(h11), zfield(h22));
+  if (min(e10, e21) < 923 || max(max(e10, e21), max(x, d)) > 1223) return false;
+  // lhs >= 2^(e10 + e21 - 2 bias); rhs < 2^-52 2^(x - bias + 1 + 2) 2^(d - bias + 1 + 2)
+  return e10 + e21 > x + d + 6 - 52;
+}
+
 // Chain warp: steps ka..ka+nst-1 inside the window (columns ..wl, rows ka-1..).  r: the reflector of
 // step ka on entry, of step ka+nst on return (unless that is past the sweep, or fix: the phase fix-up
 // comes before it).
@@ -513,10 +531,12 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
           bool split = false;
           if (k >= istart) {
             const double2 sd = HH(k + 1, k);
-            if (zabs1(sd) <= smallnum) {
+            const double2 hkk = HH(k, k), hk1 = HH(k + 1, k + 1);
+            if (no_zsplit(sd, hkk, hk1)) {
+              split = false;
+            } else if (zabs1(sd) <= smallnum) {
               split = true;
             } else {
-              const double2 hkk = HH(k, k), hk1 = HH(k + 1, k + 1);
               double tst = zabs1(hkk) + zabs1(hk1);
               if (tst == 0.0) {
                 if (k - 1 >= 1) tst += fabs(HH(k, k - 1).x);
@@ -579,7 +599,7 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
         for (int top = iend - 1; top >= istart + 1; top -= 32) {
           const int mm = top - lane;
           bool hit = false;
-          if (mm >= istart + 1) {
+          if (mm >= istart + 1 && !no_zstart(HH(mm, mm - 1).x, HH(mm + 1, mm).x, HH(mm, mm), HH(mm + 1, mm + 1), shift)) {
             const double2 h11 = HH(mm, mm), h22 = HH(mm + 1, mm + 1);
             double2 h11s = zsub(h11, shift);
             double h21 = HH(mm + 1, mm).x;
@@ -874,6 +894,11 @@ cudaError_t launch_schur_batched_cplx(const CplxBatch& bt, const int* order, int
 size_t cplx_bin_smem_bytes(int nmax, int hsmem) {
   const size_t full = hsmem ? sizeof(double2) * ((size_t)nmax * (nmax | 1) + 4 * (size_t)nmax) + 32 * sizeof(double) + 64 : 0;
   return full > ciqr_smem_bytes(nmax) ? full : ciqr_smem_bytes(nmax);
+}
+
+cudaError_t launch_schur_cplx_bin(const CplxBatch& bt, const int* order, int* sched, int bin, const BinTuning& t,
+                                  int num_sms, cudaStream_t s) {
+  return launch_shape_c(bt, order, sched, bin, t.bounds[bin], t.nt[bin], t.ctas[bin], num_sms, s);
 }
 
 cudaError_t launch_schur_cplx_one(const CplxBatch& bt, int m, const int* order, int* sched, cudaStream_t s) {

@@ -680,6 +680,70 @@ __device__ __forceinline__ void st_refl(double* l, const Refl<double>& r) {
   l[4] = r.v3;
 }
 
+// Bounds by exponents, off the FP64 pipe and without quotients: for a normal x with exponent field e(x),
+// 2^(e(x) - bias) <= |x| < 2^(e(x) - bias + 1) (0 and denormals have field 0).
+template <class T> struct ExpF;
+template <> struct ExpF<double> {
+  static constexpr int digits = 52, lo = 923, hi = 1223;  // bias 1023: |x| in [2^-100, 2^201]
+  static __device__ __forceinline__ int field(const double& x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+};
+template <> struct ExpF<float> {
+  static constexpr int digits = 23, lo = 97, hi = 157;     // bias 127: |x| in [2^-30, 2^31]
+  static __device__ __forceinline__ int field(const float& x) { return (__float_as_int(x) >> 23) & 0xff; }
+};
+
+// Whether the deflation test at row k certainly fails: |H[k,k-1]| > eps (|H[k-1,k-1]| + |H[k,k]|), all
+// of moderate size (so that it is not below the absolute threshold either).
+template <class T>
+__device__ __forceinline__ bool no_split(const T& hk, const T& hkk, const T& hkm1) {
+  using E = ExpF<T>;
+  const int e = E::field(hk), m = max(E::field(hkk), E::field(hkm1));
+  return e > E::lo && m > 0 && e > m + 2 - E::digits;
+}
+
+// Whether the start-row test at row m certainly fails:
+//   |h10| (|v1| + |v2|) > eps |v0| d,  with |v1| + |v2| >= |h21 h32| / c, |v0| <= (|h21 h12| +
+//   |(h11 - r1r)(h11 - r2r)| + |r1i r2i|) / c for the same c > 0 and d the sum of three moduli;
+// entries outside the moderate range go to the test itself.
+template <class T>
+__device__ __forceinline__ bool no_start(const T& h10, const T& h21, const T& h32, const T& h12, const T& h11,
+                                         const T& h00, const T& h22, T r1r, T r1i, T r2r, T r2i) {
+  using E = ExpF<T>;
+  const int e10 = E::field(h10), e21 = E::field(h21), e32 = E::field(h32), e11 = E::field(h11);
+  const int x = max(e11, E::field(r1r)), y = max(e11, E::field(r2r));
+  const int e12 = E::field(h12), i1 = E::field(r1i), i2 = E::field(r2i);
+  const int d = max(E::field(h00), max(e11, E::field(h22)));
+  if (min(e10, min(e21, e32)) < E::lo || max(max(max(e21, e12), max(x, y)), max(max(i1, i2), d)) > E::hi) return false;
+  const int t = max(e21 + e12, max(x + y + 2, i1 + i2));
+  // lhs >= 2^(e10 + e21 + e32 - 3 bias); rhs < 2^-digits 2^(t - 2 bias + 2 + 2) 2^(d - bias + 1 + 2)
+  return e10 + e21 + e32 > t + d + 7 - E::digits;
+}
+
+// The start vector's first entry and its reflector, with the sums and products fused as in the
+// per-lane start code that they replace (FP64: a rounding here changes the iteration's path).
+__device__ __forceinline__ float start_v0(float a, float b, float c, float d, float e, float f) { return a * b + c * d - e * f; }
+__device__ __forceinline__ double start_v0(double a, double b, double c, double d, double e, double f) {
+  return fma(-e, f, fma(a, b, c * d));
+}
+__device__ __forceinline__ Refl<float> start_refl(float a, float x1, float x2, int lane) { return chain_refl(a, x1, x2, 3, lane); }
+__device__ __forceinline__ Refl<double> start_refl(double a, double x1, double x2, int lane) {
+  const double xs = fma(x1, x1, x2 * x2);
+  const double ss = fma(a, a, xs);
+  const long long sb = __double_as_longlong(ss);
+  if (__double_as_longlong(xs) == 0 || sb <= __double_as_longlong(1.0e-290) || sb >= __double_as_longlong(1.0e290)) {
+    const double t1 = reflector_fast(a, x1, x2, 3);
+    return {t1, t1 * x1, t1 * x2, x1, x2};
+  }
+  const double y = rsqrt_nr(ss);
+  const double aa = fabs(a);
+  const double tau = fma(aa, y, 1.0);
+  const double t = copysign(rcp_nr(fma(ss, y, aa)), a);
+  const double v = ((lane & 1) ? x2 : x1) * t;
+  const double tv = tau * v;
+  return {tau, __shfl_sync(0xffffffffu, tv, 0), __shfl_sync(0xffffffffu, tv, 1), __shfl_sync(0xffffffffu, v, 0),
+          __shfl_sync(0xffffffffu, v, 1)};
+}
+
 // Chain warp: steps ka..ka+nst-1 inside the window (columns ..wl, rows ka-1..).  r: the reflector of
 // step ka on entry, of step ka+nst on return.  The loop is written for few instructions and no
 // branches: one warp runs it alone, so each costs about four cycles.  Lanes outside the window
@@ -848,10 +912,12 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
           bool split = false;
           if (k >= istart + 1) {
             const T hk = HH(k, k - 1);
-            if (fabs(hk) < smallnum) {
+            const T hkk = HH(k, k), hkm1 = HH(k - 1, k - 1);
+            if (no_split(hk, hkk, hkm1)) {
+              split = false;
+            } else if (fabs(hk) < smallnum) {
               split = true;
             } else {
-              const T hkk = HH(k, k), hkm1 = HH(k - 1, k - 1);
               T t = fabs(hkm1) + fabs(hkk);
               if (t == T(0)) {
                 if (k > 2) t += fabs(HH(k - 1, k - 2));
@@ -929,37 +995,48 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
         // start row (GenericSchur.jl:850-872): largest m with two small subdiagonals, else
         // istart; the start vector comes with it
         int mx = istart;
-        T v0 = T(0), v1 = T(0), v2 = T(0);
-        for (int top = iend - 2; top >= istart; top -= 32) {
+        for (int top = iend - 2; top >= istart + 1; top -= 32) {
           const int m = top - lane;
           bool hit = false;
-          if (m >= istart) {
+          if (m >= istart + 1 &&
+              !no_start(HH(m, m - 1), HH(m + 1, m), HH(m + 2, m + 1), HH(m, m + 1), HH(m, m), HH(m - 1, m - 1),
+                        HH(m + 1, m + 1), r1r, r1i, r2r, r2i)) {
             T h21s = HH(m + 1, m);
             T s = fabs(HH(m, m) - r2r) + fabs(r2i) + fabs(h21s);
             h21s /= s;
-            v0 = h21s * HH(m, m + 1) + (HH(m, m) - r1r) * ((HH(m, m) - r2r) / s) - r1i * (r2i / s);
-            v1 = h21s * (HH(m, m) + HH(m + 1, m + 1) - r1r - r2r);
-            v2 = h21s * HH(m + 2, m + 1);
+            T v0 = h21s * HH(m, m + 1) + (HH(m, m) - r1r) * ((HH(m, m) - r2r) / s) - r1i * (r2i / s);
+            T v1 = h21s * (HH(m, m) + HH(m + 1, m + 1) - r1r - r2r);
+            T v2 = h21s * HH(m + 2, m + 1);
             s = fabs(v0) + fabs(v1) + fabs(v2);
             v0 /= s; v1 /= s; v2 /= s;
-            hit = m == istart ||
-                  fabs(HH(m, m - 1)) * (fabs(v1) + fabs(v2)) <=
-                      eps * fabs(v0) * (fabs(HH(m - 1, m - 1)) + fabs(HH(m, m)) + fabs(HH(m + 1, m + 1)));
+            hit = fabs(HH(m, m - 1)) * (fabs(v1) + fabs(v2)) <=
+                  eps * fabs(v0) * (fabs(HH(m - 1, m - 1)) + fabs(HH(m, m)) + fabs(HH(m + 1, m + 1)));
           }
           const unsigned bal = __ballot_sync(0xffffffffu, hit);
-          if (bal) {
-            const int q = __ffs(bal) - 1;
-            mx = top - q;
-            v0 = __shfl_sync(0xffffffffu, v0, q);
-            v1 = __shfl_sync(0xffffffffu, v1, q);
-            v2 = __shfl_sync(0xffffffffu, v2, q);
-            break;
-          }
+          if (bal) { mx = top - (__ffs(bal) - 1); break; }
+        }
+        // the start vector, its two triples of quotients one division each
+        T v0, v1, v2;
+        {
+          const int q = lane % 3;
+          const T h11 = HH(mx, mx);
+          T h21s = HH(mx + 1, mx);
+          T s = fabs(h11 - r2r) + fabs(r2i) + fabs(h21s);
+          T w = (q == 0 ? h21s : (q == 1 ? h11 - r2r : r2i)) / s;
+          h21s = __shfl_sync(0xffffffffu, w, 0);
+          const T ds = __shfl_sync(0xffffffffu, w, 1), rs = __shfl_sync(0xffffffffu, w, 2);
+          v0 = start_v0(h21s, HH(mx, mx + 1), h11 - r1r, ds, r1i, rs);
+          v1 = h21s * (h11 + HH(mx + 1, mx + 1) - r1r - r2r);
+          v2 = h21s * HH(mx + 2, mx + 1);
+          s = fabs(v0) + fabs(v1) + fabs(v2);
+          w = (q == 0 ? v0 : (q == 1 ? v1 : v2)) / s;
+          v0 = __shfl_sync(0xffffffffu, w, 0);
+          v1 = __shfl_sync(0xffffffffu, w, 1);
+          v2 = __shfl_sync(0xffffffffu, w, 2);
         }
         // reflector of the first step from the start vector
-        const T t1 = reflector_fast(v0, v1, v2, min(3, iend - mx + 1));
-        if (mx > istart && lane == 0) HH(mx, mx - 1) *= (T(1) - t1);
-        r.t1 = t1; r.v2 = v1; r.v3 = v2; r.t2 = t1 * v1; r.t3 = t1 * v2;
+        r = start_refl(v0, v1, v2, lane);  // 3 elements: mx <= iend - 2
+        if (mx > istart && lane == 0) HH(mx, mx - 1) *= (T(1) - r.t1);
         __syncwarp();
         kn = mx;
         state = 1;
@@ -1243,6 +1320,16 @@ template cudaError_t launch_schur_batched_real<float, double>(const RealBatchT<f
                                                               cudaStream_t*, int);
 template cudaError_t launch_schur_batched_real<float, float>(const RealBatchT<float, float>&, const int*, int*, int,
                                                              cudaStream_t*, int);
+
+template <class T, class W>
+cudaError_t launch_schur_real_bin(const RealBatchT<T, W>& bt, const int* order, int* sched, int bin,
+                                  const BinTuning& t, int num_sms, cudaStream_t s) {
+  return launch_shape(bt, order, sched, bin, t.bounds[bin], t.nt[bin], t.ctas[bin], num_sms, s);
+}
+template cudaError_t launch_schur_real_bin<double, double>(const RealBatchT<double, double>&, const int*, int*, int,
+                                                           const BinTuning&, int, cudaStream_t);
+template cudaError_t launch_schur_real_bin<float, float>(const RealBatchT<float, float>&, const int*, int*, int,
+                                                         const BinTuning&, int, cudaStream_t);
 
 template <class T, class W>
 cudaError_t launch_schur_real_one(const RealBatchT<T, W>& bt, int m, const int* order, int* sched, cudaStream_t s) {
