@@ -99,6 +99,16 @@ int ensure_ws(gs_context* ctx, size_t bytes) {
   return GS_OK;
 }
 
+// The stream of the i-th largest size bin: the larger the orders, the higher the priority, so that the
+// longest-running matrices start first whenever room appears on an SM.  With equal priorities the bins'
+// order was left to chance: 2000 FP64 matrices n = 8..128 took 61 ms or 74 ms.
+cudaError_t bin_stream(cudaStream_t* s, int i) {
+  int least = 0, greatest = 0;
+  cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+  if (e != cudaSuccess) return e;
+  return cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, std::min(least, greatest + i));
+}
+
 // Fork the aux streams off `s`, run `body(aux)`, join back into `s`.
 template <class F> int fork_join(gs_context* ctx, cudaStream_t s, F body) {
   CK(cudaEventRecord(ctx->fork, s));
@@ -137,7 +147,7 @@ int gs_create(gs_context** out, int device) {
       break;
     }
     for (int i = 0; i < kNumBins && e == cudaSuccess; ++i) {
-      e = cudaStreamCreateWithFlags(&ctx->aux[i], cudaStreamNonBlocking);
+      e = bin_stream(&ctx->aux[i], i);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->join[i], cudaEventDisableTiming);
     }
     if (e != cudaSuccess) { rc = set_err(ctx, GS_CUDA, "aux streams: %s", cudaGetErrorString(e)); break; }
@@ -379,7 +389,7 @@ static int pipe_setup(gs_context* ctx) {
     CK(cudaEventCreateWithFlags(&ctx->pipe_fork[c], cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ctx->pipe_done[c], cudaEventDisableTiming));
     for (int i = 0; i < kNumBins; ++i) {
-      CK(cudaStreamCreateWithFlags(&ctx->pipe_aux[c][i], cudaStreamNonBlocking));
+      CK(bin_stream(&ctx->pipe_aux[c][i], i));
       CK(cudaEventCreateWithFlags(&ctx->pipe_join[c][i], cudaEventDisableTiming));
     }
   }

@@ -9,6 +9,8 @@
 //                 deflation, Wilkinson / exceptional shifts, 2-element reflector chase, the
 //                 phase fix-ups that keep the subdiagonal real, on a packed upper-Hessenberg copy
 //                 in shared memory; T = triu(H), w = diag(T), scaling undone.
+#include <algorithm>
+
 #include "device_common.cuh"
 #include "gs_internal.h"
 
@@ -799,7 +801,7 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
 template <int NT>
 __global__ void __launch_bounds__(NT, NT <= 128 ? 512 / NT : 2) k_schur_cplx(CplxBatch bt, const int* __restrict__ order,
                                                                 int* __restrict__ sched, int bin, int nmax,
-                                                                int num_sms) {
+                                                                int num_sms, int once) {
   extern __shared__ double2 smemz[];
   __shared__ int s_job;
   const int start = sched[3 * bin], end = sched[3 * bin + 1];
@@ -807,6 +809,11 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 512 / NT : 2) k_schur_cplx(Cpl
   constexpr int NW = NT / 32;
   const int slot = blockIdx.x / num_sms;
   const int cw = NW % 4 == 0 ? slot % 4 : (NW % 2 == 0 ? (slot >> 1) & 1 : 0);
+  if (once) {  // a CTA per matrix
+    const int job = start + blockIdx.x;
+    if (job < end) solve_cplx<NT>(bt, order[job], nmax, smemz, cw);
+    return;
+  }
   for (;;) {
     if (threadIdx.x == 0) s_job = start + atomicAdd(&sched[3 * bin + 2], 1);
     __syncthreads();
@@ -830,12 +837,7 @@ cudaError_t launch_hess_c(const CplxBatch& bt, const int* order, const int* sche
   const size_t elems = chess_smem_elems(nmax), smem = sizeof(double2) * elems;
   cudaError_t e = cudaFuncSetAttribute(k_hess_cplx<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hess_cplx<NC>, 4 * NC, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
-  const int ctas = num_sms * per_sm < bt.count ? num_sms * per_sm : bt.count;
-  k_hess_cplx<NC><<<ctas, 4 * NC, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
+  k_hess_cplx<NC><<<bt.count, 4 * NC, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
   return cudaGetLastError();
 }
 
@@ -853,9 +855,9 @@ cudaError_t launch_bin_c(const CplxBatch& bt, const int* order, int* sched, int 
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_cplx<NT>, NT, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
-  if (ctas > 0 && per_sm > ctas) per_sm = ctas;
-  const int grid = num_sms * per_sm < bt.count ? num_sms * per_sm : bt.count;
-  k_schur_cplx<NT><<<grid, NT, smem, s>>>(bt, order, sched, bin, nmax, num_sms);
+  int grid = bt.count;  // as launch_bin of schur_batched_real.cu
+  if (ctas > 0) grid = std::min(grid, num_sms * std::min(per_sm, ctas));
+  k_schur_cplx<NT><<<grid, NT, smem, s>>>(bt, order, sched, bin, nmax, num_sms, ctas > 0 ? 0 : 1);
   return cudaGetLastError();
 }
 

@@ -13,6 +13,7 @@
 // They are separate kernels because they want different shapes: the reduction needs the full
 // matrix (and Z) in shared memory and many threads, the iteration is a chain of short
 // dependent steps per matrix that wants as many matrices per SM as fit.
+#include <algorithm>
 #include <type_traits>
 
 #include "device_common.cuh"
@@ -1185,7 +1186,7 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
 // 768 threads per SM: at most 80 registers
 template <class T, class W, int NT>
 __global__ void __launch_bounds__(NT, 768 / NT) k_schur_real(RealBatchT<T, W> bt, const int* __restrict__ order,
-                                                   int* __restrict__ sched, int bin, int nmax, int num_sms) {
+                                                   int* __restrict__ sched, int bin, int nmax, int num_sms, int once) {
   extern __shared__ double smem_raw[];
   T* smem = (T*)smem_raw;
   __shared__ int s_job;
@@ -1195,6 +1196,11 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_schur_real(RealBatchT<T, W> bt
   constexpr int NW = NT / 32;
   const int slot = blockIdx.x / num_sms;
   const int cw = NW % 4 == 0 ? slot % 4 : (NW % 2 == 0 ? (slot >> 1) & 1 : 0);
+  if (once) {  // a CTA per matrix
+    const int job = start + blockIdx.x;
+    if (job < end) solve_real<T, W, NT>(bt, order[job], nmax, smem, cw);
+    return;
+  }
   for (;;) {
     if (threadIdx.x == 0) s_job = start + atomicAdd(&sched[3 * bin + 2], 1);
     __syncthreads();
@@ -1225,21 +1231,12 @@ cudaError_t launch_hess(const RealBatchT<T, W>& bt, const int* order, const int*
   else f = (const void*)k_hess_real32<W, NC>;
   cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  auto grid = [&](const void* k, int nt, size_t sm) -> int {
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, sm)) != cudaSuccess) return 0;
-    const int ctas = num_sms * (per_sm < 1 ? 1 : per_sm);
-    return ctas < bt.count ? ctas : bt.count;
-  };
-  int ctas = grid(f, NT, smem);
-  if (e != cudaSuccess) return e;
+  const int ctas = bt.count;
   if constexpr (sizeof(T) == 8) {
     k_hess_real64<W, NC><<<ctas, NT, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
   } else {
     k_hess_real32<W, NC><<<ctas, NT, smem, s>>>(bt, order, sched, bin, nmax);
     if (bt.wantz) {
-      ctas = grid((const void*)k_formq_real32<W, NC>, 2 * NC, 0);
-      if (e != cudaSuccess) return e;
       k_formq_real32<W, NC><<<ctas, 2 * NC, 0, s>>>(bt, order, sched, bin, nmax);
     }
   }
@@ -1260,9 +1257,11 @@ cudaError_t launch_bin(const RealBatchT<T, W>& bt, const int* order, int* sched,
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_real<T, W, NT>, NT, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
-  if (ctas > 0 && per_sm > ctas) per_sm = ctas;
-  const int grid = num_sms * per_sm < bt.count ? num_sms * per_sm : bt.count;
-  k_schur_real<T, W, NT><<<grid, NT, smem, s>>>(bt, order, sched, bin, nmax, num_sms);
+  // a CTA per matrix (those beyond the bin's share end at once), or, with a cap on CTAs per SM, as
+  // many as may be resident on a ticket queue
+  int grid = bt.count;
+  if (ctas > 0) grid = std::min(grid, num_sms * std::min(per_sm, ctas));
+  k_schur_real<T, W, NT><<<grid, NT, smem, s>>>(bt, order, sched, bin, nmax, num_sms, ctas > 0 ? 0 : 1);
   return cudaGetLastError();
 }
 
