@@ -7,8 +7,9 @@
 //   k_schur_cplx  single-shift complex QR of gschur!(H::Hessenberg{Complex}, Z)
 //                 (GenericSchur.jl:194-335) with singleShiftQR! (374-504): Ahues-Tisseur
 //                 deflation, Wilkinson / exceptional shifts, 2-element reflector chase, the
-//                 phase fix-ups that keep the subdiagonal real, on a packed upper-Hessenberg copy
-//                 in shared memory; T = triu(H), w = diag(T), scaling undone.
+//                 phase fix-ups that keep the subdiagonal real, in the (L2-resident) output buffer
+//                 with the window around the diagonal in shared memory; T = triu(H),
+//                 w = diag(T), scaling undone.
 #include <algorithm>
 
 #include "device_common.cuh"
@@ -17,12 +18,7 @@
 namespace gsk {
 namespace {
 
-// Column offset in the packed layout of the QR phase: column j (1-based) holds
-// rows 1..j+2 contiguously -- the upper Hessenberg part plus the row of the
-// single-shift bulge, H[k+1, k-1].
-__host__ __device__ __forceinline__ int pk_off(int j) { return ((j - 1) * (j + 4)) >> 1; }
-#define HH(i, j) H[pk_off(j) + (i) - 1]
-
+#define HH(i, j) H[((i) - 1) + ((j) - 1) * n]
 
 // ---------------------------------------------------------------------------------
 // Hessenberg reduction and Q formation: 4*NC threads (NC >= n).  Thread (c, p) of the first 2*NC
@@ -287,8 +283,11 @@ __global__ void __launch_bounds__(4 * NC) k_hess_cplx(CplxBatch bt, const int* _
 // a step takes 6 for the left update, 6 for the right and 23 for the reflector.
 // A sweep that starts below istart is rare: its first step is a chunk of its own, after which the far
 // warps also apply the phase that keeps H[k0+1, k0] real to every element (GenericSchur.jl:461-482).
+// H stays in the output buffer; only the window of a chunk is in shared memory, so that several
+// matrices of any order share an SM's FP64 pipe, which bounds the batch (a packed copy of one
+// order-128 matrix filled the SM, whose pipe was then 53% busy: 1824 of them took 980 ms).
 // Why: one CTA barrier per step with the near block's complex arithmetic on single lanes and the Z pass
-// after each sweep took 98 ms for one matrix of order 128, which fills an SM's shared memory.
+// after each sweep took 98 ms for one matrix of order 128.
 struct ZCmd {
   int type;     // 0 nothing, 1 chunk, 2 done
   int ka, nst;  // steps ka .. ka+nst-1
@@ -308,6 +307,8 @@ constexpr int kZChunk = 12;  // steps of a chunk of a longer sweep
 constexpr int kZMinChunk = 3;
 constexpr int kZLog = 3;     // double2 per step: t1, v2, (t2, 0)
 constexpr int kZLogElems = kZLog * (kZWin + 1);
+constexpr int kZLd = 17;     // the window: 16 columns of 16 rows at this distance
+constexpr int kZWinElems = 16 * kZLd;
 
 template <int NT> __device__ __forceinline__ void zphase_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); }
 template <int NT> __device__ __forceinline__ void zfar_barrier() { asm volatile("bar.sync 2, %0;" ::"n"(NT - 32) : "memory"); }
@@ -324,32 +325,26 @@ __device__ __forceinline__ double2 zslide(const ZR& r, double ty, double vy, dou
 
 __device__ __forceinline__ ZR ld_zr(const double2* l) { return {l[0], l[1], l[2].x}; }
 
-// The logged reflectors on one line: element e+1 follows element e at distance inc, growing by d.
-__device__ __forceinline__ double2* zapply_line(double2* p, int inc, int d, const double2* lg, int nst, bool left) {
+// The logged reflectors on one line, whose elements are inc apart; returns the last element.
+__device__ __forceinline__ double2* zapply_line(double2* p, int inc, const double2* lg, int nst, bool left) {
   double2 z0 = *p;
-  double2* q = p + inc;
-  inc += d;
   int s = 0;
-  for (; s + 2 <= nst; s += 2, lg += 2 * kZLog) {
-    double2* q2 = q + inc;
-    const double2 y0 = *q, y1 = *q2;
-    {
-      const ZR r = ld_zr(lg);
-      *p = zslide(r, left ? -r.t1.y : r.t1.y, left ? r.v2.y : -r.v2.y, z0, y0);
+  for (; s + 4 <= nst; s += 4, lg += 4 * kZLog) {
+    double2 y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[e] = p[(e + 1) * inc];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const ZR r = ld_zr(lg + e * kZLog);
+      p[e * inc] = zslide(r, left ? -r.t1.y : r.t1.y, left ? r.v2.y : -r.v2.y, z0, y[e]);
     }
-    {
-      const ZR r = ld_zr(lg + kZLog);
-      *q = zslide(r, left ? -r.t1.y : r.t1.y, left ? r.v2.y : -r.v2.y, z0, y1);
-    }
-    p = q2;
-    q = q2 + inc + d;
-    inc += 2 * d;
+    p += 4 * inc;
   }
-  if (s < nst) {
-    const double2 y0 = *q;
+  for (; s < nst; ++s, lg += kZLog) {
+    const double2 y0 = p[inc];
     const ZR r = ld_zr(lg);
     *p = zslide(r, left ? -r.t1.y : r.t1.y, left ? r.v2.y : -r.v2.y, z0, y0);
-    p = q;
+    p += inc;
   }
   *p = z0;
   return p;
@@ -404,23 +399,28 @@ __device__ __forceinline__ bool no_zstart(const double& h10, const double& h21, 
   return e10 + e21 > x + d + 6 - 52;
 }
 
-// Chain warp: steps ka..ka+nst-1 inside the window (columns ..wl, rows ka-1..).  r: the reflector of
-// step ka on entry, of step ka+nst on return (unless that is past the sweep, or fix: the phase fix-up
-// comes before it).
-__device__ __forceinline__ void zchase_chunk(double2* H, int ka, int nst, int iend, int wl, bool fix, ZR& r,
-                                             double2* lg, int lane) {
+// Chain warp: steps ka..ka+nst-1 inside the window (columns ..wl, rows ka-1..), which is loaded into W and
+// stored back.  r: the reflector of step ka on entry, of step ka+nst on return (unless that is past the
+// sweep, or fix: the phase fix-up comes before it).
+__device__ __forceinline__ void zchase_chunk(double2* H, int n, double2* W, int ka, int nst, int iend, int wl, bool fix,
+                                             ZR& r, double2* lg, int lane) {
+  // rows ka-1.. of column ka+c at W[c * kZLd]
+  const int wr = lane & 15, gr = ka - 1 + wr;  // row of the window, of H
+  const bool rin = gr >= 1 && gr <= min(ka + nst + 1, iend);
+  for (int c = lane >> 4; c <= wl - ka; c += 2)
+    if (rin) async_load(&W[wr + c * kZLd], &HH(gr, ka + c));
+  async_wait();
+  __syncwarp();
   const unsigned all = 0xffffffffu;
   const int p = lane & 1, e = lane >> 1;
   const int j = min(ka + e, wl);
   const bool colok = ka + e <= wl;
-  double2* hc = H + pk_off(j) + ka - 1;  // H(k, j)
+  double2* hc = W + (j - ka) * kZLd + 1;  // H(k, j)
   const int i = ka - 1 + e;
   const bool rowok = i >= 1 && i <= iend;
-  const int ic = min(max(i, 1), iend) - 1;
-  int c0 = pk_off(ka);
-  double2* p0 = H + c0 + ic;             // H(i, k), H(i, k+1)
-  double2* p1 = p0 + ka + 2;
-  double2* hb = H + c0 + ka;             // H(k+1, k)
+  double2* p0 = W + e;                    // H(i, k), H(i, k+1)
+  double2* p1 = p0 + kZLd;
+  double2* hb = W + 2;                    // H(k+1, k)
   for (int s = 0; s < nst; ++s) {
     const int k = ka + s;
     if (lane == 0) { lg[0] = r.t1; lg[1] = r.v2; lg[2] = make_double2(r.t2, 0.0); }
@@ -463,10 +463,13 @@ __device__ __forceinline__ void zchase_chunk(double2* H, int ka, int nst, int ie
       if (lane == 0) { hb[0] = a; hb[1] = make_double2(0.0, 0.0); }
     }
     ++hc;
-    hb += k + 3;
+    hb += kZLd + 1;
     p0 = p1;
-    p1 += k + 3;
+    p1 += kZLd;
   }
+  __syncwarp();
+  for (int c = lane >> 4; c <= wl - ka; c += 2)
+    if (rin) HH(gr, ka + c) = W[wr + c * kZLd];
   __syncwarp();
 }
 
@@ -488,7 +491,8 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
   double2* Zg = bt.wantz ? bt.Z + bt.offs[b] : nullptr;
   double2* wg = bt.w + bt.woffs[b];
   double2* logs = smem;
-  double2* H = smem + 2 * kZLogElems;
+  double2* W = smem + 2 * kZLogElems;
+  double2* H = Ag;
   // the scale that k_hess_cplx applied
   const double amax = wg[0].x;
   const double smlnum = sqrt(kSafemin) / kEps;
@@ -499,9 +503,7 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
     if (amax > 0.0 && amax < smlnum) { scaled = true; cscale = smlnum; }
     else if (amax > bignum) { scaled = true; cscale = bignum; }
   }
-  for (int j = 1 + warp; j <= n; j += NT / 32)
-    for (int i = 1 + lane; i <= j + 2; i += 32)
-      HH(i, j) = (i <= min(j + 1, n)) ? Ag[(i - 1) + (j - 1) * n] : make_double2(0.0, 0.0);
+  for (int j = 1 + tid; j <= n - 2; j += NT) HH(j + 2, j) = make_double2(0.0, 0.0);  // the bulge's row
   __syncthreads();
   const double ulp = kEps;
   const double smallnum = kSafemin * ((double)n / ulp);
@@ -659,7 +661,7 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
             // urgent columns: the previous chunk's left updates on the columns entering the window
             const double2* pl = logs + ((ph & 1) ^ 1) * kZLogElems;
             const int j = pwl + 1 + lane;
-            if (j <= wl) zapply_line(&HH(pka, j), 1, 0, pl, pnst, true);
+            if (j <= wl) zapply_line(&HH(pka, j), 1, pl, pnst, true);
             __syncwarp();
           }
           double2 pht = make_double2(1.0, 0.0);
@@ -667,7 +669,7 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
             pht = zsub(pht, r.t1);
             pht = zscal(pht, 1.0 / hypot(pht.x, pht.y));
           }
-          zchase_chunk(H, kn, nst, iend, wl, fix, r, lg, lane);
+          zchase_chunk(H, n, W, kn, nst, iend, wl, fix, r, lg, lane);
           if (fix) {
             if (lane == 0) {
               HH(kn + 1, kn) = zmul(HH(kn + 1, kn), zconj(pht));
@@ -735,20 +737,19 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
         const int nl = n - jfar + 1, nr = max(ka - 2, 0), nz = Zg ? n : 0;
         for (int t = ft; t < nl + nr + nz; t += NT - 32) {
           double2* p;
-          int inc, d = 0;
+          int inc;
           const bool left = t < nl;
           if (left) {
             p = &HH(ka, jfar + t);
             inc = 1;
           } else if (t < nl + nr) {
             p = &HH(t - nl + 1, ka);
-            inc = ka + 2;
-            d = 1;
+            inc = n;
           } else {
             p = Zg + (t - nl - nr) + (ka - 1) * n;
             inc = n;
           }
-          p = zapply_line(p, inc, d, lg, nst, left);
+          p = zapply_line(p, inc, lg, nst, left);
           if (tail_on && !cm.fix) *p = zmul(*p, left ? zconj(tail) : tail);
         }
         if (cm.fix) {
@@ -788,7 +789,7 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
   if (scaled) nf = safescale_factors(cscale, amax, mul);
   for (int idx = tid; idx < n * n; idx += NT) {
     const int i = idx % n, j = idx / n;
-    double2 v = (i > j) ? make_double2(0.0, 0.0) : HH(i + 1, j + 1);
+    double2 v = (i > j) ? make_double2(0.0, 0.0) : Ag[idx];
     for (int f = 0; f < nf; ++f) v = zscal(v, mul[f]);
     Ag[idx] = v;
     if (i == j) wg[i] = v;
@@ -825,7 +826,7 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 512 / NT : 2) k_schur_cplx(Cpl
 }
 
 // Dynamic shared memory of one CTA of the iteration and of the reduction for orders up to nmax.
-size_t ciqr_smem_bytes(int nmax) { return sizeof(double2) * (2 * kZLogElems + (size_t)pk_off(nmax + 1)); }
+size_t ciqr_smem_bytes() { return sizeof(double2) * (2 * kZLogElems + kZWinElems); }
 size_t chess_smem_elems(int nmax) {
   const size_t one = (size_t)nmax * (nmax | 1), most = (kMaxDynSmem - 8 * 1024) / sizeof(double2);
   return one <= most ? one : most;
@@ -848,7 +849,7 @@ cudaError_t launch_bin_c(const CplxBatch& bt, const int* order, int* sched, int 
                              : (nmax <= 64 ? launch_hess_c<64>(bt, order, sched, bin, nmax, num_sms, s)
                                            : launch_hess_c<128>(bt, order, sched, bin, nmax, num_sms, s));
   if (e != cudaSuccess) return e;
-  const size_t smem = ciqr_smem_bytes(nmax);
+  const size_t smem = ciqr_smem_bytes();
   e = cudaFuncSetAttribute(k_schur_cplx<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
@@ -895,7 +896,7 @@ cudaError_t launch_schur_batched_cplx(const CplxBatch& bt, const int* order, int
 // matrix fits); a row that asks for it where a full matrix does not fit is refused as before.
 size_t cplx_bin_smem_bytes(int nmax, int hsmem) {
   const size_t full = hsmem ? sizeof(double2) * ((size_t)nmax * (nmax | 1) + 4 * (size_t)nmax) + 32 * sizeof(double) + 64 : 0;
-  return full > ciqr_smem_bytes(nmax) ? full : ciqr_smem_bytes(nmax);
+  return full > ciqr_smem_bytes() ? full : ciqr_smem_bytes();
 }
 
 cudaError_t launch_schur_cplx_bin(const CplxBatch& bt, const int* order, int* sched, int bin, const BinTuning& t,
