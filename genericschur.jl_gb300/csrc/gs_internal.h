@@ -186,6 +186,9 @@ cudaError_t launch_ggschur_real(const QzrBatch& bt, int num_sms, cudaStream_t s)
 struct HeCtlBuf {
   alignas(16) unsigned char bytes[64];
 };
+// where the control block holds the int that says that a grid-wide wait gave up
+template <class S> constexpr size_t kHeErrOffset = 2 * sizeof(S) + 4 * sizeof(unsigned);
+// W: 2 n entries
 template <class S>
 cudaError_t launch_he_tridiag(const S* A, long long lda, int n, int upper, S* B, S* W, S* partial, int npart,
                               HeCtlBuf* ctl, S* tau, double* d, double* e, int num_sms, cudaStream_t s);

@@ -3052,7 +3052,7 @@ template <class S> HeLayout he_layout(int64_t n, bool host_a, bool wantq, int nu
   L.npart = std::max(1, 4 * num_sms);
   L.o_A = ar.take<S>(host_a ? nn : 1);
   L.o_B = ar.take<S>(std::max<size_t>(nn, 1));
-  L.o_W = ar.take<S>(std::max<int64_t>(n, 1));
+  L.o_W = ar.take<S>(2 * std::max<int64_t>(n, 1));
   L.o_part = ar.take<S>(L.npart);
   L.o_ctl = ar.take<HeCtlBuf>(1);
   L.o_tau = ar.take<S>(std::max<int64_t>(n, 1));
@@ -3140,8 +3140,11 @@ int heev_impl(gs_context* ctx, int64_t n, double* A, int64_t lda, int uplo, doub
   if (rc == GS_CUDA) return rc;
   // sorteig!(w, V, eigsortby): stable ascending order
   std::vector<double> dh(n);
+  int gave_up = 0;
   CK(cudaMemcpyAsync(dh.data(), d, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(&gave_up, base + L.o_ctl + kHeErrOffset<S>, sizeof(int), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
+  if (gave_up) return set_err(ctx, GS_CUDA, "tridiagonalization: a grid-wide wait gave up");
   std::vector<int> p(n);
   for (int64_t i = 0; i < n; ++i) p[i] = (int)i;
   std::stable_sort(p.begin(), p.end(), [&](int a, int b) { return dh[a] < dh[b]; });
@@ -3197,12 +3200,15 @@ int hetrd_impl(gs_context* ctx, int64_t n, double* A, int64_t lda, int uplo, dou
   // d, e, tau to the host (reversed for the upper form), then out
   std::vector<double> hd(n), he(n > 1 ? n - 1 : 1);
   std::vector<S> ht(n > 1 ? n - 1 : 1);
+  int gave_up = 0;
+  CK(cudaMemcpyAsync(&gave_up, base + L.o_ctl + kHeErrOffset<S>, sizeof(int), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(hd.data(), dd, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   if (n > 1) {
     CK(cudaMemcpyAsync(he.data(), de, sizeof(double) * (n - 1), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(ht.data(), dtau, sizeof(S) * (n - 1), cudaMemcpyDeviceToHost, s));
   }
   CK(cudaStreamSynchronize(s));
+  if (gave_up) return set_err(ctx, GS_CUDA, "tridiagonalization: a grid-wide wait gave up");
   if (upper) {
     std::reverse(hd.begin(), hd.end());
     if (n > 1) {

@@ -4,7 +4,9 @@
 //
 // 1. Tridiagonalization (zhetd2, lower form): the matrix is kept full (both triangles,
 //    exactly Hermitian) in a device work array so that every access is a column read.
-//    Step i, two launches:
+//    Where it fits in the shared memory of the chip (real n up to about 1900, complex
+//    about 1300), k_he_tridiag runs all steps in one cooperative launch; above that each
+//    step i is two launches:
 //      k_he_matvec  w = tau A22 v, warp per column j (w_j = tau sum_k conj(A22[k,j]) v_k),
 //                   per-CTA partial dots; the last CTA (ticket) forms
 //                   alpha = -(tau/2) w^H v;
@@ -14,8 +16,10 @@
 //    Hermitian(A, :U) is the lower form applied to J A J (J the index reversal): the
 //    reference's :U sweep (hessenberg.jl:60-96) takes the same reflectors with their
 //    tails in the opposite order, so the results agree up to summation order.
-// 2. Q = H_1 ... H_{n-1} accumulated backwards into the identity (k_he_formq, one launch
-//    per reflector, warp per column: y_j = u^H Q[:,j], Q[:,j] -= tau u y_j).
+// 2. Q = H_1 ... H_{n-1} accumulated backwards into the identity, warp per column
+//    (y_j = u^H Q[:,j], Q[:,j] -= tau u y_j): k_he_formq_cols, one launch with the columns
+//    in shared memory, or, where four columns do not fit in a CTA, k_he_formq, one launch
+//    per reflector.
 // 3. Tridiagonal QR (k_steqr): one cooperative kernel.  Thread 0 of block 0 runs the
 //    reference's state machine (splits, scaling, QL or QR per block, 2x2 deflation,
 //    Givens sweeps with LinearAlgebra's givensAlgorithm); each sweep's rotations go to a
@@ -26,10 +30,14 @@
 #include "device_common.cuh"
 #include "gs_internal.h"
 
+#include <cstddef>
+
 namespace gsk {
 namespace {
 
 constexpr int kHeT = 256;
+constexpr int kHeOneCta = 32;  // orders of k_he_tridiag that one CTA takes alone
+constexpr int kHeCols = 4;     // columns per CTA above that, until every SM has a CTA
 
 template <class S> struct Hs;
 template <> struct Hs<double> {
@@ -75,9 +83,15 @@ template <class S> __device__ __forceinline__ S warp_sum(S v) {
 template <class S> struct HeCtl {
   S tau;          // reflector of the current step
   S alpha;        // -(tau/2) w^H v
-  unsigned t_mv;  // ticket of k_he_matvec
-  unsigned t_up;  // ticket of k_he_update
+  unsigned t_mv;    // ticket of k_he_matvec
+  unsigned t_up;    // ticket of k_he_update
+  unsigned arrive;  // k_he_tridiag: CTAs that have written their part of w, over all steps
+  unsigned ready;   // k_he_tridiag: number of reflectors published
+  int err;          // a wait of k_he_tridiag gave up
 };
+static_assert(sizeof(HeCtl<double2>) <= sizeof(HeCtlBuf), "control block");
+static_assert(offsetof(HeCtl<double>, err) == kHeErrOffset<double> && offsetof(HeCtl<double2>, err) == kHeErrOffset<double2>,
+              "the host reads err at this offset");
 
 // Full Hermitian matrix B (ld n) in the lower-form frame from the triangle `upper` of A.
 template <class S>
@@ -227,6 +241,253 @@ __global__ void __launch_bounds__(kHeT) k_he_formq(const S* __restrict__ B, int 
       const S uk = k == 0 ? O::one() : u[k];
       q[k] = O::sub(q[k], O::mul(ts, uk));
     }
+  }
+}
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Wait until *p >= target (all CTAs are resident).  Gives up, and sets *err, after some
+// seconds or when another CTA has.
+__device__ bool he_wait(const unsigned* p, unsigned target, int* err) {
+  for (int it = 0; ld_acquire(p) < target; ++it) {
+    if (it >= (1 << 22)) atomicOr(err, 1);
+    if ((it & 1023) == 1023 && *(volatile int*)err) return false;
+  }
+  return true;
+}
+
+// Sum over the CTA, in every thread, in one order for every CTA.
+template <class V, class F> __device__ __forceinline__ V he_cta_sum(V v, V* red, F add_xor) {
+  const int lane = threadIdx.x & 31;
+  for (int o = 16; o > 0; o >>= 1) v = add_xor(v, o);
+  if (lane == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = red[lane & (kHeT / 32 - 1)];
+  for (int o = kHeT / 64; o > 0; o >>= 1) v = add_xor(v, o);
+  return v;
+}
+
+__device__ __forceinline__ double he_abs2(double a) { return a * a; }
+__device__ __forceinline__ double he_abs2(double2 a) { return fma(a.x, a.x, a.y * a.y); }
+__device__ __forceinline__ double he_acc2(double a, double s) { return fma(a, a, s); }
+__device__ __forceinline__ double he_acc2(double2 a, double s) { return fma(a.x, a.x, fma(a.y, a.y, s)); }
+
+// tau and 1 / (alpha - beta) of the reflector with head alpha and beta given.
+__device__ __forceinline__ void he_scalars(double a, double beta, double* tau, double* t) {
+  *tau = (beta - a) / beta;
+  *t = 1.0 / (a - beta);
+}
+__device__ __forceinline__ void he_scalars(double2 a, double beta, double2* tau, double2* t) {
+  *tau = make_double2((beta - a.x) / beta, -a.y / beta);
+  *t = zdiv(make_double2(1.0, 0.0), make_double2(a.x - beta, a.y));
+}
+
+// _reflector! (householder.jl:12-102) on x[0..m) in shared memory; ssq is each thread's
+// share of the tail's sum of squares.  Squares that are safe from over- and underflow give
+// the norm directly; anything else takes cta_reflector's scaled passes.
+template <class S> __device__ S he_reflector(S* x, int m, double ssq, double* red, S* bc) {
+  using O = Hs<S>;
+  const S a = x[0];  // before the sum's barrier: x[0] is written below
+  ssq = he_cta_sum(ssq, red, [](double v, int o) { return v + __shfl_xor_sync(0xffffffffu, v, o); });
+  const double tot = ssq + he_abs2(a);
+  if (!(m >= 2 && ssq >= 0x1p-900 && tot <= 0x1p900)) {
+    __syncthreads();
+    return cta_reflector<kHeT>(x, m, red);
+  }
+  if (threadIdx.x < 32) {
+    const double beta = -copysign(sqrt(tot), O::re(a));
+    S tau, t;
+    he_scalars(a, beta, &tau, &t);
+    __syncwarp();
+    if (threadIdx.x == 0) {
+      bc[0] = tau;
+      bc[1] = t;
+      x[0] = O::from(beta);
+    }
+  }
+  __syncthreads();
+  const S t = bc[1];
+  for (int k = 1 + threadIdx.x; k < m; k += kHeT) x[k] = O::mul(x[k], t);
+  __syncthreads();
+  return bc[0];
+}
+
+// The whole tridiagonalization as one cooperative kernel, the columns of the full matrix
+// in shared memory (column j in CTA j mod G, so that the trailing block stays spread).
+// Step i: every CTA takes v and tau, forms w_j = tau a_j^H v of its columns (warp per
+// column) and publishes them; after the grid's arrival count every CTA reads w, forms
+// alpha and w' = w + alpha v for itself; the CTA of column i+1 updates that column first,
+// makes its reflector and publishes it while all others update their columns.  Bound by
+// the latency of that chain (a grid-wide arrival, the reflector, a flag), not by memory.
+// Against the two launches per step, which read the matrix three times from L2 and spend
+// their time on launches, tickets and one CTA's reflector: n = 1000
+// real 24.1 ms, now 10.5 (with the launch gaps the whole call 48.8 -> 26.6 ms); 64: 2.7 -> 1.7 ms.
+// One CTA alone is as fast up to about 40 columns; 2 to 8 columns per CTA measure alike, 16
+// are 10% slower at 1000.
+// col: columns of ceil(n / G) * n elements, then v and w' (n each).  W: 2 n (by the
+// step's parity: a CTA may still read the last step's when the next is written).
+template <class S>
+__global__ void __launch_bounds__(kHeT) k_he_tridiag(S* B, int n, S* W, HeCtl<S>* ctl, S* tau, double* d, double* e) {
+  using O = Hs<S>;
+  extern __shared__ __align__(16) unsigned char he_smem[];
+  __shared__ S reds[kHeT / 32], bc[2];
+  __shared__ double red[32];
+  __shared__ int bad;
+  const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int nc = (n - b + G - 1) / G;
+  S* C = reinterpret_cast<S*>(he_smem);
+  S* vs = C + (size_t)((n + G - 1) / G) * n;
+  S* ws = vs + n;
+  if (tid == 0) bad = 0;
+  for (int q = 0; q < nc; ++q)
+    for (int k = tid; k < n; k += kHeT) async_load(C + (size_t)q * n + k, B + (size_t)(b + q * G) * n + k);
+  async_wait();
+  __syncthreads();
+
+  // column j (in slot j / G, its rows from j on) is final: its reflector, then out
+  auto publish = [&](int j, double ssq) {
+    S* x = C + (size_t)(j / G) * n + j;
+    S* g = B + (size_t)j * n + j;
+    if (j == n - 1) {
+      if (tid == 0) {
+        d[j] = O::re(x[0]);
+        g[0] = x[0];
+      }
+      return;
+    }
+    const S t = he_reflector<S>(x + 1, n - 1 - j, ssq, red, bc);
+    for (int k = tid; k < n - j; k += kHeT) g[k] = x[k];
+    if (tid == 0) {
+      d[j] = O::re(x[0]);
+      e[j] = O::re(x[1]);
+      tau[j] = t;
+    }
+    if (G > 1) {
+      __syncthreads();
+      if (tid == 0) {
+        __threadfence();
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&ctl->ready), "r"(j + 1) : "memory");
+      }
+    }
+  };
+  if (b == 0) {
+    double ssq = 0.0;
+    for (int k = 2 + tid; k < n; k += kHeT) ssq = he_acc2(C[k], ssq);
+    publish(0, ssq);
+  }
+
+  for (int i = 0; i <= n - 2; ++i) {
+    const int m = n - 1 - i;
+    S* Wi = W + (size_t)(i & 1) * n;
+    if (G > 1 && tid == 0 && !he_wait(&ctl->ready, i + 1, &ctl->err)) bad = 1;
+    __syncthreads();
+    if (bad) break;
+    const S* vg = B + (size_t)i * n + (i + 1);
+    const S t = __ldcg(tau + i);
+    for (int k = tid; k < m; k += kHeT) vs[k] = k == 0 ? O::one() : __ldcg(vg + k);
+    __syncthreads();
+    const int q0 = b > i ? 0 : (i + 1 - b + G - 1) / G;  // first slot with a column > i
+    for (int q = q0 + wid; q < nc; q += kHeT / 32) {
+      const S* col = C + (size_t)q * n + (i + 1);
+      S s = O::zero();
+#pragma unroll 4
+      for (int k = lane; k < m; k += 32) s = O::fmac(col[k], vs[k], s);
+      s = warp_sum(s);
+      if (lane == 0) Wi[b + q * G - (i + 1)] = O::mul(t, s);
+    }
+    __syncthreads();
+    if (G > 1) {
+      if (tid == 0) {
+        __threadfence();
+        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&ctl->arrive), "r"(1u) : "memory");
+        if (!he_wait(&ctl->arrive, (unsigned)G * (i + 1), &ctl->err)) bad = 1;
+      }
+      __syncthreads();
+      if (bad) break;
+    }
+    S dw = O::zero();
+    for (int k = tid; k < m; k += kHeT) {
+      const S w = __ldcg(Wi + k);
+      ws[k] = w;
+      dw = O::fmac(w, vs[k], dw);
+    }
+    dw = he_cta_sum(dw, reds, [](S v, int o) { return O::add(v, O::shfl(v, o)); });
+    const S alpha = O::mul(O::scal(t, -0.5), dw);
+    for (int k = tid; k < m; k += kHeT) ws[k] = O::fma(alpha, vs[k], ws[k]);
+    __syncthreads();
+    // a - (v_k conj(w'_j) + w'_k conj(v_j)), one rounding of a
+    auto upd = [&](S a, S cw, S cv, int k) {
+      return O::sub(a, O::fma(ws[k], cv, O::mul(vs[k], cw)));
+    };
+    if (b == (i + 1) % G) {
+      S* col = C + (size_t)((i + 1) / G) * n + (i + 1);
+      const S cw = O::conj(ws[0]), cv = O::conj(vs[0]);
+      double ssq = 0.0;
+      for (int k = tid; k < m; k += kHeT) {
+        S a = upd(col[k], cw, cv, k);
+        if (k == 0) a = O::from(O::re(a));
+        if (k >= 2) ssq = he_acc2(a, ssq);
+        col[k] = a;
+      }
+      __syncthreads();
+      publish(i + 1, ssq);
+    }
+    const int q1 = b > i + 1 ? 0 : (i + 2 - b + G - 1) / G;  // first slot with a column > i + 1
+    for (int q = q1 + wid; q < nc; q += kHeT / 32) {
+      const int jj = b + q * G - (i + 1);
+      S* col = C + (size_t)q * n + (i + 1);
+      const S cw = O::conj(ws[jj]), cv = O::conj(vs[jj]);
+#pragma unroll 4
+      for (int k = lane; k < m; k += 32) {
+        S a = upd(col[k], cw, cv, k);
+        if (k == jj) a = O::from(O::re(a));
+        col[k] = a;
+      }
+    }
+  }
+  if (bad && b == 0)
+    for (int k = tid; k < n; k += kHeT) {
+      d[k] = 0.0;
+      if (k < n - 1) e[k] = 0.0;
+    }
+}
+
+// Q = H_1 ... H_{n-1}, column by column: column j of Q is e_j under the reflectors
+// j-1, ..., 0, which no other column takes part in.  A warp per column, the column in
+// shared memory, all reflectors in one launch; columns dealt so that each CTA has long
+// and short ones.  Bound by the FP64 pipe (2 fused operations per entry and reflector).
+// Against one launch per reflector, with the matrix read and written each time: n = 1000
+// real 5.8 ms, now 3.3.
+template <class S>
+__global__ void __launch_bounds__(kHeT) k_he_formq_cols(const S* __restrict__ B, int n, const S* __restrict__ tau, S* Q) {
+  using O = Hs<S>;
+  extern __shared__ __align__(16) unsigned char he_smem[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  S* x = reinterpret_cast<S*>(he_smem) + (size_t)wid * n;
+  for (int j = blockIdx.x + gridDim.x * wid; j < n; j += gridDim.x * (blockDim.x >> 5)) {
+    for (int k = lane; k < n; k += 32) x[k] = k == j ? O::one() : O::zero();
+    __syncwarp();
+    for (int i = j - 1; i >= 0; --i) {
+      const S t = tau[i];
+      if (O::is0(t)) continue;
+      const int m = n - 1 - i;
+      const S* u = B + (size_t)i * n + (i + 1);
+      S* q = x + (i + 1);
+      S s = O::zero();
+#pragma unroll 8
+      for (int k = lane; k < m; k += 32) s = O::fmac(k == 0 ? O::one() : u[k], q[k], s);
+      s = warp_sum(s);
+      const S ts = O::mul(t, s);
+#pragma unroll 8
+      for (int k = lane; k < m; k += 32) q[k] = O::sub(q[k], O::mul(ts, k == 0 ? O::one() : u[k]));
+      __syncwarp();
+    }
+    for (int k = lane; k < n; k += 32) Q[(size_t)j * n + k] = x[k];
+    __syncwarp();
   }
 }
 
@@ -737,6 +998,15 @@ cudaError_t launch_he_tridiag(const S* A, long long lda, int n, int upper, S* B,
   k_he_prep<S><<<grid_of((size_t)n * n), 256, 0, s>>>(A, lda, n, upper, B);
   cudaError_t err = cudaMemsetAsync(ctl, 0, sizeof(HeCtl<S>), s);
   if (err != cudaSuccess) return err;
+  // one kernel where the matrix fits in the chip's shared memory
+  const int G = n <= kHeOneCta ? 1 : std::min(num_sms, (n + kHeCols - 1) / kHeCols);
+  const size_t smem = ((size_t)((n + G - 1) / G) + 2) * n * sizeof(S);
+  if (smem <= kMaxDynSmem) {
+    err = cudaFuncSetAttribute(k_he_tridiag<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
+    if (err != cudaSuccess) return err;
+    void* args[] = {&B, &n, &W, &ctl, &tau, &d, &e};
+    return cudaLaunchCooperativeKernel((const void*)k_he_tridiag<S>, dim3(G), dim3(kHeT), args, smem, s);
+  }
   k_he_first<S><<<1, kHeT, 0, s>>>(B, n, ctl, tau, d, e);
   for (int i = 0; i <= n - 2; ++i) {
     const int m = n - 1 - i;
@@ -750,6 +1020,15 @@ cudaError_t launch_he_tridiag(const S* A, long long lda, int n, int upper, S* B,
 
 template <class S>
 cudaError_t launch_he_formq(const S* B, int n, const S* tau, S* Q, int num_sms, cudaStream_t s) {
+  // warps whose columns fit in a CTA's shared memory; with fewer than four the launches per reflector
+  const int nw = (int)std::min<size_t>(kHeT / 32, kMaxDynSmem / ((size_t)n * sizeof(S)));
+  if (nw >= 4) {
+    const size_t smem = (size_t)nw * n * sizeof(S);
+    cudaError_t err = cudaFuncSetAttribute(k_he_formq_cols<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
+    if (err != cudaSuccess) return err;
+    k_he_formq_cols<S><<<std::min(n, num_sms), 32 * nw, smem, s>>>(B, n, tau, Q);
+    return cudaGetLastError();
+  }
   k_he_identity<S><<<grid_of((size_t)n * n), 256, 0, s>>>(Q, n);
   for (int i = n - 2; i >= 0; --i) {
     const int m = n - 1 - i;
