@@ -103,77 +103,180 @@ __global__ void __launch_bounds__(256) k_sylv_rhs(int n, int nT, int D, const do
   for (int k = 0; k < 4; ++k) out[(cb + 8 * k) * kSt + r] = acc[k];
 }
 
-// Level D, step 2: one CTA per tile pair sums its partials (fixed order) and -L_PQ,
-// then solves the block pairs inside the tile pair by local anti-diagonal waves, warp
-// per block pair (the in-tile sums over the lanes, lane 0 solves the <= 4x4 Kronecker
-// system (I (x) T_pp - T_qq^T (x) I) vec(W_pq) = rhs).
-__global__ void __launch_bounds__(256) k_sylv_solve(int n, int nT, int D, const double* __restrict__ At,
-                                                    double* __restrict__ W, const int* __restrict__ bs,
-                                                    const int* __restrict__ bz, const int* __restrict__ blk,
-                                                    const int* __restrict__ ts, const int* __restrict__ tbk,
-                                                    const double* __restrict__ part, int nchunk, double floor) {
+// The solution of T_pp W - W T_qq = R at one entry of its block, as four weights of the
+// block's R: W[a][b] = sum_{a'b'} k[a' + 2 b'] R[a'][b'].  With c the mean of T_qq's
+// diagonal, A = T_pp - c I and B = T_qq - c I, a 2x2 B has B^2 = -det(B) I, so
+// (A^2 + det(B) I) W = A R + R B; a 1x1 B is 0 and A W = R.  False when the weights could
+// lose more than about eight digits (nearly equal eigenvalues): Newton's step would still
+// converge with those, but such a tile is left to the pivoted elimination.
+__device__ __forceinline__ bool block_weights(const double (*Ta)[kSt + 1], const double (*Tb)[kSt + 1], int sp, int zp,
+                                              int sq, int zq, int a, int b, double floor, double k[4]) {
+  k[0] = k[1] = k[2] = k[3] = 0.0;
+  if (zp == 1 && zq == 1) {
+    double m = Ta[sp][sp] - Tb[sq][sq];
+    if (fabs(m) < floor) m = (m < 0.0) ? -floor : floor;
+    k[0] = 1.0 / m;
+    return true;
+  }
+  double c = Tb[sq][sq], b00 = 0.0, b01 = 0.0, b10 = 0.0, det = 0.0;
+  if (zq == 2) {
+    c = 0.5 * (Tb[sq][sq] + Tb[sq + 1][sq + 1]);
+    b00 = 0.5 * (Tb[sq][sq] - Tb[sq + 1][sq + 1]);
+    b01 = Tb[sq][sq + 1];
+    b10 = Tb[sq + 1][sq];
+    det = -fma(b00, b00, b01 * b10);
+  }
+  const double a00 = Ta[sp][sp] - c;
+  if (zp == 1) {  // zq == 2: (a^2 + det) W = R (a I + B)
+    const double q = fma(a00, a00, det);
+    const double r = 1.0 / q;
+    k[0] = (b == 0 ? a00 + b00 : b01) * r;  // R[0][0]
+    k[2] = (b == 0 ? b10 : a00 - b00) * r;  // R[0][1]
+    return fma(a00, a00, fabs(det)) <= 1e8 * fabs(q);
+  }
+  const double a01 = Ta[sp][sp + 1], a10 = Ta[sp + 1][sp], a11 = Ta[sp + 1][sp + 1] - c;
+  double q00 = a00, q01 = a01, q10 = a10, q11 = a11;
+  double big = fmax(fmax(fabs(a00), fabs(a11)), fmax(fabs(a01), fabs(a10)));
+  if (zq == 2) {
+    const double tr = a00 + a11, x = a01 * a10;
+    q00 = fma(a00, a00, x + det);
+    q11 = fma(a11, a11, x + det);
+    q01 = a01 * tr;
+    q10 = a10 * tr;
+    big = fma(big, big, fabs(det));
+  }
+  const double dq = fma(q00, q11, -q01 * q10);
+  const double r = 1.0 / dq;
+  // row a of the inverse
+  const double i0 = (a == 0 ? q11 : -q10) * r, i1 = (a == 0 ? -q01 : q00) * r;
+  if (zq == 2) {
+    const double m0 = fma(i0, a00, i1 * a10), m1 = fma(i0, a01, i1 * a11);  // row a of (A^2 + det I)^-1 A
+    const double c0 = b == 0 ? b00 : b01, c1 = b == 0 ? b10 : -b00;         // column b of B
+    k[0] = fma(i0, c0, b == 0 ? m0 : 0.0);
+    k[1] = fma(i1, c0, b == 0 ? m1 : 0.0);
+    k[2] = fma(i0, c1, b == 1 ? m0 : 0.0);
+    k[3] = fma(i1, c1, b == 1 ? m1 : 0.0);
+  } else {
+    k[0] = i0;
+    k[1] = i1;
+  }
+  const double qm = fmax(fmax(fabs(q00), fabs(q11)), fmax(fabs(q01), fabs(q10)));
+  return qm * big <= 1e8 * fabs(dq);
+}
+
+// Level D, step 2: one CTA per tile pair sums its partials (fixed order) and -L_PQ, then
+// solves the block pairs inside the tile pair by local anti-diagonal waves.  A thread
+// holds one entry's right-hand side in a register and the weights of its block's solution
+// (block_weights: they depend on T alone, so all are made before the first wave).  A wave
+// is: its blocks' right-hand sides to shared memory, four products each, then every later
+// entry subtracts the new blocks of its column and row.  Bound by the two barriers and the
+// FP64 latency of 31 (2x2 blocks) to 63 waves.  A warp per block pair with shuffled sums
+// and a pivoted 4x4 elimination by one lane took 600 us a launch at n = 2048 (78 ms of
+// a 511 ms call); this takes 66 us (8.6 ms of 467).  The elimination stays for tiles that block_weights
+// refuses.
+constexpr int kSolveT = kSt * kSt;
+__global__ void __launch_bounds__(kSolveT) k_sylv_solve(int n, int nT, int D, const double* __restrict__ At,
+                                                        double* __restrict__ W, const int* __restrict__ bs,
+                                                        const int* __restrict__ bz, const int* __restrict__ blk,
+                                                        const int* __restrict__ ts, const int* __restrict__ tbk,
+                                                        const double* __restrict__ part, int nchunk, double floor) {
   __shared__ double Ta[kSt][kSt + 1];
   __shared__ double Tb[kSt][kSt + 1];
   __shared__ double Wl[kSt][kSt + 1];
+  __shared__ double Rl[kSt][kSt + 1];
+  __shared__ int ps[kSt], qs[kSt];  // first local row of the tile's blocks, + 64 for a 2x2 block
   const int Q = blockIdx.x, P = Q + D;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int p0 = ts[P], pw = ts[P + 1] - p0, q0 = ts[Q], qw = ts[Q + 1] - q0;
   const int nused = (nT - 1 - D + kSplit - 1) / kSplit;
-  for (int idx = tid; idx < kSt * kSt; idx += 256) {
-    const int x = idx % kSt, y = idx / kSt;
-    double v = (x < pw && y < qw) ? -At[(size_t)(q0 + y) * n + p0 + x] : 0.0;
-    for (int c = 0; c < nused; ++c) v += part[((size_t)Q * nchunk + c) * (kSt * kSt) + y * kSt + x];
-    Wl[x][y] = v;
-    Ta[x][y] = (x < pw && y < pw) ? At[(size_t)(p0 + y) * n + p0 + x] : 0.0;  // T_PP
-    Tb[x][y] = (x < qw && y < qw) ? At[(size_t)(q0 + y) * n + q0 + x] : 0.0;  // T_QQ
-  }
-  __syncthreads();
+  const int x = lane, y = warp;  // this thread's entry of the tile
+  const bool in = x < pw && y < qw;
+  double v = in ? -At[(size_t)(q0 + y) * n + p0 + x] : 0.0;
+  for (int c = 0; c < nused; ++c) v += part[((size_t)Q * nchunk + c) * (kSt * kSt) + y * kSt + x];
+  Wl[x][y] = v;
+  Ta[x][y] = (x < pw && y < pw) ? At[(size_t)(p0 + y) * n + p0 + x] : 0.0;  // T_PP
+  Tb[x][y] = (x < qw && y < qw) ? At[(size_t)(q0 + y) * n + q0 + x] : 0.0;  // T_QQ
   const int pb0 = tbk[P], pb1 = tbk[P + 1], qb0 = tbk[Q], qb1 = tbk[Q + 1];
   const int np = pb1 - pb0, nq = qb1 - qb0;
-  for (int d = 0; d < np + nq - 1; ++d) {
-    for (int i = warp; i < np; i += 8) {
-      const int j = d - i;
-      if (j < 0 || j >= nq) continue;
-      const int p = pb1 - 1 - i, q = qb0 + j;
-      if (P == Q && p <= q) continue;
-      const int sp = bs[p] - p0, zp = bz[p], sq = bs[q] - q0, zq = bz[q];
-      double s2[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-      for (int k = sp + zp + lane; k < pw; k += 32)
-        for (int a = 0; a < zp; ++a)
-          for (int b = 0; b < zq; ++b) s2[a][b] -= Ta[sp + a][k] * Wl[k][sq + b];
-      for (int k = lane; k < sq; k += 32)
-        for (int a = 0; a < zp; ++a)
-          for (int b = 0; b < zq; ++b) s2[a][b] += Wl[sp + a][k] * Tb[k][sq + b];
-      for (int a = 0; a < 2; ++a)
-        for (int b = 0; b < 2; ++b)
-          for (int o = 16; o > 0; o >>= 1) s2[a][b] += __shfl_xor_sync(0xffffffffu, s2[a][b], o);
-      if (lane == 0) {
-        const int m = zp * zq;
-        double M[4][4] = {{0}}, rr[4];
-        for (int b = 0; b < zq; ++b)
-          for (int a = 0; a < zp; ++a) rr[a + b * zp] = Wl[sp + a][sq + b] + s2[a][b];
-        for (int b = 0; b < zq; ++b)
-          for (int a = 0; a < zp; ++a) {
-            const int row = a + b * zp;
-            for (int a2 = 0; a2 < zp; ++a2) M[row][a2 + b * zp] += Ta[sp + a][sp + a2];
-            for (int b2 = 0; b2 < zq; ++b2) M[row][a + b2 * zp] -= Tb[sq + b2][sq + b];
-          }
-        small_solve(m, M, rr, floor);
-        for (int b = 0; b < zq; ++b)
-          for (int a = 0; a < zp; ++a) Wl[sp + a][sq + b] = rr[a + b * zp];
+  const int px = in ? blk[p0 + x] : pb0, qy = in ? blk[q0 + y] : qb0;  // the entry's block pair
+  const bool mine = in && (P != Q || px > qy);
+  const int sp = bs[px] - p0, zp = bz[px], sq = bs[qy] - q0, zq = bz[qy];
+  if (tid < np) ps[tid] = bs[pb0 + tid] - p0 + (bz[pb0 + tid] == 2 ? 64 : 0);
+  if (tid < nq) qs[tid] = bs[qb0 + tid] - q0 + (bz[qb0 + tid] == 2 ? 64 : 0);
+  __syncthreads();
+  double k[4] = {0.0, 0.0, 0.0, 0.0};
+  const bool fine = !mine || block_weights(Ta, Tb, sp, zp, sq, zq, x - sp, y - sq, floor, k);
+  if (__syncthreads_and(fine)) {
+    const int wave = (pb1 - 1 - px) + (qy - qb0);
+    for (int d = 0; d < np + nq - 1; ++d) {
+      const bool now = mine && wave == d;
+      if (now) Rl[x][y] = v;
+      __syncthreads();
+      if (now) {
+        double w = k[0] * Rl[sp][sq];
+        if (zp == 2) w = fma(k[1], Rl[sp + 1][sq], w);
+        if (zq == 2) {
+          w = fma(k[2], Rl[sp][sq + 1], w);
+          if (zp == 2) w = fma(k[3], Rl[sp + 1][sq + 1], w);
+        }
+        Wl[x][y] = w;
       }
-      __syncwarp();
+      __syncthreads();
+      if (mine && wave > d) {
+        // the wave's block in this block column, and the one in this block row
+        const int p = pb1 - 1 - (d - (qy - qb0)), q = qb0 + d - (pb1 - 1 - px);
+        if (p > px && p < pb1 && (P != Q || p > qy)) {
+          const int t = ps[p - pb0], s = t & 63;
+          v = fma(-Ta[x][s], Wl[s][y], v);
+          if (t >= 64) v = fma(-Ta[x][s + 1], Wl[s + 1][y], v);
+        }
+        if (q < qy && q >= qb0 && (P != Q || px > q)) {
+          const int t = qs[q - qb0], s = t & 63;
+          v = fma(Wl[x][s], Tb[s][y], v);
+          if (t >= 64) v = fma(Wl[x][s + 1], Tb[s + 1][y], v);
+        }
+      }
     }
-    __syncthreads();
+  } else {
+    for (int d = 0; d < np + nq - 1; ++d) {
+      for (int i = warp; i < np; i += kSolveT / 32) {
+        const int j = d - i;
+        if (j < 0 || j >= nq) continue;
+        const int p = pb1 - 1 - i, q = qb0 + j;
+        if (P == Q && p <= q) continue;
+        const int sp = bs[p] - p0, zp = bz[p], sq = bs[q] - q0, zq = bz[q];
+        double s2[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        for (int k = sp + zp + lane; k < pw; k += 32)
+          for (int a = 0; a < zp; ++a)
+            for (int b = 0; b < zq; ++b) s2[a][b] -= Ta[sp + a][k] * Wl[k][sq + b];
+        for (int k = lane; k < sq; k += 32)
+          for (int a = 0; a < zp; ++a)
+            for (int b = 0; b < zq; ++b) s2[a][b] += Wl[sp + a][k] * Tb[k][sq + b];
+        for (int a = 0; a < 2; ++a)
+          for (int b = 0; b < 2; ++b)
+            for (int o = 16; o > 0; o >>= 1) s2[a][b] += __shfl_xor_sync(0xffffffffu, s2[a][b], o);
+        if (lane == 0) {
+          const int m = zp * zq;
+          double M[4][4] = {{0}}, rr[4];
+          for (int b = 0; b < zq; ++b)
+            for (int a = 0; a < zp; ++a) rr[a + b * zp] = Wl[sp + a][sq + b] + s2[a][b];
+          for (int b = 0; b < zq; ++b)
+            for (int a = 0; a < zp; ++a) {
+              const int row = a + b * zp;
+              for (int a2 = 0; a2 < zp; ++a2) M[row][a2 + b * zp] += Ta[sp + a][sp + a2];
+              for (int b2 = 0; b2 < zq; ++b2) M[row][a + b2 * zp] -= Tb[sq + b2][sq + b];
+            }
+          small_solve(m, M, rr, floor);
+          for (int b = 0; b < zq; ++b)
+            for (int a = 0; a < zp; ++a) Wl[sp + a][sq + b] = rr[a + b * zp];
+        }
+        __syncwarp();
+      }
+      __syncthreads();
+    }
   }
   // write the tile back: block-lower entries only (the diagonal tile keeps zeros elsewhere)
-  for (int idx = tid; idx < kSt * kSt; idx += 256) {
-    const int x = idx % kSt, y = idx / kSt;
-    if (x < pw && y < qw) {
-      const bool lower = blk[p0 + x] > blk[q0 + y];
-      W[(size_t)(q0 + y) * n + p0 + x] = lower ? Wl[x][y] : 0.0;
-    }
-  }
+  if (in) W[(size_t)(q0 + y) * n + p0 + x] = px > qy ? Wl[x][y] : 0.0;
 }
 
 // S = W - W^T (+ I when add_identity), and block-lower norm accumulation helpers.
@@ -331,7 +434,7 @@ cudaError_t launch_sylv_tiled(int n, int nT, const double* At, double* W, const 
       dim3 g(nT - D, (nprod + kSplit - 1) / kSplit);
       k_sylv_rhs<<<g, 256, 0, s>>>(n, nT, D, At, W, ts, part, nchunk);
     }
-    k_sylv_solve<<<nT - D, 256, 0, s>>>(n, nT, D, At, W, bs, bz, blk, ts, tbk, part, nchunk, floor);
+    k_sylv_solve<<<nT - D, kSolveT, 0, s>>>(n, nT, D, At, W, bs, bz, blk, ts, tbk, part, nchunk, floor);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
