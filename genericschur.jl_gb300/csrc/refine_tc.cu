@@ -24,12 +24,16 @@
 // Kernel k_refine_tc: persistent CTAs of 512 threads (one per SM: the eight level
 // accumulators fill the SM's 512 TMEM columns), each taking the matrices still being
 // refined from a ticket counter, largest first.  Per product, per 64-column panel of Y:
-// chunks of 32 contraction indices are split by all threads straight into shared memory
+// chunks of 32 contraction indices are split straight into shared memory
 // in the tensor core's canonical K-major layout (no swizzle; 8 x 8 core matrices of 128
 // contiguous bytes, K-adjacent core matrices 128 B apart, 8-row groups 512 B apart),
-// double-buffered so that one chunk is split while the MMAs of the previous one run;
-// thread 0 issues the 36 slice products per 16-wide K step (tcgen05.mma, M = 128,
-// N = 64, K = 16) into the accumulator of their level; after the panel's last chunk the
+// double-buffered so that one chunk is split while the MMAs of the previous one run: a
+// thread of warp 0 issues the 36 slice products per 16-wide K step (tcgen05.mma, M = 128,
+// N = 64, K = 16) into the accumulator of their level, and the other fifteen warps split
+// (with thread 0 also splitting and a CTA barrier per chunk, the issue of 72 MMAs, which
+// read 6 KiB of shared memory each, came on top of the split: the products of 20000
+// matrices of orders 8 to 128 36.2 -> 31.6 ms);
+// after the panel's last chunk the
 // sixteen warps (four per TMEM lane quarter, 16 columns each) drain the levels with
 // tcgen05.ld.  Every wait is bounded: a timeout hands the matrix to the FP64 kernel
 // (status kStFallback), records the error, waits for the CTA's MMAs, frees TMEM and ends
@@ -54,6 +58,7 @@ constexpr int kQThreads = 512;
 constexpr int kQXSlice = kQM * kQK * 2;            // bytes of one X slice of a chunk (8 KiB)
 constexpr int kQYSlice = kQN * kQK * 2;            // bytes of one Y slice of a chunk (4 KiB)
 constexpr int kQStage = kQSlices * (kQXSlice + kQYSlice);  // 96 KiB
+constexpr int kQD = 8;                             // columns that a warp drains at once (16 spill)
 constexpr int kQSbo = (kQK / 8) * 128;             // bytes between 8-row groups
 constexpr uint32_t kQIdesc = idesc_bf16(kQM, kQN);
 constexpr int kQExpZero = kExpZeroRow;             // row / column of zeros
@@ -86,20 +91,12 @@ __device__ __forceinline__ unsigned long long fixed56(double x, int e) {
   return sh <= -64 ? 0ull : (m >> (-sh));
 }
 
-// The integer value of an FP32 word holding an integer of magnitude below 2^24 (a level
-// sum), by integer operations: the significand shifted by the exponent, with the sign.
-__device__ __forceinline__ long long level_int(uint32_t u) {
-  const int e = (int)((u >> 23) & 255u);
-  const uint32_t m = (u & 0x7fffffu) | 0x800000u;
-  const int mag = e >= 127 ? (int)(m >> (150 - e)) : 0;
-  return (long long)((int)u < 0 ? -mag : mag);
-}
-
 // (hs 2^28 + ls) 2^e rounded to nearest even, |hs|, |ls| < 2^47: what
 // ldexp(fma((double)hs, 2^28, (double)ls), e) gives, by integer operations.  The drain is
 // every element of every product, and the FP64 pipe takes 19 cycles a warp for each of its
 // conversions and operations: with those the products of 20000 matrices of orders 8 to 128
-// took 50 ms, with integers 40.6.
+// took 50 ms, with integers 40.6 (and 36.2 with the levels read by float-to-int conversions
+// and only the rows split that reach an output).
 __device__ __forceinline__ double level_sum(long long hs, long long ls, int e) {
   long long t = hs + (ls >> 28);
   unsigned l = (unsigned)ls & 0xfffffffu;
@@ -184,6 +181,15 @@ __device__ __forceinline__ void zero8(unsigned char* dst, int slice_bytes) {
   for (int s = 0; s < kQSlices; ++s) *reinterpret_cast<uint4*>(dst + s * slice_bytes) = make_uint4(0u, 0u, 0u, 0u);
 }
 
+// A stage is full: the splitting warps arrive, the issuing warp waits.  (A stage's second
+// arrival follows a wait for the MMAs that its first one released, so arrivals never mix.)
+__device__ __forceinline__ void named_sync(int id, int count) {
+  asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int count) {
+  asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
 // One product C = op(X) Y of n x n column-major FP64 matrices with the exponents of the
 // rows of op(X) in ex and of the columns of Y in fy.  XT = 0: op(X) = X, XT = 1:
 // op(X) = X^T.  KIND 0: P = C 2^extra; KIND 1: Q = C, F = fp32(C); KIND 2:
@@ -195,98 +201,95 @@ __device__ bool tc_product(int n, const double* X, const double* Y, const int* e
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nchunks = (n + kQK - 1) / kQK;
   const uint32_t s0 = smem_u32(smem);
+  const auto vfail = [&]() { return *(volatile int*)&ctl.fail != 0; };
+  // one thread: the MMAs of chunk c, in stage st, of the panel at column j0
+  const auto issue = [&](int c, int st, int j0) {
+    tc_fence_after();
+    const uint32_t xa = s0 + st * kQStage;
+    const uint32_t ya = KIND == 2 ? xa + (j0 >> 3) * kQSbo : xa + kQSlices * kQXSlice;
+    constexpr int kBSlice = KIND == 2 ? kQXSlice : kQYSlice;
+    const uint64_t adesc = smem_desc(xa, 128, kQSbo), bdesc = smem_desc(ya, 128, kQSbo);
+    // the 36 slice pairs (s, t), s + t = L <= 7, into the accumulator of level L; the
+    // level's first pair at the panel's first K step overwrites it (descriptor start
+    // addresses are in units of 16 bytes)
+#pragma unroll
+    for (int L = 0; L < kQLevels; ++L) {
+#pragma unroll
+      for (int s = 0; s <= L; ++s) {
+#pragma unroll
+        for (int kk = 0; kk < kQK / 16; ++kk) {
+          const uint32_t acc = (c > 0 || kk > 0 || s > 0) ? 1u : 0u;
+          tc_mma(tmem + (uint32_t)(L * kQN), adesc + (uint64_t)((s * kQXSlice + kk * 256) >> 4),
+                 bdesc + (uint64_t)(((L - s) * kBSlice + kk * 256) >> 4), kQIdesc, acc);
+        }
+      }
+    }
+    tc_commit(&ctl.bar[st]);
+  };
   for (int j0 = 0; j0 < n; j0 += kQN) {
     for (int c = 0; c < nchunks; ++c, ++gchunk) {
       const int st = gchunk & 1;
-      // the MMAs that last read this stage must be complete before it is overwritten
-      if (tid == 0) {
-        ctl.fail = 0;
-        if (gchunk >= 2 && !mbar_wait(&ctl.bar[st], ((gchunk >> 1) - 1) & 1u, kQTimeout)) ctl.fail = 1;
+      if (warp == 0) {
+        // the issuing warp: every splitting warp has filled the stage
+        named_sync(1 + st, kQThreads);
+        if (lane == 0 && !vfail()) issue(c, st, j0);
+        __syncwarp();
+        continue;
       }
-      __syncthreads();
-      if (ctl.fail) return false;
+      // the MMAs that last read this stage must be complete before it is overwritten
+      if (lane == 0 && gchunk >= 2 && !vfail() && !mbar_wait(&ctl.bar[st], ((gchunk >> 1) - 1) & 1u, kQTimeout))
+        *(volatile int*)&ctl.fail = 1;
+      __syncwarp();
       unsigned char* xs = smem + st * kQStage;
-      unsigned char* ys = xs + kQSlices * kQXSlice;
       const int k0 = c * kQK;
-      // items: op(X) rows (128 rows x 4 groups of 8 k), then the panel's Y columns (64 x 4);
-      // rows of op(X) and columns of Y beyond n only reach outputs that are not stored, so
-      // they are skipped; contraction indices beyond n are zero in both operands
-      constexpr int kXItems = kQM * (kQK / 8), kItems = kXItems + kQN * (kQK / 8);
-      constexpr int kPer = (kItems + kQThreads - 1) / kQThreads;  // 2
+      // items: (row of op(X) or column of Y) x 4 groups of 8 k, only those that reach a stored
+      // output, dealt to all threads (by fixed rows, an order of 72 left every fourth warp,
+      // and with it a scheduler, without work); contraction indices beyond n are zero in
+      // both operands.  In Z^T Z the columns of Y are rows of op(X): split once.
+      const int x0 = KIND == 2 ? j0 : 0, nx = n - x0;
+      const int nrow = nx + (KIND == 2 ? 0 : min(kQN, n - j0));
+      constexpr int kPer = ((kQM + (KIND == 2 ? 0 : kQN)) * (kQK / 8) + kQThreads - 33) / (kQThreads - 32);
       double v[kPer][8];
-      int eit[kPer];
-      unsigned char* dst[kPer];
-      bool live[kPer];
+      int eit[kPer], sb[kPer];
+      int dst[kPer];  // byte offset in the stage
 #pragma unroll
       for (int u = 0; u < kPer; ++u) {
-        const int it = tid + u * kQThreads;
-        int row = 0, kg = 0, e = kQExpZero;
-        if (it >= kItems) {
-          live[u] = false;
-          dst[u] = xs;
-        } else if (it < kXItems) {
-          row = it & (kQM - 1); kg = it >> 7;
-          live[u] = row < n;
-          dst[u] = xs + (((row >> 3) * (kQK / 8) + kg) * 64 + (row & 7) * 8) * 2;
-          if (live[u]) e = ex[row];
-        } else {
-          const int jt = it - kXItems;
-          const int jl = jt & (kQN - 1);
-          kg = jt >> 6;
-          row = j0 + jl;
-          live[u] = row < n;
-          dst[u] = ys + (((jl >> 3) * (kQK / 8) + kg) * 64 + (jl & 7) * 8) * 2;
-          if (live[u]) e = fy[row];
-        }
-        eit[u] = e;
+        const int it = tid - 32 + u * (kQThreads - 32);
+        const int kg = it / nrow, r = it - kg * nrow;
+        sb[u] = 0;
+        if (kg >= kQK / 8) continue;
+        const bool isx = r < nx;
+        const int slot = isx ? x0 + r : r - nx;  // row of the stage's X or Y part
+        const int row = isx ? slot : j0 + slot;  // row of op(X) or column of Y
+        sb[u] = isx ? kQXSlice : kQYSlice;
+        dst[u] = (isx ? 0 : kQSlices * kQXSlice) + (((slot >> 3) * (kQK / 8) + kg) * 64 + (slot & 7) * 8) * 2;
         const int kb = k0 + kg * 8;
+        eit[u] = kb < n ? (isx ? ex[row] : fy[row]) : kQExpZero;
 #pragma unroll
         for (int x = 0; x < 8; ++x) {
           const int k = kb + x;
           double val = 0.0;
-          if (live[u] && k < n) {
-            if (it < kXItems) val = XT ? X[(size_t)row * n + k] : X[(size_t)k * n + row];
+          if (k < n) {
+            if (isx) val = XT ? X[(size_t)row * n + k] : X[(size_t)k * n + row];
             else val = Y[(size_t)row * n + k];
           }
           v[u][x] = val;
         }
-        if (kb >= n) eit[u] = kQExpZero;  // live rows whose k-group lies beyond n: zero slices
       }
 #pragma unroll
       for (int u = 0; u < kPer; ++u) {
-        if (!live[u]) continue;
-        const int sb = (tid + u * kQThreads) < kXItems ? kQXSlice : kQYSlice;
-        if (eit[u] == kQExpZero) zero8(dst[u], sb);
-        else split8(v[u], eit[u], dst[u], sb);
+        if (sb[u] == 0) continue;
+        if (eit[u] == kQExpZero) zero8(xs + dst[u], sb[u]);
+        else split8(v[u], eit[u], xs + dst[u], sb[u]);
       }
       fence_proxy_async_smem();
-      __syncthreads();
-      if (tid == 0) {
-        tc_fence_after();
-        const uint32_t xa = s0 + st * kQStage, ya = xa + kQSlices * kQXSlice;
-        const uint64_t adesc = smem_desc(xa, 128, kQSbo), bdesc = smem_desc(ya, 128, kQSbo);
-        // the 36 slice pairs (s, t), s + t = L <= 7, into the accumulator of level L; the
-        // level's first pair at the panel's first K step overwrites it (descriptor start
-        // addresses are in units of 16 bytes)
-#pragma unroll
-        for (int L = 0; L < kQLevels; ++L) {
-#pragma unroll
-          for (int s = 0; s <= L; ++s) {
-#pragma unroll
-            for (int kk = 0; kk < kQK / 16; ++kk) {
-              const uint32_t acc = (c > 0 || kk > 0 || s > 0) ? 1u : 0u;
-              tc_mma(tmem + (uint32_t)(L * kQN), adesc + (uint64_t)((s * kQXSlice + kk * 256) >> 4),
-                     bdesc + (uint64_t)(((L - s) * kQYSlice + kk * 256) >> 4), kQIdesc, acc);
-            }
-          }
-        }
-        tc_commit(&ctl.bar[st]);
-      }
+      __syncwarp();
+      named_arrive(1 + st, kQThreads);
     }
     // drain the panel: the last chunk's commit covers every MMA before it
-    if (tid == 0) {
+    if (tid == 0 && !vfail()) {
       const unsigned last = gchunk - 1;
-      ctl.fail = mbar_wait(&ctl.bar[last & 1], (last >> 1) & 1u, kQTimeout) ? 0 : 1;
+      if (!mbar_wait(&ctl.bar[last & 1], (last >> 1) & 1u, kQTimeout)) *(volatile int*)&ctl.fail = 1;
     }
     __syncthreads();
     if (ctl.fail) return false;
@@ -294,33 +297,36 @@ __device__ bool tc_product(int n, const double* X, const double* Y, const int* e
     {
       const int q = warp & 3, cq = warp >> 2;  // TMEM lane quarter, 16-column quarter of the panel
       const int i = q * 32 + lane;
-      const int jb = j0 + cq * 16;
-      // G = Z^T Z is symmetric: only the lower triangle is formed (and mirrored)
-      const bool need = KIND != 2 || q * 32 + 32 > jb;
-      if (jb < n && q * 32 < n && need) {  // warp-uniform
-        // the eight exact level sums, as integers, combined in two 64-bit Horner sums of
-        // four levels each (below 2^46, so their FP64 conversions are exact)
-        long long hs[16], ls[16];
-#pragma unroll
-        for (int x = 0; x < 16; ++x) { hs[x] = 0; ls[x] = 0; }
-        const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cq * 16);
+      const int ei = i < n ? ex[i] : 0;
 #pragma unroll 1
-        for (int L = 0; L < kQLevels; ++L) {  // most significant level first
-          uint32_t v[16];
-          tc_ld16(tb + L * kQN, v);
-          tc_wait_ld();
-          if (L < 4) {
+      for (int jl = cq * 16; jl < cq * 16 + 16; jl += kQD) {
+        const int jb = j0 + jl;
+        // G = Z^T Z is symmetric: only the lower triangle is formed (and mirrored)
+        if (jb >= n || q * 32 >= n || (KIND == 2 && q * 32 + 32 <= jb)) break;  // warp-uniform
+        // the eight exact level sums as integers: level L is at most (L + 1) 127^2 128, so two
+        // levels make one 32-bit integer (128 v6 + v7 < 2^31) and four a 64-bit one
+        long long hs[kQD], ls[kQD];
+        const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)jl;
 #pragma unroll
-            for (int x = 0; x < 16; ++x) hs[x] = hs[x] * 128 + level_int(v[x]);
-          } else {
+        for (int h = 0; h < 2; ++h) {  // most significant levels first
+          int p[kQD];
 #pragma unroll
-            for (int x = 0; x < 16; ++x) ls[x] = ls[x] * 128 + level_int(v[x]);
+          for (int g = 0; g < 2; ++g) {
+            uint32_t v0[kQD], v1[kQD];
+            tc_ld8(tb + (4 * h + 2 * g) * kQN, v0);
+            tc_ld8(tb + (4 * h + 2 * g + 1) * kQN, v1);
+            tc_wait_ld();
+#pragma unroll
+            for (int x = 0; x < kQD; ++x) {
+              const int w = __float2int_rn(__uint_as_float(v0[x])) * 128 + __float2int_rn(__uint_as_float(v1[x]));
+              if (g == 0) p[x] = w;
+              else (h == 0 ? hs : ls)[x] = (long long)p[x] * 16384 + w;
+            }
           }
         }
         if (i < n) {
-          const int ei = ex[i];
 #pragma unroll
-          for (int x = 0; x < 16; ++x) {
+          for (int x = 0; x < kQD; ++x) {
             const int j = jb + x;
             if (j < n && (KIND != 2 || i >= j)) {
               const int fj = fy[j];
@@ -358,6 +364,7 @@ __global__ void __launch_bounds__(kQThreads, 1) k_refine_tc(RefineArgs a, int st
     mbar_init(&ctl.bar[0], 1);
     mbar_init(&ctl.bar[1], 1);
     mbar_init(&ctl.done, 1);
+    ctl.fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if ((tid >> 5) == 0) {
