@@ -707,12 +707,15 @@ int schur_large_cplx_run(double2* A, double2* Z, double2* w, int n, int scale, l
 
   // Blocks up to nmin go to the batched kernel; a sweep chases at most bmax bulges, chunk
   // steps per window; aedw is the early-deflation window (0: off).  Defaults measured on
-  // GB300 with complex N(0,1/2) matrices: 12 bulges without early deflation are fastest up
-  // to n ~ 700 (n = 256: 0.19 s against 0.28 s for 32 bulges), 24 bulges with a 32-wide
-  // early-deflation window above (n = 1024: 1.74 s against 1.95 s).  GS_CPLX_NMIN,
-  // GS_CPLX_BULGES, GS_CPLX_CHUNK and GS_CPLX_AEDW override them for tuning runs.
+  // GB300 with complex N(0,1/2) matrices.  Up to n ~ 700, 8 bulges (one per warp of the chase
+  // kernel) without early deflation: n = 144 / 256 / 400 / 600 68 / 169 / 337 / 673 ms, with 12
+  // bulges 77 / 186 / 354 / 709, with a 32-wide early-deflation window 1047 at 600; blocks of
+  // order <= 48 to the batched kernel are 1% ahead of 64.  Above, 24 bulges with a 32-wide
+  // early-deflation window (n = 1024: 1.41 s, 16 bulges 1.51, 8 without the window 1.72; at
+  // 760 0.96 against 1.02).  GS_CPLX_NMIN, GS_CPLX_BULGES, GS_CPLX_CHUNK and GS_CPLX_AEDW
+  // override them for tuning runs.
   const bool big = n >= 768;
-  int nmin = 64, bmax = big ? 24 : 12, chunk = kZChunk, aedw = big ? kZAedW : 0;
+  int nmin = big ? 64 : 48, bmax = big ? 24 : 8, chunk = kZChunk, aedw = big ? kZAedW : 0;
   if (const char* ev = std::getenv("GS_CPLX_NMIN")) nmin = std::max(16, std::min(nb, std::atoi(ev)));
   if (const char* ev = std::getenv("GS_CPLX_BULGES")) bmax = std::max(1, std::min(kZMaxB, std::atoi(ev)));
   if (const char* ev = std::getenv("GS_CPLX_CHUNK")) chunk = std::max(1, std::min(kZChunkMax, std::atoi(ev)));
