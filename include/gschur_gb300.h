@@ -76,8 +76,8 @@ GS_API float gs_last_kernel_ms(const gs_context* ctx);
  * batched form).  gs_set_tuning loads a table written by the project's tuner
  * (genericschur.jl_gb300/tune.py) for this context: per size bin of the real FP64, the
  * complex, and the FP32 stage of the mixed real (GS_MIXED) batched Schur kernels, the
- * bin's largest order, threads per CTA, whether the Hessenberg phase runs in shared
- * memory, and a cap on CTAs per SM.  Text lines "kind bin nmax threads hsmem ctas_per_sm"
+ * bin's largest order, threads per CTA, a Hessenberg flag (0 or 1; accepted, selects
+ * nothing), and a cap on CTAs per SM.  Text lines "kind bin nmax threads hsmem ctas_per_sm"
  * (kind real_f64, complex_f64 or mixed_f32; '#' starts a comment; bins not listed keep
  * their defaults; mixed_f32 bins keep the default bounds 32/64/96/128).  path NULL or ""
  * restores the built-in defaults.  GS_BADARG (message in gs_last_error) for an unreadable
