@@ -370,7 +370,7 @@ def run_ours(args):
     peak = fp64_peak_tflops(torch, dev)
     peak32 = fp32_peak_tflops(torch, dev)
     # roofline of the mixed step's dominant kernel: the FP32 batched Schur kernel
-    # (k_schur_real<float>, four size-bin launches running concurrently), timed by the CUDA
+    # (a reduction, a Q and an iteration launch per size bin, running concurrently), timed by the CUDA
     # events the library records at the start of the call's kernels and at the start of the
     # refinement (the conversion k_mixed_prep, ~1% of the stage, is inside that window);
     # bound by the FP32 FMA pipe (25 n^3 FLOP per matrix), which the bulge chase's
@@ -379,7 +379,7 @@ def run_ours(args):
     ach32 = flops / fp32_s / 1e12 if fp32_s else None
     roof = {"bound": "fp32", "achieved": ach32, "peak": peak32, "unit": "TFLOP/s",
             "frac": (ach32 / peak32) if ach32 else None, "traffic": None,
-            "kernel": "k_schur_real<float> (FP32 stage of the mixed step, four size-bin launches)",
+            "kernel": "k_hess_real32, k_formq_real32, k_schur_real<float> (FP32 stage of the mixed step, a launch of each per size bin)",
             "phase_ms": info["fp32_us"] * 1e-3, "step_kernel_ms": kms_mixed,
             "algorithmic": "25 n^3 FP32 FLOP per matrix, summed over the batch (%.4g FLOP per launch)" % flops,
             "peak_source": "measured: cuBLAS SGEMM 4096^3 in this run (FP32 FMA pipe, TF32 off)",
@@ -403,8 +403,8 @@ def run_ours(args):
     per_matrix_bytes = measured_traffic_per_matrix()
     traffic = per_matrix_bytes * count if per_matrix_bytes else None
     roof64 = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-              "traffic": traffic, "kernel": "k_schur_real<double> (four size-bin launches)",
-              "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of the 4 size-bin launches of one "
+              "traffic": traffic, "kernel": "k_hess_real64, k_schur_real<double> (a launch of each per size bin)",
+              "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of the 8 size-bin launches of one "
                                 "step, ncu capture of a 6000-matrix case of the same law scaled by matrices "
                                 "(profiles/k_schur_real_traffic.txt); algorithmic bytes 24 n^2 + 16 n per matrix "
                                 "= %.4g per step" % float(np.sum(24.0 * ns.astype(np.float64) ** 2 + 16.0 * ns)),
@@ -413,7 +413,7 @@ def run_ours(args):
     accuracy = {"mixed": schur_errors_sample(packed, ns, offs, woffs, res_mixed),
                 "fp64": schur_errors_sample(packed, ns, offs, woffs, res_fp64)}
     fp64 = {"value": value64, "unit": UNIT, "ms_per_step": ms_fp64, "unconverged": bad64, "roofline": roof64,
-            "e2e": e2e64, "gpu_launches_per_step": 5}
+            "e2e": e2e64, "gpu_launches_per_step": 9}
     cpu = None if args.no_cpu else cpu_baseline_sample(args.count, SEED)
     per_matrix = measure_per_matrix(ctx, packed, ns, offs)
     secondary = measure_complex_and_adjoint(ctx, torch, dev, stream)
@@ -440,7 +440,7 @@ def run_ours(args):
                    "sample in this run)",
            "config": bench_config(args.count), "graph": not args.no_graph,
            "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "clocks": clk,
-           "gpu_launches": 42 * args.steps, "unconverged": bad, "refinement": refinement,
+           "gpu_launches": 54 * args.steps, "unconverged": bad, "refinement": refinement,
            "fp64": fp64, "mixed_vs_fp64": value / value64,
            "mixed_vs_fp64_e2e": (e2e["value"] / e2e64["value"]) if (e2e and e2e64) else None,
            "accuracy": accuracy, "plain_fp64_per_matrix": per_matrix,
@@ -557,7 +557,7 @@ def measure_c1(ctx, n=256):
 def measure_per_matrix(ctx, packed, ns, offs, sample=200):
     """The plain FP64 path one matrix per call (gs_schur_f64 with device buffers,
     synchronised per call) on the first `sample` matrices of the batch: what a caller
-    without the batched form gets, for comparison with the persistent batched launch."""
+    without the batched form gets, for comparison with the batched launch."""
     import torch
     from genericschur_gb300 import _capi
     dev = torch.device("cuda", torch.cuda.current_device())
