@@ -251,6 +251,9 @@ struct TriBatch {
   int* colmap;             // may be null
 };
 cudaError_t launch_triangularize(const TriBatch& tb, int num_sms, cudaStream_t s);
+// One matrix of any order over the whole GPU (Zr null: identity; Zc, w, colmap may be null).
+cudaError_t launch_triangularize_one(int n, const double* Tr, const double* Zr, double2* Tc, double2* Zc, double2* w,
+                                     int* colmap, cudaStream_t s);
 
 // Eigenvalue adjoint: grad = Y diag(gbar / conj(diag(Y^H X))) X^H per matrix.
 struct AdjBatch {

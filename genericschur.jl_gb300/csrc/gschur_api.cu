@@ -1266,12 +1266,11 @@ static int eigvecs_large_driver(gs_context* ctx, int64_t n, const double* T, con
   Arena ar;
   const size_t o_ws = ar.take<double2>(eigvecs_large_ws_elems((int)n));
   const size_t o_bad = ar.take<int>(4);
-  size_t o_T = 0, o_Z = 0, o_VR = 0, o_VL = 0, o_Tc = 0, o_Zc = 0, o_map = 0, o_meta = 0;
+  size_t o_T = 0, o_Z = 0, o_VR = 0, o_VL = 0, o_Tc = 0, o_Zc = 0, o_map = 0;
   if (real) {
     o_Tc = ar.take<double2>(nn);
     o_Zc = ar.take<double2>(Z ? nn : 1);
     o_map = ar.take<int>(n);
-    o_meta = ar.take<long long>(4);
   }
   if (!dev) {
     o_T = ar.take<char>(es * nn);
@@ -1302,27 +1301,14 @@ static int eigvecs_large_driver(gs_context* ctx, int64_t n, const double* T, con
   const double2* cZ = (const double2*)d_Z;
   const int* cmap = nullptr;
   if (real) {
-    long long meta_h[4] = {0, 0, 0, 0};
-    int n32 = (int)n;
-    long long* meta = (long long*)(base + o_meta);
-    CK(cudaMemcpyAsync(meta, meta_h, sizeof(meta_h), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(meta + 2, &n32, sizeof(int), cudaMemcpyHostToDevice, s));
-    TriBatch tb{};
-    tb.count = 1;
-    tb.ns = (const int*)(meta + 2);
-    tb.offs = meta;
-    tb.woffs = meta + 1;
-    tb.Tr = (const double*)d_T;
-    tb.Zr = (const double*)d_Z;
-    tb.Tc = (double2*)(base + o_Tc);
-    tb.Zc = d_Z ? (double2*)(base + o_Zc) : nullptr;
-    tb.w = nullptr;
-    tb.colmap = (int*)(base + o_map);
-    cudaError_t e = launch_triangularize(tb, ctx->num_sms, s);
+    double2* tc = (double2*)(base + o_Tc);
+    double2* zc = d_Z ? (double2*)(base + o_Zc) : nullptr;
+    int* map = (int*)(base + o_map);
+    cudaError_t e = launch_triangularize_one((int)n, (const double*)d_T, (const double*)d_Z, tc, zc, nullptr, map, s);
     if (e != cudaSuccess) return set_err(ctx, GS_CUDA, "triangularize launch: %s", cudaGetErrorString(e));
-    cT = tb.Tc;
-    cZ = tb.Zc;
-    cmap = tb.colmap;
+    cT = tc;
+    cZ = zc;
+    cmap = map;
   }
   cudaError_t e = launch_eigvecs_large((int)n, cT, cZ, d_VR, d_VL, !(flags & GS_RAW), cmap,
                                        (double2*)(base + o_ws), bad, s);
@@ -1393,7 +1379,6 @@ int gs_triangularize_f64(gs_context* ctx, int64_t n, const double* T, const doub
   const bool dev = flags & GS_DEVICE;
   const size_t nn = (size_t)n * n;
   Arena ar;
-  const size_t o_meta = ar.take<long long>(4);
   size_t o_T = 0, o_Z = 0, o_Tc = 0, o_Zc = 0, o_w = 0;
   if (!dev) {
     o_T = ar.take<double>(nn);
@@ -1406,16 +1391,7 @@ int gs_triangularize_f64(gs_context* ctx, int64_t n, const double* T, const doub
   if (rc) return rc;
   char* base = ctx->dws;
   cudaStream_t s = ctx->stream;
-  long long meta_h[4] = {0, 0, 0, 0};
-  int n32 = (int)n;
-  long long* meta = (long long*)(base + o_meta);
-  CK(cudaMemcpyAsync(meta, meta_h, sizeof(meta_h), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(meta + 2, &n32, sizeof(int), cudaMemcpyHostToDevice, s));
   TriBatch tb{};
-  tb.count = 1;
-  tb.ns = (const int*)(meta + 2);
-  tb.offs = meta;
-  tb.woffs = meta + 1;
   if (!dev) {
     CK(cudaMemcpyAsync(base + o_T, T, nn * sizeof(double), cudaMemcpyHostToDevice, s));
     if (Z) CK(cudaMemcpyAsync(base + o_Z, Z, nn * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -1431,8 +1407,7 @@ int gs_triangularize_f64(gs_context* ctx, int64_t n, const double* T, const doub
     tb.Zc = (double2*)Zc;
     tb.w = (double2*)w;
   }
-  tb.colmap = nullptr;
-  cudaError_t e = launch_triangularize(tb, ctx->num_sms, s);
+  cudaError_t e = launch_triangularize_one((int)n, tb.Tr, tb.Zr, tb.Tc, tb.Zc, tb.w, nullptr, s);
   if (e != cudaSuccess) return set_err(ctx, GS_CUDA, "triangularize launch: %s", cudaGetErrorString(e));
   if (dev) return GS_OK;
   CK(cudaMemcpyAsync(Tc, tb.Tc, nn * sizeof(double2), cudaMemcpyDeviceToHost, s));

@@ -228,6 +228,34 @@ def test_batched_mixed_blocks(gs, kind):
         assert_schur_real(A, T, Z, w)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("first", [0, 1, 3])
+@pytest.mark.parametrize("n", [1, 2, 3, 127, 128, 129, 130, 257])
+def test_triangularize_orders(gs, n, first):
+    """Blocks on and across the launch's row tiles: 1x1 up to `first`, then 2x2 (every third 1x1)."""
+    rng = np.random.default_rng(52 + n)
+    T = np.triu(rng.standard_normal((n, n)))
+    i, pairs = first, []
+    while i + 1 < n:
+        if i % 3 != 2:
+            T[i + 1, i + 1] = T[i, i]
+            T[i, i + 1], T[i + 1, i] = 1.5, -0.75
+            pairs.append(i)
+            i += 2
+        else:
+            i += 1
+    Z = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    S = gs.triangularize(gs.Schur(T, Z, np.zeros(n, dtype=complex)))
+    assert np.all(np.tril(S.T, -1) == 0)
+    assert np.linalg.norm(S.Z @ S.T @ S.Z.conj().T - Z @ T @ Z.T) <= 10 * n * EPS * np.linalg.norm(T)
+    assert np.linalg.norm(S.Z.conj().T @ S.Z - np.eye(n)) <= 10 * n * EPS
+    w = np.diag(T).astype(complex)
+    for k in pairs:  # in either order
+        w[k:k + 2] = S.T[k, k].real + 1j * np.sqrt(1.5 * 0.75) * np.sign(S.T[k, k].imag) * np.array([1, -1])
+        assert abs(S.T[k, k].real - T[k, k]) <= 10 * EPS * (abs(T[k, k]) + 1.5)
+    assert np.max(np.abs(np.diag(S.T) - w)) <= 10 * EPS * (np.max(np.abs(w)) + 1.5)
+
+
 def _block_weights(tp, tq, floor=1e-30):
     """The four weights per entry of k_sylv_solve's block solution, as the kernel forms them."""
     zp, zq = tp.shape[0], tq.shape[0]
