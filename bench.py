@@ -583,7 +583,7 @@ def measure_per_matrix(ctx, packed, ns, offs, sample=200):
 
 def measure_complex_and_adjoint(ctx, torch, dev, stream, steps=3):
     """Secondary configs on device-resident inputs, CUDA events on the library's stream:
-    (a) gschur! over 5,000 ComplexF64 matrices, n ~ U{8..128}, seed 5 (one persistent
+    (a) gschur! over 5,000 ComplexF64 matrices, n ~ U{8..128}, seed 5 (one
     launch sequence); (b) the differentiation workload -- 4,096 complex 64 x 64 matrices,
     seed 7: forward Schur + eigenvalue adjoint (eigenvectors recomputed from T, Z) per step."""
     from genericschur_gb300 import _capi

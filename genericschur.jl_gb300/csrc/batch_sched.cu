@@ -1,4 +1,4 @@
-// Work-queue construction for the persistent batched kernels: a counting sort of
+// Work-queue construction for the batched kernels: a counting sort of
 // the matrices by order, largest first, split into the size bins (bounds: the largest
 // order of each bin, ascending).
 // Runs on the device so that the whole batched pipeline is graph-capturable and

@@ -411,16 +411,15 @@ cudaError_t launch_std_blocks(int n, int N, const int* bs, const int* bz, double
 template <class S, class D> cudaError_t convert_array(const S* src, D* dst, size_t count, double scale, cudaStream_t s);
 cudaError_t launch_absmax(const double* A, size_t cnt, unsigned long long* out, int num_sms, cudaStream_t s);
 
-// Size bins of the persistent batched kernels.  `sched` holds, per bin, the
+// Size bins of the batched kernels.  `sched` holds, per bin, the
 // [start, end) range of that bin inside the sorted work order and a queue ticket
 // counter: sched[3*bin + {0,1,2}].
 constexpr int kNumBins = 4;
 __host__ __device__ constexpr int bin_max(int bin) { return 32 * (bin + 1); }  // 32, 64, 96, 128 (defaults)
 
-// Launch shape of the persistent batched kernels, per size bin: the largest order of
-// the bin (ascending, the last one kSmallMax), threads per CTA, whether the
-// Hessenberg phase runs on a full copy of the matrix in shared memory, and a cap on
-// resident CTAs per SM (0: as many as fit).  Chosen per GPU by the tuner
+// Launch shape of the batched kernels, per size bin: the largest order of
+// the bin (ascending, the last one kSmallMax), threads per CTA, a Hessenberg flag that
+// selects nothing any more, and a cap on resident CTAs per SM (0: a CTA per matrix).  Chosen per GPU by the tuner
 // (tune.py) and loaded with gs_set_tuning; the defaults are the hand-picked shapes.
 struct BinTuning {
   int bounds[kNumBins];

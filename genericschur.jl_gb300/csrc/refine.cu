@@ -9,7 +9,7 @@
 //     T_pp W_pq - W_pq T_qq = -L_pq - sum_{r>p} T_pr W_rq + sum_{r<q} W_pr T_rq,
 // a block triangular Sylvester equation (the iteration of Bujanovic, Kressner and
 // Schroeder, "Iterative refinement of Schur decompositions", Numer. Algorithms 2023),
-// solved in 32-row tiles (k_sylv_tile).
+// solved in 32-row tiles (k_sylv_rhs, k_sylv_solve).
 // Z is then updated to Z (I + S), which departs from orthogonality by O(|S|^2); a
 // Newton-Schulz step Z <- Z (3 I - Z^T Z) / 2 follows whenever |S| is above 1e-8.
 // Products with the small corrections S and (I - Z^T Z)/2 run in FP32 (their error is

@@ -125,7 +125,9 @@ __global__ void __launch_bounds__(128) k_tri_apply(int n, const double* __restri
   const int i = blockIdx.y * blockDim.x + threadIdx.x, j = blockIdx.x;
   if (i >= n) return;
   const auto sub = [&](int k) { return k >= 0 && k + 1 < n && Tr[(k + 1) + (long long)k * n] != 0.0; };
-  if (sub(j - 1)) return;  // second column of a block
+  // (in a T that is not quasi-triangular a third column or row in a run still gets values)
+  const auto second = [&](int k) { return sub(k - 1) && !sub(k - 2); };
+  if (second(j)) return;  // second column of a block
   const bool c2 = sub(j);
   const double2 gj = c2 ? Tc[(j + 1) + (long long)j * n] : make_double2(1.0, 0.0);
   if (Zc) {
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(128) k_tri_apply(int n, const double* __restri
     }
     Zc[i + (long long)j * n] = z1;
   }
-  if (i > j || sub(i - 1)) return;  // below the diagonal blocks, or second row of a block
+  if (i > j || second(i)) return;  // below the diagonal blocks, or second row of a block
   const bool r2 = sub(i);
   const auto tin = [&](int a, int b) { return make_double2(Tr[a + (long long)b * n], 0.0); };
   const double2 zero = make_double2(0.0, 0.0);

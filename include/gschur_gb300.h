@@ -125,7 +125,7 @@ GS_API int gs_schur_c64(gs_context* ctx, int64_t n, double* A, int64_t lda, doub
 
 /* ---------------------------------------------------------------------------
  * Batched forms (no reference counterpart: the reference handles one matrix per
- * call; these run gschur! on every matrix of a ragged batch in one persistent
+ * call; these run gschur! on every matrix of a ragged batch in one
  * launch sequence).  Matrix b has order ns[b] <= 128 and is stored column-major
  * with leading dimension ns[b] at element offset offs[b] of A and Z; its
  * eigenvalues start at element woffs[b] of wr/wi (or of w, complex).  status[b]
