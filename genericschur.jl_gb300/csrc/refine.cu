@@ -106,9 +106,13 @@ __global__ void __launch_bounds__(256) k_sylv_rhs(int n, int nT, int D, const do
 // The solution of T_pp W - W T_qq = R at one entry of its block, as four weights of the
 // block's R: W[a][b] = sum_{a'b'} k[a' + 2 b'] R[a'][b'].  With c the mean of T_qq's
 // diagonal, A = T_pp - c I and B = T_qq - c I, a 2x2 B has B^2 = -det(B) I, so
-// (A^2 + det(B) I) W = A R + R B; a 1x1 B is 0 and A W = R.  False when the weights could
-// lose more than about eight digits (nearly equal eigenvalues): Newton's step would still
-// converge with those, but such a tile is left to the pivoted elimination.
+// (A^2 + det(B) I) W = A R + R B; a 1x1 B is 0 and A W = R.  False, and the tile is left to
+// the pivoted elimination, when the weights could lose more than about eight digits (nearly
+// equal eigenvalues: Newton's step would still converge with those) or when a pivot of the
+// elimination could fall below `floor`, which it then raises: for blocks that are equal, or
+// equal to the last digits, W is bounded by that alone.  With m an order of the system and x
+// its largest entry, no pivot is below |det| / (pmax)^(m-1), pmax = x for m = 2 (at most two
+// entries meet) and 8 x for m = 4 (each of three steps at most doubles the entries).
 __device__ __forceinline__ bool block_weights(const double (*Ta)[kSt + 1], const double (*Tb)[kSt + 1], int sp, int zp,
                                               int sq, int zq, int a, int b, double floor, double k[4]) {
   k[0] = k[1] = k[2] = k[3] = 0.0;
@@ -132,12 +136,16 @@ __device__ __forceinline__ bool block_weights(const double (*Ta)[kSt + 1], const
     const double r = 1.0 / q;
     k[0] = (b == 0 ? a00 + b00 : b01) * r;  // R[0][0]
     k[2] = (b == 0 ? b10 : a00 - b00) * r;  // R[0][1]
-    return fma(a00, a00, fabs(det)) <= 1e8 * fabs(q);
+    const double x = fmax(fabs(a00) + fabs(b00), fmax(fabs(b01), fabs(b10)));
+    return fma(a00, a00, fabs(det)) <= 1e8 * fabs(q) && fabs(q) > 2.0 * floor * x;
   }
   const double a01 = Ta[sp][sp + 1], a10 = Ta[sp + 1][sp], a11 = Ta[sp + 1][sp + 1] - c;
   double q00 = a00, q01 = a01, q10 = a10, q11 = a11;
   double big = fmax(fmax(fabs(a00), fabs(a11)), fmax(fabs(a01), fabs(a10)));
+  double least = 2.0 * floor * big;  // of |dq|
   if (zq == 2) {
+    const double x8 = 8.0 * fmax(big + fabs(b00), fmax(fabs(b01), fabs(b10)));
+    least = floor * x8 * x8 * x8;
     const double tr = a00 + a11, x = a01 * a10;
     q00 = fma(a00, a00, x + det);
     q11 = fma(a11, a11, x + det);
@@ -161,7 +169,7 @@ __device__ __forceinline__ bool block_weights(const double (*Ta)[kSt + 1], const
     k[1] = i1;
   }
   const double qm = fmax(fmax(fabs(q00), fabs(q11)), fmax(fabs(q01), fabs(q10)));
-  return qm * big <= 1e8 * fabs(dq);
+  return qm * big <= 1e8 * fabs(dq) && fabs(dq) > least;
 }
 
 // Level D, step 2: one CTA per tile pair sums its partials (fixed order) and -L_PQ, then
