@@ -19,6 +19,49 @@
 namespace gsk {
 namespace {
 
+// One rotation after the other by one CTA, on a copy of T and Z in Tc and Zc (everything but the
+// closing triu!).
+template <int NT>
+__device__ void tri_sequential(int n, const double* __restrict__ Tr, const double* __restrict__ Zr,
+                               double2* __restrict__ Tc, double2* __restrict__ Zc) {
+  const int tid = threadIdx.x;
+  for (long long idx = tid; idx < (long long)n * n; idx += NT) {
+    Tc[idx] = make_double2(Tr[idx], 0.0);
+    if (Zc) Zc[idx] = make_double2(Zr ? Zr[idx] : ((idx % n) == (idx / n) ? 1.0 : 0.0), 0.0);
+  }
+  __syncthreads();
+  for (int j = n; j >= 2; --j) {
+    const double sub = Tr[(j - 1) + (long long)(j - 2) * n];  // Tr[j, j-1]
+    if (sub == 0.0) continue;
+    const double s = sqrt(fabs(sub));
+    const double cc = sqrt(fabs(Tr[(j - 2) + (long long)(j - 1) * n]));  // sqrt|Tr[j-1, j]|
+    const double r = hypot(s, cc);
+    const double gc = cc / r;      // Givens c (real)
+    const double gs = -(s / r);    // Givens s = i * gs (purely imaginary)
+    const int p = j - 2, q = j - 1;  // 0-based rows/cols of the block
+    // lmul!(G, T): rows p, q; new_p = c a1 + s a2; new_q = -conj(s) a1 + c a2, s = i gs
+    for (int k = tid; k < n; k += NT) {
+      const double2 a1 = Tc[p + (long long)k * n], a2 = Tc[q + (long long)k * n];
+      Tc[p + (long long)k * n] = make_double2(gc * a1.x - gs * a2.y, gc * a1.y + gs * a2.x);
+      Tc[q + (long long)k * n] = make_double2(gc * a2.x - gs * a1.y, gc * a2.y + gs * a1.x);
+    }
+    __syncthreads();
+    // rmul!(T, G') and rmul!(Z, G'): columns p, q; new_p = a1 c + a2 conj(s); new_q = -a1 s + a2 c
+    for (int k = tid; k < n; k += NT) {
+      double2 a1 = Tc[k + (long long)p * n], a2 = Tc[k + (long long)q * n];
+      Tc[k + (long long)p * n] = make_double2(gc * a1.x + gs * a2.y, gc * a1.y - gs * a2.x);
+      Tc[k + (long long)q * n] = make_double2(gc * a2.x + gs * a1.y, gc * a2.y - gs * a1.x);
+      if (Zc) {
+        a1 = Zc[k + (long long)p * n];
+        a2 = Zc[k + (long long)q * n];
+        Zc[k + (long long)p * n] = make_double2(gc * a1.x + gs * a2.y, gc * a1.y - gs * a2.x);
+        Zc[k + (long long)q * n] = make_double2(gc * a2.x + gs * a1.y, gc * a2.y - gs * a1.x);
+      }
+    }
+    __syncthreads();
+  }
+}
+
 template <int NT>
 __global__ void __launch_bounds__(NT) k_triangularize(TriBatch tb) {
   const int tid = threadIdx.x;
@@ -26,44 +69,8 @@ __global__ void __launch_bounds__(NT) k_triangularize(TriBatch tb) {
     const int n = tb.ns[b];
     const long long off = tb.offs[b];
     const double* __restrict__ Tr = tb.Tr + off;
-    const double* __restrict__ Zr = tb.Zr ? tb.Zr + off : nullptr;
     double2* __restrict__ Tc = tb.Tc + off;
-    double2* __restrict__ Zc = tb.Zc ? tb.Zc + off : nullptr;
-    for (int idx = tid; idx < n * n; idx += NT) {
-      Tc[idx] = make_double2(Tr[idx], 0.0);
-      if (Zc) Zc[idx] = make_double2(Zr ? Zr[idx] : ((idx % n) == (idx / n) ? 1.0 : 0.0), 0.0);
-    }
-    __syncthreads();
-    for (int j = n; j >= 2; --j) {
-      const double sub = Tr[(j - 1) + (long long)(j - 2) * n];  // Tr[j, j-1]
-      if (sub == 0.0) continue;
-      const double s = sqrt(fabs(sub));
-      const double cc = sqrt(fabs(Tr[(j - 2) + (long long)(j - 1) * n]));  // sqrt|Tr[j-1, j]|
-      const double r = hypot(s, cc);
-      const double gc = cc / r;      // Givens c (real)
-      const double gs = -(s / r);    // Givens s = i * gs (purely imaginary)
-      const int p = j - 2, q = j - 1;  // 0-based rows/cols of the block
-      // lmul!(G, T): rows p, q; new_p = c a1 + s a2; new_q = -conj(s) a1 + c a2, s = i gs
-      for (int k = tid; k < n; k += NT) {
-        const double2 a1 = Tc[p + (long long)k * n], a2 = Tc[q + (long long)k * n];
-        Tc[p + (long long)k * n] = make_double2(gc * a1.x - gs * a2.y, gc * a1.y + gs * a2.x);
-        Tc[q + (long long)k * n] = make_double2(gc * a2.x - gs * a1.y, gc * a2.y + gs * a1.x);
-      }
-      __syncthreads();
-      // rmul!(T, G') and rmul!(Z, G'): columns p, q; new_p = a1 c + a2 conj(s); new_q = -a1 s + a2 c
-      for (int k = tid; k < n; k += NT) {
-        double2 a1 = Tc[k + (long long)p * n], a2 = Tc[k + (long long)q * n];
-        Tc[k + (long long)p * n] = make_double2(gc * a1.x + gs * a2.y, gc * a1.y - gs * a2.x);
-        Tc[k + (long long)q * n] = make_double2(gc * a2.x + gs * a1.y, gc * a2.y - gs * a1.x);
-        if (Zc) {
-          a1 = Zc[k + (long long)p * n];
-          a2 = Zc[k + (long long)q * n];
-          Zc[k + (long long)p * n] = make_double2(gc * a1.x + gs * a2.y, gc * a1.y - gs * a2.x);
-          Zc[k + (long long)q * n] = make_double2(gc * a2.x + gs * a1.y, gc * a2.y - gs * a1.x);
-        }
-      }
-      __syncthreads();
-    }
+    tri_sequential<NT>(n, Tr, tb.Zr ? tb.Zr + off : nullptr, Tc, tb.Zc ? tb.Zc + off : nullptr);
     // triu!(T), values = diag(T), column map
     for (int idx = tid; idx < n * n; idx += NT) {
       const int i = idx % n, jj = idx / n;
@@ -91,7 +98,11 @@ __global__ void __launch_bounds__(NT) k_triangularize(TriBatch tb) {
 // block's and then its row block's (descending order), and each 2x2 tile of blocks is one
 // thread's.  k_tri_rot leaves (cs, -sn) of each block in the block's subdiagonal place, which
 // k_tri_finish clears.  One CTA, two passes and two barriers per block, took 12.8 ms at
-// n = 1024 with vectors; these three launches take less than 0.4 ms together.
+// n = 1024 with vectors; these launches take less than 0.4 ms together.
+// In a T that is not quasi-triangular (two nonzero subdiagonal entries in a row) the rotations
+// overlap: k_tri_rot then sets the flag, and k_tri_runs applies them one after the other.
+__host__ __device__ __forceinline__ double* tri_flag(int n, double2* Tc) { return n > 2 ? &Tc[2].x : nullptr; }  // place (3, 1)
+
 __global__ void k_tri_rot(int n, const double* __restrict__ Tr, double2* __restrict__ Tc) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x + 2;
   if (j > n) return;
@@ -102,6 +113,7 @@ __global__ void k_tri_rot(int n, const double* __restrict__ Tr, double2* __restr
     const double cc = sqrt(fabs(Tr[(j - 2) + (long long)(j - 1) * n]));  // sqrt|Tr[j-1, j]|
     const double r = hypot(s, cc);
     g = make_double2(cc / r, -(s / r));
+    if (j > 2 && Tr[(j - 2) + (long long)(j - 3) * n] != 0.0) *tri_flag(n, Tc) = 1.0;
   }
   Tc[(j - 1) + (long long)(j - 2) * n] = g;
 }
@@ -123,10 +135,9 @@ __device__ __forceinline__ void tri_rows(double gc, double gs, double2& x1, doub
 __global__ void __launch_bounds__(128) k_tri_apply(int n, const double* __restrict__ Tr, const double* __restrict__ Zr,
                                                    double2* Tc, double2* __restrict__ Zc) {
   const int i = blockIdx.y * blockDim.x + threadIdx.x, j = blockIdx.x;
-  if (i >= n) return;
+  if (i >= n || (n > 2 && *tri_flag(n, Tc) != 0.0)) return;
   const auto sub = [&](int k) { return k >= 0 && k + 1 < n && Tr[(k + 1) + (long long)k * n] != 0.0; };
-  // (in a T that is not quasi-triangular a third column or row in a run still gets values)
-  const auto second = [&](int k) { return sub(k - 1) && !sub(k - 2); };
+  const auto second = [&](int k) { return sub(k - 1); };
   if (second(j)) return;  // second column of a block
   const bool c2 = sub(j);
   const double2 gj = c2 ? Tc[(j + 1) + (long long)j * n] : make_double2(1.0, 0.0);
@@ -170,6 +181,13 @@ __global__ void __launch_bounds__(128) k_tri_apply(int n, const double* __restri
   if (r2 && c2) Tc[(i + 1) + (long long)(j + 1) * n] = x22;
 }
 
+// One CTA; nothing to do for a quasi-triangular T.
+__global__ void __launch_bounds__(256) k_tri_runs(int n, const double* Tr, const double* Zr, double2* Tc, double2* Zc) {
+  const bool runs = *tri_flag(n, Tc) != 0.0;
+  __syncthreads();  // the flag is in the way of the copy
+  if (runs) tri_sequential<256>(n, Tr, Zr, Tc, Zc);
+}
+
 // triu!(T), values = diag(T), column map
 __global__ void k_tri_finish(int n, const double* __restrict__ Tr, double2* __restrict__ Tc, double2* __restrict__ w,
                              int* __restrict__ colmap) {
@@ -196,8 +214,13 @@ __global__ void k_tri_finish(int n, const double* __restrict__ Tr, double2* __re
 cudaError_t launch_triangularize_one(int n, const double* Tr, const double* Zr, double2* Tc, double2* Zc, double2* w,
                                      int* colmap, cudaStream_t s) {
   if (n < 1) return cudaSuccess;
+  if (double* flag = tri_flag(n, Tc)) {
+    cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(double), s);
+    if (e != cudaSuccess) return e;
+  }
   k_tri_rot<<<(n + 127) / 128, 128, 0, s>>>(n, Tr, Tc);
   k_tri_apply<<<dim3(n, (n + 127) / 128), 128, 0, s>>>(n, Tr, Zr, Tc, Zc);
+  if (n > 2) k_tri_runs<<<1, 256, 0, s>>>(n, Tr, Zr, Tc, Zc);
   k_tri_finish<<<(int)std::min<size_t>(((size_t)n * n + 255) / 256, 4096), 256, 0, s>>>(n, Tr, Tc, w, colmap);
   return cudaGetLastError();
 }
