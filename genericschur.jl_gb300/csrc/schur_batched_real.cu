@@ -179,6 +179,14 @@ __device__ __forceinline__ void hess_scale(double amax, F each) {
   __syncthreads();
 }
 
+// Where the reduction leaves max|a| for the iteration, which undoes the scaling: below the subdiagonal of
+// A.  (Not with the eigenvalues: where the iteration gives up, those that it did not find keep what the
+// caller had there.)  Orders 1 and 2 have no such place, but deflate at once.
+template <class T, class W>
+__device__ __forceinline__ T* amax_place(T* Ag, W* wr, int n) {
+  return n > 2 ? Ag + (n - 1) : reinterpret_cast<T*>(wr);
+}
+
 template <class W, int NC>
 __global__ void __launch_bounds__(4 * NC) k_hess_real64(RealBatchT<double, W> bt, const int* __restrict__ order,
                                                         const int* __restrict__ sched, int bin, int nmax, int cap) {
@@ -278,7 +286,7 @@ __global__ void __launch_bounds__(4 * NC) k_hess_real64(RealBatchT<double, W> bt
       if (i <= j + 1) Ag[idx] = A[i + j * ld];
       if (zs) Zg[idx] = Z[i + j * ld];
     }
-    if (tid == 0) bt.wr[bt.woffs[b]] = (W)amax;  // for the unscaling; k_schur_real overwrites it
+    if (tid == 0) *amax_place(Ag, bt.wr + bt.woffs[b], n) = amax;
   }
 }
 
@@ -287,8 +295,8 @@ __global__ void __launch_bounds__(4 * NC) k_hess_real64(RealBatchT<double, W> bt
 // are kernels of their own.  A pair of neighbouring lanes holds a column or row of A.  A line's entries
 // stay in registers between its dot product and its update, in blocks of eight (A is padded by 16
 // zero rows and columns so that a block needs no bounds), and the reflector is read four entries at a
-// time.  The essential parts of the reflectors stay below the subdiagonal of A and their scalars
-// in the (not yet computed) imaginary parts of the eigenvalues, for k_formq_real32.
+// time.  The essential parts of the reflectors stay below the subdiagonal of A, for k_formq_real32, and
+// their scalars and max|a|, whose place they take, in the (not yet formed) Z.
 constexpr int kHessPad = 16;
 // leading dimension = 18 mod 32: sixteen columns' pairs of neighbouring rows fall into 32 banks,
 // and sixteen rows' pairs of neighbouring columns into 30
@@ -356,7 +364,7 @@ __global__ void __launch_bounds__(NC == 32 ? 128 : 2 * NC, NC == 128 ? 2 : (NC =
     const int n = bt.ns[b];
     if (n <= 0 || n > nmax) continue;  // k_schur_real reports it
     T* __restrict__ Ag = bt.A + bt.offs[b];
-    W* __restrict__ taus = bt.wi + bt.woffs[b];
+    T* __restrict__ taus = bt.wantz ? bt.Z + bt.offs[b] : nullptr;
     const int ld = hess_ld32(n);
     T* A = (T*)smem_raw;
     __syncthreads();  // the previous matrix is out of shared memory
@@ -397,7 +405,7 @@ __global__ void __launch_bounds__(NC == 32 ? 128 : 2 * NC, NC == 128 ? 2 : (NC =
         if (tid == 0) {
           sh.c.mode = mode;
           sh.c.tau = tau;
-          taus[i - 1] = (W)tau;
+          if (taus) taus[i - 1] = tau;
           if (mode == 1) col[0] = beta;
         }
         if (mode == 1 && tid < NC) {
@@ -418,7 +426,10 @@ __global__ void __launch_bounds__(NC == 32 ? 128 : 2 * NC, NC == 128 ? 2 : (NC =
           if (1 + tid < m) col[1 + tid] = v;
           ca[tid & 1][tid >> 1] = v;
         }
-        if (tid == 0) { col[0] = beta; taus[i - 1] = (W)tau; }
+        if (tid == 0) {
+          col[0] = beta;
+          if (taus) taus[i - 1] = tau;
+        }
         __syncthreads();
       }
       if (tau == T(0)) continue;
@@ -433,11 +444,15 @@ __global__ void __launch_bounds__(NC == 32 ? 128 : 2 * NC, NC == 128 ? 2 : (NC =
     __syncthreads();
     for (int j = warp; j < n; j += NT / 32)
       for (int i = lane; i < n; i += 32) Ag[i + j * n] = A[i + j * ld];
-    if (tid == 0) bt.wr[bt.woffs[b]] = (W)amax;  // for the unscaling; k_schur_real overwrites it
+    __syncthreads();
+    if (tid == 0) {
+      if (taus && n > 2) taus[n - 1] = (T)amax;
+      else *amax_place(Ag, bt.wr + bt.woffs[b], n) = (T)amax;
+    }
   }
 }
 
-// FP32 formation of Z (hessenberg.jl:150-166) from the reflectors that k_hess_real32 left in A and wi.
+// FP32 formation of Z (hessenberg.jl:150-166) from the reflectors that k_hess_real32 left in A and Z.
 // Z stays in registers from the identity to the end: a pair of neighbouring lanes holds a row, one lane
 // the even columns, the other the odd ones.  Two reflectors are staged in shared memory ahead, by
 // absolute column: cd with 0, cu with 1 at column i.
@@ -456,9 +471,9 @@ __global__ void __launch_bounds__(2 * NC, NC == 128 ? 2 : (NC == 64 ? 6 : 16))
     const int b = order[job];
     const int n = bt.ns[b];
     if (n <= 0 || n > nmax) continue;
-    const T* __restrict__ Ag = bt.A + bt.offs[b];
-    T* __restrict__ Zg = bt.Z + bt.offs[b];
-    if (tid < n) taus[tid] = (T)bt.wi[bt.woffs[b] + tid];
+    T* Ag = bt.A + bt.offs[b];
+    T* Zg = bt.Z + bt.offs[b];
+    if (tid < n && n > 2) taus[tid] = Zg[tid];
     const bool zrow = (c & ~15) < n;
     const int bz = ((n + 1) / 2 + 7) / 8;
     T z[HC];  // Z(c, par + 2 e)
@@ -502,6 +517,7 @@ __global__ void __launch_bounds__(2 * NC, NC == 128 ? 2 : (NC == 64 ? 6 : 16))
       for (int e = 0; e < HC; ++e)
         if (2 * e + par < n) Zg[c + (2 * e + par) * n] = z[e];
     }
+    if (tid == n - 1 && n > 2) *amax_place(Ag, bt.wr, n) = taus[tid];  // (this thread alone has read that place)
     __syncthreads();  // before the next matrix's reflectors
   }
 }
@@ -859,6 +875,7 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
   __shared__ T blks[kSmallMax * 2];  // kInOrder: the standardised blocks
   constexpr bool kInOrder = sizeof(T) == 4 && sizeof(W) == 8;
   __shared__ int s_giv;
+  __shared__ double s_amax;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const int n = bt.ns[b];
@@ -872,16 +889,7 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
   W* __restrict__ wi = bt.wi + bt.woffs[b];
   T* logs = smem;
   T* H = smem + kLogElems;  // packed H
-  // the scale that the reduction applied
-  const double amax = (double)wr[0];
-  const double smlnum = sqrt((double)Prec<T>::fmin) / (double)Prec<T>::eps;
-  const double bignum = 1.0 / smlnum;
-  bool scaled = false;
-  double cscale = 1.0;
-  if (bt.scale) {
-    if (amax > 0.0 && amax < smlnum) { scaled = true; cscale = smlnum; }
-    else if (amax > bignum) { scaled = true; cscale = bignum; }
-  }
+  if (tid == 0) s_amax = (double)*amax_place(Ag, wr, n);
   for (int j = 1 + warp; j <= n; j += NT / 32)
     for (int i = 1 + lane; i <= j + 3; i += 32)
       HH(i, j) = (i <= min(j + 1, n)) ? Ag[(i - 1) + (long long)(j - 1) * n] : T(0);
@@ -1163,16 +1171,22 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
   __syncthreads();
 
   // ---- write back ----
+  // (undoing the scale that the reduction applied)
   double mul[8];
   int nf = 0;
-  if (scaled) nf = safescale_factors(cscale, amax, mul);
+  if (bt.scale) {
+    const double smlnum = sqrt((double)Prec<T>::fmin) / (double)Prec<T>::eps, amax = s_amax;
+    const double bignum = 1.0 / smlnum;
+    if (amax > 0.0 && amax < smlnum) nf = safescale_factors(smlnum, amax, mul);
+    else if (amax > bignum) nf = safescale_factors(bignum, amax, mul);
+  }
   for (int idx = tid; idx < n * n; idx += NT) {
     const int i = idx % n, j = idx / n;
     double v = (i > j + 1) ? 0.0 : (double)HH(i + 1, j + 1);
     for (int f = 0; f < nf; ++f) v *= mul[f];
     Ag[idx] = (T)v;
   }
-  if (scaled)
+  if (nf)
     for (int i = tid; i < n; i += NT) {
       double a = wr[i], bq = wi[i];
       for (int f = 0; f < nf; ++f) { a *= mul[f]; bq *= mul[f]; }
