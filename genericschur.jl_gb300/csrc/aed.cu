@@ -505,7 +505,7 @@ cudaError_t launch_ordschur_cplx(double2* T, double2* Z, int n, const int* selec
 
 template <class T>
 __global__ void __launch_bounds__(kAedThreads) k_aed(AedArgs<T> g) {
-  extern __shared__ double aed_raw[];
+  extern __shared__ __align__(16) double aed_raw[];
   __shared__ AedShared<T> sh;
   __shared__ double red[32];
   const int tid = threadIdx.x;

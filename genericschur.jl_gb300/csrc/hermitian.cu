@@ -879,7 +879,7 @@ __device__ __forceinline__ void apply_phase(S* Z, long long ldz, int r, const St
 template <class S>
 __global__ void __launch_bounds__(kHeT) k_steqr(int n, double* dg, double* eg, S* Z, long long ldz, int nz,
                                                  double* rot, StCtl* ctl, long long maxsweeps, int smem_de) {
-  extern __shared__ double sde[];
+  extern __shared__ __align__(16) double sde[];
   const bool wantZ = Z != nullptr && nz > 0;
   const bool chain = blockIdx.x == 0 && threadIdx.x < 32;  // warp 0 of block 0, lanes in lockstep
   const int lane = threadIdx.x & 31;

@@ -998,7 +998,7 @@ __device__ void ht_real(double* H, double* B, int ld, double* Q, double* Z, int 
 }
 
 __global__ void __launch_bounds__(kQrT, 3) k_ggschur_real(QzrBatch bt, int cap) {
-  extern __shared__ double smq[];
+  extern __shared__ __align__(16) double smq[];
   __shared__ double red[kQrT / 32];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int b = blockIdx.x; b < bt.count; b += gridDim.x) {

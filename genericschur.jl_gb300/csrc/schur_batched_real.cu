@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(4 * NC) k_hess_real64(RealBatchT<double, W> bt
                                                         const int* __restrict__ sched, int bin, int nmax, int cap) {
   typedef double T;
   constexpr int NT = 4 * NC;
-  extern __shared__ double smem_raw[];
+  extern __shared__ __align__(16) double smem_raw[];
   __shared__ T part[4][NC];
   __shared__ HessShared<T> sh;
   const int tid = threadIdx.x;
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(NC == 32 ? 128 : 2 * NC, NC == 128 ? 2 : (NC =
   typedef float T;
   // at least the four warps of the norm
   constexpr int NT = 2 * NC < 128 ? 128 : 2 * NC, HC = NC / 2, NB = HC / 8;
-  extern __shared__ double smem_raw[];
+  extern __shared__ __align__(16) double smem_raw[];
   __shared__ __align__(16) T ca[2][HC + 4];  // the reflector's odd and even entries, in different banks
   __shared__ HessShared<T> sh;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1201,7 +1201,7 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
 template <class T, class W, int NT>
 __global__ void __launch_bounds__(NT, 768 / NT) k_schur_real(RealBatchT<T, W> bt, const int* __restrict__ order,
                                                    int* __restrict__ sched, int bin, int nmax, int num_sms, int once) {
-  extern __shared__ double smem_raw[];
+  extern __shared__ __align__(16) double smem_raw[];
   T* smem = (T*)smem_raw;
   __shared__ int s_job;
   const int start = sched[3 * bin], end = sched[3 * bin + 1];

@@ -52,7 +52,7 @@ struct ChaseRf {
 
 template <class T>
 __global__ void __launch_bounds__(32 * kChaseWarps) k_chase_chunk(ChaseArgs<T> ca) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   T* W = (T*)smraw;
   const int nw = ca.whi - ca.wlo + 1;
   const int ldw = nw | 1;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(32 * kChaseWarps) k_chase_chunk(ChaseArgs<T> c
 // (right updates on H), then tiles of rows of Z (right updates on Z).
 template <class T>
 __global__ void __launch_bounds__(256) k_chase_far(ChaseArgs<T> ca, int nleft, int nright, int nz) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   const int nw = ca.whi - ca.wlo + 1;
   const int steps = ca.w;
   T* lr = (T*)smraw;                                    // steps*B*5 reflector scalars
