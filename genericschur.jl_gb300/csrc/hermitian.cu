@@ -38,6 +38,9 @@ namespace {
 constexpr int kHeT = 256;
 constexpr int kHeOneCta = 32;  // orders of k_he_tridiag that one CTA takes alone
 constexpr int kHeCols = 4;     // columns per CTA above that, until every SM has a CTA
+#ifndef GS_HE_WAIT_POLLS  // polls of a grid-wide wait before it gives up, some seconds (a test builds with 0)
+#define GS_HE_WAIT_POLLS (1 << 22)
+#endif
 
 template <class S> struct Hs;
 template <> struct Hs<double> {
@@ -95,14 +98,20 @@ static_assert(offsetof(HeCtl<double>, err) == kHeErrOffset<double> && offsetof(H
 
 // Full Hermitian matrix B (ld n) in the lower-form frame from the triangle `upper` of A.
 template <class S>
-__global__ void k_he_prep(const S* __restrict__ A, long long lda, int n, int upper, S* __restrict__ B) {
+__global__ void k_he_prep(const S* __restrict__ A, long long lda, int n, int upper, S* __restrict__ B, S* __restrict__ tau,
+                          double* __restrict__ d, double* __restrict__ sub) {
   const size_t tot = (size_t)n * n;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
     const int k = (int)(e % n), l = (int)(e / n);
     S v;
     if (!upper) v = (k >= l) ? A[k + l * lda] : Hs<S>::conj(A[l + k * lda]);
     else v = (k >= l) ? A[(n - 1 - k) + (n - 1 - l) * lda] : Hs<S>::conj(A[(n - 1 - l) + (n - 1 - k) * lda]);
-    if (k == l) v = Hs<S>::from(Hs<S>::re(v));
+    if (k == l) {
+      v = Hs<S>::from(Hs<S>::re(v));
+      // defined values for what runs before the host learns that a wait gave up
+      d[k] = 0.0;
+      if (k < n - 1) { sub[k] = 0.0; tau[k] = Hs<S>::zero(); }
+    }
     B[e] = v;
   }
 }
@@ -254,7 +263,7 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 // seconds or when another CTA has.
 __device__ bool he_wait(const unsigned* p, unsigned target, int* err) {
   for (int it = 0; ld_acquire(p) < target; ++it) {
-    if (it >= (1 << 22)) atomicOr(err, 1);
+    if (it >= GS_HE_WAIT_POLLS) atomicOr(err, 1);
     if ((it & 1023) == 1023 && *(volatile int*)err) return false;
   }
   return true;
@@ -449,11 +458,6 @@ __global__ void __launch_bounds__(kHeT) k_he_tridiag(S* B, int n, S* W, HeCtl<S>
       }
     }
   }
-  if (bad && b == 0)
-    for (int k = tid; k < n; k += kHeT) {
-      d[k] = 0.0;
-      if (k < n - 1) e[k] = 0.0;
-    }
 }
 
 // Q = H_1 ... H_{n-1}, column by column: column j of Q is e_j under the reflectors
@@ -995,7 +999,7 @@ template <class S>
 cudaError_t launch_he_tridiag(const S* A, long long lda, int n, int upper, S* B, S* W, S* partial, int npart,
                               HeCtlBuf* cbuf, S* tau, double* d, double* e, int num_sms, cudaStream_t s) {
   HeCtl<S>* ctl = reinterpret_cast<HeCtl<S>*>(cbuf);
-  k_he_prep<S><<<grid_of((size_t)n * n), 256, 0, s>>>(A, lda, n, upper, B);
+  k_he_prep<S><<<grid_of((size_t)n * n), 256, 0, s>>>(A, lda, n, upper, B, tau, d, e);
   cudaError_t err = cudaMemsetAsync(ctl, 0, sizeof(HeCtl<S>), s);
   if (err != cudaSuccess) return err;
   // one kernel where the matrix fits in the chip's shared memory
@@ -1005,7 +1009,10 @@ cudaError_t launch_he_tridiag(const S* A, long long lda, int n, int upper, S* B,
     err = cudaFuncSetAttribute(k_he_tridiag<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
     if (err != cudaSuccess) return err;
     void* args[] = {&B, &n, &W, &ctl, &tau, &d, &e};
-    return cudaLaunchCooperativeKernel((const void*)k_he_tridiag<S>, dim3(G), dim3(kHeT), args, smem, s);
+    err = cudaLaunchCooperativeKernel((const void*)k_he_tridiag<S>, dim3(G), dim3(kHeT), args, smem, s);
+    // a process that may use a part of the SMs only (MPS) cannot have them all resident
+    if (err != cudaErrorCooperativeLaunchTooLarge) return err;
+    (void)cudaGetLastError();
   }
   k_he_first<S><<<1, kHeT, 0, s>>>(B, n, ctl, tau, d, e);
   for (int i = 0; i <= n - 2; ++i) {
