@@ -720,7 +720,7 @@ size_t aed_smem_bytes(int nw) {
 template <class T>
 cudaError_t launch_aed(const AedArgs<T>& g, cudaStream_t s) {
   const size_t sm = aed_smem_bytes<T>(g.nw);
-  cudaError_t e = cudaFuncSetAttribute(k_aed<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k_aed<T>, kMostSmem);
   if (e != cudaSuccess) return e;
   k_aed<T><<<1, kAedThreads, sm, s>>>(g);
   return cudaGetLastError();

@@ -66,7 +66,7 @@ size_t eig_adjoint_smem_bytes(int nmax) { return sizeof(double2) * (size_t)nmax;
 
 cudaError_t launch_eig_adjoint(const AdjBatch& ab, int nmax, int num_sms, cudaStream_t s) {
   const size_t smem = eig_adjoint_smem_bytes(nmax);
-  cudaError_t e = cudaFuncSetAttribute(k_eig_adjoint<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k_eig_adjoint<256>, eig_adjoint_smem_bytes(kSmallMax));
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_eig_adjoint<256>, 256, smem);

@@ -389,7 +389,7 @@ size_t eigvecs_smem_bytes(int nmax) {
 
 cudaError_t launch_eigvecs_batched(const EigBatch& eb, int nmax, int num_sms, cudaStream_t s) {
   const size_t smem = eigvecs_smem_bytes(nmax);
-  cudaError_t e = cudaFuncSetAttribute(k_eigvecs<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k_eigvecs<128>, eigvecs_smem_bytes(kSmallMax));
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_eigvecs<128>, 128, smem);

@@ -13,6 +13,15 @@ constexpr int kSmallMax = 128;
 // Largest dynamic shared memory a CTA may use on sm_103 (227 KiB), less the kernels'
 // static shared memory.
 constexpr size_t kMaxDynSmem = 227 * 1024 - 1024;
+// ... beside up to 9 KB of static arrays.
+constexpr size_t kMostSmem = kMaxDynSmem - 8 * 1024;
+
+// Lets a kernel's launches ask for up to `most` bytes of dynamic shared memory.  The limit belongs to the
+// function, not to a launch: `most` is the same in every call, so that a launch that another thread makes
+// in between cannot lower it below what this one needs.
+template <class F> cudaError_t allow_smem(F* kernel, size_t most) {
+  return cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
 
 // Per-matrix status codes (also the C-ABI return codes).
 enum : int { ST_OK = 0, ST_UNCONVERGED = 1, ST_BADARG = 2, ST_CUDA = 3 };

@@ -1006,7 +1006,7 @@ cudaError_t launch_he_tridiag(const S* A, long long lda, int n, int upper, S* B,
   const int G = n <= kHeOneCta ? 1 : std::min(num_sms, (n + kHeCols - 1) / kHeCols);
   const size_t smem = ((size_t)((n + G - 1) / G) + 2) * n * sizeof(S);
   if (smem <= kMaxDynSmem) {
-    err = cudaFuncSetAttribute(k_he_tridiag<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
+    err = allow_smem(k_he_tridiag<S>, kMaxDynSmem);
     if (err != cudaSuccess) return err;
     void* args[] = {&B, &n, &W, &ctl, &tau, &d, &e};
     err = cudaLaunchCooperativeKernel((const void*)k_he_tridiag<S>, dim3(G), dim3(kHeT), args, smem, s);
@@ -1031,7 +1031,7 @@ cudaError_t launch_he_formq(const S* B, int n, const S* tau, S* Q, int num_sms, 
   const int nw = (int)std::min<size_t>(kHeT / 32, kMaxDynSmem / ((size_t)n * sizeof(S)));
   if (nw >= 4) {
     const size_t smem = (size_t)nw * n * sizeof(S);
-    cudaError_t err = cudaFuncSetAttribute(k_he_formq_cols<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
+    cudaError_t err = allow_smem(k_he_formq_cols<S>, kMaxDynSmem);
     if (err != cudaSuccess) return err;
     k_he_formq_cols<S><<<std::min(n, num_sms), 32 * nw, smem, s>>>(B, n, tau, Q);
     return cudaGetLastError();

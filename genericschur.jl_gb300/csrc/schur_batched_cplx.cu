@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 512 / NT : 2) k_schur_cplx(Cpl
 // Dynamic shared memory of one CTA of the iteration and of the reduction for orders up to nmax.
 size_t ciqr_smem_bytes() { return sizeof(double2) * (2 * kZLogElems + kZWinElems); }
 size_t chess_smem_elems(int nmax) {
-  const size_t one = (size_t)nmax * (nmax | 1), most = (kMaxDynSmem - 8 * 1024) / sizeof(double2);
+  const size_t one = (size_t)nmax * (nmax | 1), most = kMostSmem / sizeof(double2);
   return one <= most ? one : most;
 }
 
@@ -836,7 +836,7 @@ template <int NC>
 cudaError_t launch_hess_c(const CplxBatch& bt, const int* order, const int* sched, int bin, int nmax, int num_sms,
                           cudaStream_t s) {
   const size_t elems = chess_smem_elems(nmax), smem = sizeof(double2) * elems;
-  cudaError_t e = cudaFuncSetAttribute(k_hess_cplx<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k_hess_cplx<NC>, sizeof(double2) * chess_smem_elems(NC));
   if (e != cudaSuccess) return e;
   k_hess_cplx<NC><<<bt.count, 4 * NC, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
   return cudaGetLastError();
@@ -850,7 +850,7 @@ cudaError_t launch_bin_c(const CplxBatch& bt, const int* order, int* sched, int 
                                            : launch_hess_c<128>(bt, order, sched, bin, nmax, num_sms, s));
   if (e != cudaSuccess) return e;
   const size_t smem = ciqr_smem_bytes();
-  e = cudaFuncSetAttribute(k_schur_cplx<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = allow_smem(k_schur_cplx<NT>, smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_cplx<NT>, NT, smem);

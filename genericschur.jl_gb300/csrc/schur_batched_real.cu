@@ -1231,7 +1231,7 @@ size_t bin_smem_elems(int nmax) { return kLogElems + (size_t)rpk(nmax + 1); }
 // ... of the reduction: FP64 the matrix, and Z where both fit; FP32 the padded matrix.
 size_t hess_smem_elems(int nmax, size_t tsize) {
   if (tsize == 4) return (size_t)(nmax + kHessPad) * hess_ld32(nmax);
-  const size_t one = (size_t)nmax * (nmax | 1), most = (kMaxDynSmem - 8 * 1024) / tsize;
+  const size_t one = (size_t)nmax * (nmax | 1), most = kMostSmem / tsize;
   return 2 * one <= most ? 2 * one : (one > most ? one : most);
 }
 
@@ -1243,7 +1243,7 @@ cudaError_t launch_hess(const RealBatchT<T, W>& bt, const int* order, const int*
   const void* f;
   if constexpr (sizeof(T) == 8) f = (const void*)k_hess_real64<W, NC>;
   else f = (const void*)k_hess_real32<W, NC>;
-  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(f, sizeof(T) * hess_smem_elems(NC, sizeof(T)));
   if (e != cudaSuccess) return e;
   const int ctas = bt.count;
   if constexpr (sizeof(T) == 8) {
@@ -1265,7 +1265,7 @@ cudaError_t launch_bin(const RealBatchT<T, W>& bt, const int* order, int* sched,
                                            : launch_hess<T, W, 128>(bt, order, sched, bin, nmax, num_sms, s));
   if (e != cudaSuccess) return e;
   const size_t smem = sizeof(T) * bin_smem_elems(nmax);
-  e = cudaFuncSetAttribute(k_schur_real<T, W, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = allow_smem(k_schur_real<T, W, NT>, sizeof(T) * bin_smem_elems(kSmallMax));
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_real<T, W, NT>, NT, smem);

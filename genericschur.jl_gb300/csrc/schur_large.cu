@@ -350,7 +350,7 @@ template <class T>
 cudaError_t launch_chase_chunk(const ChaseArgs<T>& ca, int num_sms, cudaStream_t s) {
   const int nw = ca.whi - ca.wlo + 1;
   size_t sm = chase_smem_bytes<T>(nw);
-  cudaError_t e = cudaFuncSetAttribute(k_chase_chunk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k_chase_chunk<T>, kMostSmem);
   if (e != cudaSuccess) return e;
   k_chase_chunk<T><<<1, 32 * kChaseWarps, sm, s>>>(ca);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -360,7 +360,7 @@ cudaError_t launch_chase_chunk(const ChaseArgs<T>& ca, int num_sms, cudaStream_t
   const int tiles = nleft + nright + nz;
   if (tiles == 0) return cudaSuccess;
   sm = far_smem_bytes<T>(nw, ca.w, ca.B);
-  e = cudaFuncSetAttribute(k_chase_far<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  e = allow_smem(k_chase_far<T>, kMostSmem);
   if (e != cudaSuccess) return e;
   k_chase_far<T><<<tiles, 256, sm, s>>>(ca, nleft, nright, nz);
   (void)num_sms;

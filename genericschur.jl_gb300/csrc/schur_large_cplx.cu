@@ -759,7 +759,7 @@ int schur_large_cplx_run(double2* A, double2* Z, double2* w, int n, int scale, l
       const int kwtop = ihi - nw + 1;
       if (small_solve(kwtop, ihi, true, bw)) return -1;
       const size_t sm = sizeof(double2) * (2 * (size_t)nw * nw + 2 * nw);
-      CKZ(cudaFuncSetAttribute(k_zaed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+      CKZ(allow_smem(k_zaed, kMostSmem));
       k_zaed<<<1, 256, sm, s>>>(H, n, kwtop, ilo, blk, U, nw, aout, bw, abeta);
       CKZ(cudaGetLastError());
       int ao[2] = {0, 0}, wst = 0;
@@ -839,7 +839,7 @@ int schur_large_cplx_run(double2* A, double2* Z, double2* w, int n, int scale, l
       ca.logr = logr;
       const int nw = ca.whi - ca.wlo + 1;
       size_t sm = sizeof(double2) * (size_t)nw * nw;
-      CKZ(cudaFuncSetAttribute(k_zchase_chunk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+      CKZ(allow_smem(k_zchase_chunk, kMostSmem));
       k_zchase_chunk<<<1, 256, sm, s>>>(ca);
       CKZ(cudaGetLastError());
       const int nleft = (n - ca.whi + kZFarTile - 1) / kZFarTile;
@@ -848,7 +848,7 @@ int schur_large_cplx_run(double2* A, double2* Z, double2* w, int n, int scale, l
       const int tiles = nleft + nright + nz;
       if (tiles > 0) {
         sm = sizeof(double2) * ((size_t)wc * B * 3 + (size_t)nw * kZFarTile) + sizeof(int) * (size_t)wc * B + 16;
-        CKZ(cudaFuncSetAttribute(k_zchase_far, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        CKZ(allow_smem(k_zchase_far, kMostSmem));
         k_zchase_far<<<tiles, 256, sm, s>>>(ca, nleft, nright);
         CKZ(cudaGetLastError());
       }
