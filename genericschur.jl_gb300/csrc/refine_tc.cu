@@ -64,6 +64,10 @@ constexpr uint32_t kQIdesc = idesc_bf16(kQM, kQN);
 constexpr int kQExpZero = kExpZeroRow;             // row / column of zeros
 constexpr int kQExpBad = kExpBadRow;               // row / column with Inf or NaN
 constexpr unsigned long long kQTimeout = 4000000000ull;  // ~2 s of SM clock
+#ifndef GS_TC_WAIT_CYCLES  // limit of the pipeline's waits (a test builds with 0)
+#define GS_TC_WAIT_CYCLES kQTimeout
+#endif
+constexpr unsigned long long kQWait = GS_TC_WAIT_CYCLES;
 
 struct QCtl {
   uint64_t bar[2];     // MMA completion per stage (tcgen05.commit)
@@ -71,6 +75,7 @@ struct QCtl {
   uint32_t tslot;
   int ticket;
   int fail;
+  unsigned passed;     // chunks whose stage the issuing warp has seen full
   int exA[kQM];        // row exponents of A (the rows of op(X) in A_s Z)
   int exZ[kQM];        // column exponents of Z (rows of Z^T, columns of Z)
   int exP[kQM];        // column exponents of P = A_s Z
@@ -181,8 +186,10 @@ __device__ __forceinline__ void zero8(unsigned char* dst, int slice_bytes) {
   for (int s = 0; s < kQSlices; ++s) *reinterpret_cast<uint4*>(dst + s * slice_bytes) = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// A stage is full: the splitting warps arrive, the issuing warp waits.  (A stage's second
-// arrival follows a wait for the MMAs that its first one released, so arrivals never mix.)
+// A stage is full: the splitting warps arrive, the issuing warp waits.  A stage's second arrival
+// follows a wait for the MMAs that its first one released, or, once a wait has timed out, the issuing
+// warp's count, so arrivals never mix: the barrier counts threads, and with the arrivals of two chunks in
+// one phase the issuing warp could wait for ever.
 __device__ __forceinline__ void named_sync(int id, int count) {
   asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
@@ -232,13 +239,22 @@ __device__ bool tc_product(int n, const double* X, const double* Y, const int* e
       if (warp == 0) {
         // the issuing warp: every splitting warp has filled the stage
         named_sync(1 + st, kQThreads);
-        if (lane == 0 && !vfail()) issue(c, st, j0);
+        if (lane == 0) {
+          *(volatile unsigned*)&ctl.passed = gchunk + 1;
+          if (!vfail()) issue(c, st, j0);
+        }
         __syncwarp();
         continue;
       }
       // the MMAs that last read this stage must be complete before it is overwritten
-      if (lane == 0 && gchunk >= 2 && !vfail() && !mbar_wait(&ctl.bar[st], ((gchunk >> 1) - 1) & 1u, kQTimeout))
-        *(volatile int*)&ctl.fail = 1;
+      if (lane == 0 && gchunk >= 2) {
+        if (!vfail() && !mbar_wait(&ctl.bar[st], ((gchunk >> 1) - 1) & 1u, kQWait)) *(volatile int*)&ctl.fail = 1;
+        if (vfail()) {
+          // (ends as soon as the slowest splitting warp's own wait does)
+          const unsigned long long t0 = clock64();
+          while (*(volatile unsigned*)&ctl.passed < gchunk - 1 && clock64() - t0 <= 4 * kQTimeout) __nanosleep(200);
+        }
+      }
       __syncwarp();
       unsigned char* xs = smem + st * kQStage;
       const int k0 = c * kQK;
@@ -289,7 +305,7 @@ __device__ bool tc_product(int n, const double* X, const double* Y, const int* e
     // drain the panel: the last chunk's commit covers every MMA before it
     if (tid == 0 && !vfail()) {
       const unsigned last = gchunk - 1;
-      if (!mbar_wait(&ctl.bar[last & 1], (last >> 1) & 1u, kQTimeout)) *(volatile int*)&ctl.fail = 1;
+      if (!mbar_wait(&ctl.bar[last & 1], (last >> 1) & 1u, kQWait)) *(volatile int*)&ctl.fail = 1;
     }
     __syncthreads();
     if (ctl.fail) return false;
@@ -365,6 +381,7 @@ __global__ void __launch_bounds__(kQThreads, 1) k_refine_tc(RefineArgs a, int st
     mbar_init(&ctl.bar[1], 1);
     mbar_init(&ctl.done, 1);
     ctl.fail = 0;
+    ctl.passed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if ((tid >> 5) == 0) {
