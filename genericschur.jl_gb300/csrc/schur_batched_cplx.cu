@@ -838,7 +838,7 @@ cudaError_t launch_hess_c(const CplxBatch& bt, const int* order, const int* sche
   const size_t elems = chess_smem_elems(nmax), smem = sizeof(double2) * elems;
   cudaError_t e = allow_smem(k_hess_cplx<NC>, sizeof(double2) * chess_smem_elems(NC));
   if (e != cudaSuccess) return e;
-  k_hess_cplx<NC><<<bt.count, 4 * NC, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
+  k_hess_cplx<NC><<<bin_grid(bt.count, num_sms), 4 * NC, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
   return cudaGetLastError();
 }
 
@@ -852,13 +852,16 @@ cudaError_t launch_bin_c(const CplxBatch& bt, const int* order, int* sched, int 
   const size_t smem = ciqr_smem_bytes();
   e = allow_smem(k_schur_cplx<NT>, smem);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_cplx<NT>, NT, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
-  int grid = bt.count;  // as launch_bin of schur_batched_real.cu
-  if (ctas > 0) grid = std::min(grid, num_sms * std::min(per_sm, ctas));
-  k_schur_cplx<NT><<<grid, NT, smem, s>>>(bt, order, sched, bin, nmax, num_sms, ctas > 0 ? 0 : 1);
+  // as launch_bin of schur_batched_real.cu
+  int grid = bin_grid(bt.count, num_sms);
+  const int once = ctas == 0 && grid == bt.count;
+  if (ctas > 0) {
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_cplx<NT>, NT, smem);
+    if (e != cudaSuccess) return e;
+    grid = std::min(bt.count, num_sms * std::min(std::max(per_sm, 1), ctas));
+  }
+  k_schur_cplx<NT><<<grid, NT, smem, s>>>(bt, order, sched, bin, nmax, num_sms, once);
   return cudaGetLastError();
 }
 

@@ -1245,7 +1245,7 @@ cudaError_t launch_hess(const RealBatchT<T, W>& bt, const int* order, const int*
   else f = (const void*)k_hess_real32<W, NC>;
   cudaError_t e = allow_smem(f, sizeof(T) * hess_smem_elems(NC, sizeof(T)));
   if (e != cudaSuccess) return e;
-  const int ctas = bt.count;
+  const int ctas = bin_grid(bt.count, num_sms);
   if constexpr (sizeof(T) == 8) {
     k_hess_real64<W, NC><<<ctas, NT, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
   } else {
@@ -1267,15 +1267,17 @@ cudaError_t launch_bin(const RealBatchT<T, W>& bt, const int* order, int* sched,
   const size_t smem = sizeof(T) * bin_smem_elems(nmax);
   e = allow_smem(k_schur_real<T, W, NT>, sizeof(T) * bin_smem_elems(kSmallMax));
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_real<T, W, NT>, NT, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
-  // a CTA per matrix (those beyond the bin's share end at once), or, with a cap on CTAs per SM, as
-  // many as may be resident on a ticket queue
-  int grid = bt.count;
-  if (ctas > 0) grid = std::min(grid, num_sms * std::min(per_sm, ctas));
-  k_schur_real<T, W, NT><<<grid, NT, smem, s>>>(bt, order, sched, bin, nmax, num_sms, ctas > 0 ? 0 : 1);
+  // a CTA per matrix, or a ticket queue: of bin_grid's CTAs, or, with a cap on CTAs per SM, of as many as
+  // may be resident
+  int grid = bin_grid(bt.count, num_sms);
+  const int once = ctas == 0 && grid == bt.count;
+  if (ctas > 0) {
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur_real<T, W, NT>, NT, smem);
+    if (e != cudaSuccess) return e;
+    grid = std::min(bt.count, num_sms * std::min(std::max(per_sm, 1), ctas));
+  }
+  k_schur_real<T, W, NT><<<grid, NT, smem, s>>>(bt, order, sched, bin, nmax, num_sms, once);
   return cudaGetLastError();
 }
 
