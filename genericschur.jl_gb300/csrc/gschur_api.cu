@@ -101,12 +101,13 @@ int ensure_ws(gs_context* ctx, size_t bytes) {
 
 // The stream of the i-th largest size bin: the larger the orders, the higher the priority, so that the
 // longest-running matrices start first whenever room appears on an SM.  With equal priorities the bins'
-// order was left to chance: 2000 FP64 matrices n = 8..128 took 61 ms or 74 ms.
+// order was left to chance: 2000 FP64 matrices n = 8..128 took 61 ms or 74 ms.  Only that order is
+// wanted: the smallest orders have the default priority, and the highest is left to callers.
 cudaError_t bin_stream(cudaStream_t* s, int i) {
   int least = 0, greatest = 0;
   cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
   if (e != cudaSuccess) return e;
-  return cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, std::min(least, greatest + i));
+  return cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, std::max(greatest, least - (kNumBins - 1 - i)));
 }
 
 // Fork the aux streams off `s`, run `body(aux)`, join back into `s`.
