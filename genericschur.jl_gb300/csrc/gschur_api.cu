@@ -1115,8 +1115,12 @@ int gs_schur_c64(gs_context* ctx, int64_t n, double* A, int64_t lda, double* Z, 
   } else {
     int* order = (int*)(base + o_order);
     int* sched = (int*)(base + o_sched);
-    rc = run_single(ctx, (int)n, ctx->tun_cplx, order, sched, [&](int bin, cudaStream_t st) {
-      return launch_schur_cplx_bin(bt, order, sched, bin, ctx->tun_cplx, ctx->num_sms, st);
+    // at most a warp per sub-partition, whatever suits a batch: a fifth shares the chain warp's FP64 pipe
+    // (n = 128, eigenvalues alone 81.0 ms with 160 threads, 78.6 with 128; with Z 88.0, 83.9)
+    BinTuning tun = ctx->tun_cplx;
+    for (int& nt : tun.nt) nt = std::min(nt, 128);
+    rc = run_single(ctx, (int)n, tun, order, sched, [&](int bin, cudaStream_t st) {
+      return launch_schur_cplx_bin(bt, order, sched, bin, tun, ctx->num_sms, st);
     });
     if (rc) return rc;
   }
