@@ -631,16 +631,6 @@ __device__ __forceinline__ void apply_line(T* p, int inc, int d, const T* lg, in
   *p1 = z1;
 }
 
-// Correctly rounded 1/d of a normal d whose reciprocal is normal: one Newton step on a seed within one
-// ulp, exact for every significand but all ones (P. Markstein, IBM J. Res. Dev. 34, 1990); the seed
-// of that one is exact enough too (all 2^23 significands compared with __frcp_rn).  28 cycles
-// against 79 for __frcp_rn with its range test.
-__device__ __forceinline__ float rcp_markstein(float d) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
-  return fmaf(y, fmaf(-d, y, 1.0f), y);
-}
-
 // Reflector (householder.jl:12-54, as reflector_fast) of (a, x1, x2), x2 = 0 for a 2-element one;
 // a <- beta.  One test sends every case off the plain path to reflector_fast.
 __device__ __forceinline__ Refl<float> chain_refl(float& a, float x1, float x2, int nr, int) {
