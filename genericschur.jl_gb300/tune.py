@@ -1,8 +1,9 @@
 """Tuner of the batched Schur kernels' launch shapes (run on the GPU it tunes for).
 
-The persistent batched kernels (one CTA per matrix, a work queue per size bin) have a
-launch shape per bin: the bin's largest order, threads per CTA, whether the Hessenberg
-phase runs on a full copy of the matrix in shared memory, and a cap on CTAs per SM.
+The batched kernels (one CTA per matrix, a launch sequence per size bin) have a
+launch shape per bin: the bin's largest order, threads per CTA of the iteration, and a cap on
+CTAs per SM.  (The table's hsmem column, whether the Hessenberg reduction runs in shared
+memory, selects nothing since the reduction is a kernel of its own; it is written as 0.)
 This script times every compiled shape on each bin's share of the benchmark batches --
 20,000 real N(0,1) matrices with orders ~ U{8..128} (seed 4) and 5,000 complex ones
 (seed 5) -- picks the fastest per bin, then tries a few bin boundaries with the chosen
@@ -33,21 +34,8 @@ sys.path.insert(0, HERE)
 THREADS = [64, 96, 128, 160, 192, 256]
 DEFAULT_BOUNDS = [32, 64, 96, 128]
 DEFAULT_THREADS = [64, 64, 128, 128]
-DEFAULT_HSMEM = [1, 1, 0, 0]
 BOUND_SETS = [[32, 64, 96, 128], [32, 64, 104, 128], [32, 72, 104, 128], [40, 72, 104, 128],
               [32, 64, 112, 128], [48, 80, 112, 128], [24, 56, 96, 128]]
-MAX_DYN_SMEM = 227 * 1024 - 1024
-
-
-def smem_bytes(kind, nmax, hsmem):
-    """Dynamic shared memory per CTA, as the kernels size it."""
-    if kind in ("real_f64", "mixed_f32"):
-        full = nmax * (nmax | 1) if hsmem else 0
-        rpk = (nmax * (nmax + 7)) // 2  # real packed QR layout: column j keeps rows 1..j+3
-        return (8 if kind == "real_f64" else 4) * (max(full, rpk) + 6 * nmax + 32)
-    pk = (nmax * (nmax + 5)) // 2  # complex packed QR layout: column j keeps rows 1..j+2
-    h = nmax * (nmax | 1) if hsmem else pk
-    return 16 * (h + 4 * nmax) + 32 * 8 + 64
 
 
 def table_text(shapes, note):
@@ -55,8 +43,8 @@ def table_text(shapes, note):
     lines += ["# " + x for x in note]
     lines.append("# kind bin nmax threads hsmem ctas_per_sm")
     for kind in ("real_f64", "complex_f64", "mixed_f32"):
-        for b, (nmax, nt, hs, ctas) in enumerate(shapes[kind]):
-            lines.append("%s %d %d %d %d %d" % (kind, b, nmax, nt, hs, ctas))
+        for b, (nmax, nt, ctas) in enumerate(shapes[kind]):
+            lines.append("%s %d %d %d 0 %d" % (kind, b, nmax, nt, ctas))
     return "\n".join(lines) + "\n"
 
 
@@ -143,7 +131,7 @@ def main():
     os.environ["GS_TUNING"] = ""  # start from the built-in shapes
     ctx = gs.Context(0)
     t_start = time.time()
-    base_shapes = [(b, nt, hs, 0) for b, nt, hs in zip(DEFAULT_BOUNDS, DEFAULT_THREADS, DEFAULT_HSMEM)]
+    base_shapes = [(b, nt, 0) for b, nt in zip(DEFAULT_BOUNDS, DEFAULT_THREADS)]
     default = {"real_f64": list(base_shapes), "complex_f64": list(base_shapes), "mixed_f32": list(base_shapes)}
     batches = {"real_f64": batched_real(20000, seed=4), "complex_f64": batched_cplx(5000, seed=5)}
     chosen = {k: list(v) for k, v in default.items()}
@@ -164,20 +152,17 @@ def main():
                 assert bad == 0
                 best = (base_ms, default[kind][b])
                 for nt in THREADS:
-                    for hs in (0, 1):
-                        if smem_bytes(kind, hi, hs) > MAX_DYN_SMEM:
-                            continue
-                        cand = {k: list(v) for k, v in default.items()}
-                        cand[kind][b] = (hi, nt, hs, 0)
-                        apply(ctx, cand, tmp)
-                        ms = r.time(args.reps)
-                        w, bad = r.eigenvalues()
-                        ok = bad == 0 and close_enough(w, w_ref)
-                        log.append("%s bin %d (n %d..%d, %d matrices) threads %d hsmem %d: %.2f ms%s"
-                                   % (kind, b, blo, hi, len(sel), nt, hs, ms, "" if ok else " REJECTED"))
-                        print(log[-1], flush=True)
-                        if ok and ms < best[0] and ms < base_ms * (1.0 - args.margin):
-                            best = (ms, (hi, nt, hs, 0))
+                    cand = {k: list(v) for k, v in default.items()}
+                    cand[kind][b] = (hi, nt, 0)
+                    apply(ctx, cand, tmp)
+                    ms = r.time(args.reps)
+                    w, bad = r.eigenvalues()
+                    ok = bad == 0 and close_enough(w, w_ref)
+                    log.append("%s bin %d (n %d..%d, %d matrices) threads %d: %.2f ms%s"
+                               % (kind, b, blo, hi, len(sel), nt, ms, "" if ok else " REJECTED"))
+                    print(log[-1], flush=True)
+                    if ok and ms < best[0] and ms < base_ms * (1.0 - args.margin):
+                        best = (ms, (hi, nt, 0))
                 chosen[kind][b] = best[1]
                 del r
                 torch.cuda.empty_cache()
@@ -191,10 +176,8 @@ def main():
                 shapes = []
                 for b, hi in enumerate(bounds):
                     src = next(i for i, d in enumerate(DEFAULT_BOUNDS) if hi <= d)
-                    _, nt, hs, ctas = chosen[kind][src]
-                    if smem_bytes(kind, hi, hs) > MAX_DYN_SMEM:
-                        hs = 0
-                    shapes.append((hi, nt, hs, ctas))
+                    _, nt, ctas = chosen[kind][src]
+                    shapes.append((hi, nt, ctas))
                 cand[kind] = shapes
                 apply(ctx, cand, tmp)
                 ms = r.time(args.reps)
@@ -220,21 +203,19 @@ def main():
         for b in reversed(range(len(DEFAULT_BOUNDS))):
             hi = DEFAULT_BOUNDS[b]
             for nt in THREADS:
-                for hs in (0, 1):
-                    if nt == 160 or smem_bytes("mixed_f32", hi, hs) > MAX_DYN_SMEM or \
-                            (hi, nt, hs, 0) == chosen["mixed_f32"][b]:
-                        continue
-                    cand = {k: list(v) for k, v in chosen.items()}
-                    cand["mixed_f32"][b] = (hi, nt, hs, 0)
-                    apply(ctx, cand, tmp)
-                    ms = r.time(args.reps)
-                    _, bad = r.eigenvalues()
-                    log.append("mixed_f32 bin %d threads %d hsmem %d: whole mixed batch %.2f ms%s"
-                               % (b, nt, hs, ms, "" if bad == 0 else " REJECTED"))
-                    print(log[-1], flush=True)
-                    if bad == 0 and ms < cur * (1.0 - args.margin):
-                        cur = ms
-                        chosen["mixed_f32"][b] = (hi, nt, hs, 0)
+                if nt == 160 or (hi, nt, 0) == chosen["mixed_f32"][b]:  # 160 is not compiled in FP32
+                    continue
+                cand = {k: list(v) for k, v in chosen.items()}
+                cand["mixed_f32"][b] = (hi, nt, 0)
+                apply(ctx, cand, tmp)
+                ms = r.time(args.reps)
+                _, bad = r.eigenvalues()
+                log.append("mixed_f32 bin %d threads %d: whole mixed batch %.2f ms%s"
+                           % (b, nt, ms, "" if bad == 0 else " REJECTED"))
+                print(log[-1], flush=True)
+                if bad == 0 and ms < cur * (1.0 - args.margin):
+                    cur = ms
+                    chosen["mixed_f32"][b] = (hi, nt, 0)
         log.append("mixed_f32 whole mixed batch: default shapes %.2f ms, chosen %.2f ms" % (base, cur))
         print(log[-1], flush=True)
         del r
