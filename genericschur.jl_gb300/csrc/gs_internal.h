@@ -421,11 +421,15 @@ cudaError_t launch_std_blocks(int n, int N, const int* bs, const int* bz, double
 template <class S, class D> cudaError_t convert_array(const S* src, D* dst, size_t count, double scale, cudaStream_t s);
 cudaError_t launch_absmax(const double* A, size_t cnt, unsigned long long* out, int num_sms, cudaStream_t s);
 
-// CTAs of a bin's launch over a batch of `count` matrices: one per matrix of the bin, whose size only the
-// device knows, so those beyond it end at once.  Above 64 per SM, more than are resident whatever the bin,
-// CTAs take several: with one per matrix in each of the twelve launches, a million FP32 matrices of
-// orders 2 and 3 took 19.1 ms, now 12.8, and 100,000 of 2 to 4 2.21 ms, now 1.65.
-inline int bin_grid(int count, int num_sms) { return count < 64 * num_sms ? count : 64 * num_sms; }
+// CTAs of a bin's launches over a batch of `count` matrices: one per matrix of the bin, whose size only the
+// device knows, so those beyond it end at once, up to a number per SM above which CTAs take several: the
+// reductions stride, the iteration takes a ticket queue.  In FP32 the queue starts at 64 per SM: with a CTA
+// per matrix in each of the twelve launches, 100,000 matrices of orders 2 to 4 took 2.21 ms (now 1.65), a
+// million of 2 and 3 19.1 (12.8).  In FP64 a queue's CTAs of large orders stay where the next bin's could
+// start (20,000 matrices of orders 8 to 128 531 ms, 526 without; 97 to 128 1306, 1287), and the empty CTAs
+// weigh less: 1024 per SM.
+inline int bin_grid(int count, int num_sms, int per_sm) { return count < per_sm * num_sms ? count : per_sm * num_sms; }
+constexpr int kReduceCtas = 64, kIterCtas32 = 64, kIterCtas64 = 1024;
 
 // Size bins of the batched kernels.  `sched` holds, per bin, the
 // [start, end) range of that bin inside the sorted work order and a queue ticket

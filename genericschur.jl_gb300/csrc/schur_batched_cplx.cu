@@ -838,7 +838,7 @@ cudaError_t launch_hess_c(const CplxBatch& bt, const int* order, const int* sche
   const size_t elems = chess_smem_elems(nmax), smem = sizeof(double2) * elems;
   cudaError_t e = allow_smem(k_hess_cplx<NC>, sizeof(double2) * chess_smem_elems(NC));
   if (e != cudaSuccess) return e;
-  k_hess_cplx<NC><<<bin_grid(bt.count, num_sms), 4 * NC, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
+  k_hess_cplx<NC><<<bin_grid(bt.count, num_sms, kReduceCtas), 4 * NC, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
   return cudaGetLastError();
 }
 
@@ -853,7 +853,7 @@ cudaError_t launch_bin_c(const CplxBatch& bt, const int* order, int* sched, int 
   e = allow_smem(k_schur_cplx<NT>, smem);
   if (e != cudaSuccess) return e;
   // as launch_bin of schur_batched_real.cu
-  int grid = bin_grid(bt.count, num_sms);
+  int grid = bin_grid(bt.count, num_sms, kIterCtas64);
   const int once = ctas == 0 && grid == bt.count;
   if (ctas > 0) {
     int per_sm = 0;

@@ -1235,7 +1235,7 @@ cudaError_t launch_hess(const RealBatchT<T, W>& bt, const int* order, const int*
   else f = (const void*)k_hess_real32<W, NC>;
   cudaError_t e = allow_smem(f, sizeof(T) * hess_smem_elems(NC, sizeof(T)));
   if (e != cudaSuccess) return e;
-  const int ctas = bin_grid(bt.count, num_sms);
+  const int ctas = bin_grid(bt.count, num_sms, kReduceCtas);
   if constexpr (sizeof(T) == 8) {
     k_hess_real64<W, NC><<<ctas, NT, smem, s>>>(bt, order, sched, bin, nmax, (int)elems);
   } else {
@@ -1259,7 +1259,7 @@ cudaError_t launch_bin(const RealBatchT<T, W>& bt, const int* order, int* sched,
   if (e != cudaSuccess) return e;
   // a CTA per matrix, or a ticket queue: of bin_grid's CTAs, or, with a cap on CTAs per SM, of as many as
   // may be resident
-  int grid = bin_grid(bt.count, num_sms);
+  int grid = bin_grid(bt.count, num_sms, sizeof(T) == 4 ? kIterCtas32 : kIterCtas64);
   const int once = ctas == 0 && grid == bt.count;
   if (ctas > 0) {
     int per_sm = 0;
