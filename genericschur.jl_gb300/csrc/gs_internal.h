@@ -250,7 +250,8 @@ cudaError_t launch_eigvecs_batched(const EigBatch& eb, int nmax, int num_sms, cu
 // Real quasi-triangular -> complex triangular Schur pairs (triang.jl:9-43).
 struct TriBatch {
   int count;
-  const int* ns;
+  const int* ns;           // null: one matrix, of order n1, at offset 0
+  int n1;
   const long long* offs;   // element offsets of T/Z (real and complex buffers alike)
   const long long* woffs;  // offsets of w / colmap
   const double* Tr;
@@ -261,7 +262,7 @@ struct TriBatch {
   int* colmap;             // may be null
 };
 cudaError_t launch_triangularize(const TriBatch& tb, int num_sms, cudaStream_t s);
-// One matrix of any order over the whole GPU (Zr null: identity; Zc, w, colmap may be null).
+// One matrix of any order, from order 17 over the whole GPU (Zr null: identity; Zc, w, colmap may be null).
 cudaError_t launch_triangularize_one(int n, const double* Tr, const double* Zr, double2* Tc, double2* Zc, double2* w,
                                      int* colmap, cudaStream_t s);
 

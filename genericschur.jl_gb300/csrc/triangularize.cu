@@ -66,8 +66,8 @@ template <int NT>
 __global__ void __launch_bounds__(NT) k_triangularize(TriBatch tb) {
   const int tid = threadIdx.x;
   for (int b = blockIdx.x; b < tb.count; b += gridDim.x) {
-    const int n = tb.ns[b];
-    const long long off = tb.offs[b];
+    const int n = tb.ns ? tb.ns[b] : tb.n1;
+    const long long off = tb.ns ? tb.offs[b] : 0, woff = tb.ns ? tb.woffs[b] : 0;
     const double* __restrict__ Tr = tb.Tr + off;
     double2* __restrict__ Tc = tb.Tc + off;
     tri_sequential<NT>(n, Tr, tb.Zr ? tb.Zr + off : nullptr, Tc, tb.Zc ? tb.Zc + off : nullptr);
@@ -79,14 +79,14 @@ __global__ void __launch_bounds__(NT) k_triangularize(TriBatch tb) {
     __syncthreads();
     for (int k = tid; k < n; k += NT) {
       const double2 d = Tc[k + (long long)k * n];
-      if (tb.w) tb.w[tb.woffs[b] + k] = d;
+      if (tb.w) tb.w[woff + k] = d;
       if (tb.colmap) {
         int dst = k;
         const bool lower = (k + 1 < n) && Tr[(k + 1) + (long long)k * n] != 0.0;  // k is first of a pair
         const bool upper = (k > 0) && Tr[k + (long long)(k - 1) * n] != 0.0;      // k is second of a pair
         if (lower && d.y < 0.0) dst = k + 1;
         if (upper && Tc[(k - 1) + (long long)(k - 1) * n].y < 0.0) dst = k - 1;
-        tb.colmap[tb.woffs[b] + k] = dst;
+        tb.colmap[woff + k] = dst;
       }
     }
     __syncthreads();
@@ -214,6 +214,22 @@ __global__ void k_tri_finish(int n, const double* __restrict__ Tr, double2* __re
 cudaError_t launch_triangularize_one(int n, const double* Tr, const double* Zr, double2* Tc, double2* Zc, double2* w,
                                      int* colmap, cudaStream_t s) {
   if (n < 1) return cudaSuccess;
+  // One CTA up to order 16: there a launch costs more than the rotations one after the other (host
+  // call, n = 3 40.7 us, with the launches below 48.4; 10 50.9, 57.6; 16 64.2, 67.1 with the one-CTA
+  // kernel and its orders in device memory).
+  if (n <= 16) {
+    TriBatch tb{};
+    tb.count = 1;
+    tb.n1 = n;
+    tb.Tr = Tr;
+    tb.Zr = Zr;
+    tb.Tc = Tc;
+    tb.Zc = Zc;
+    tb.w = w;
+    tb.colmap = colmap;
+    k_triangularize<128><<<1, 128, 0, s>>>(tb);
+    return cudaGetLastError();
+  }
   if (double* flag = tri_flag(n, Tc)) {
     cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(double), s);
     if (e != cudaSuccess) return e;

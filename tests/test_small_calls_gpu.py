@@ -1,0 +1,25 @@
+"""Calls whose launches depend on the order or the number of matrices: the small forms give what the general
+ones give."""
+import numpy as np
+import pytest
+
+EPS = np.finfo(float).eps
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 18])
+@pytest.mark.parametrize("wantz", [True, False])
+def test_triangularize_one_cta_bound(gs, n, wantz):
+    # orders on both sides of the one-CTA bound
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n))
+    S = gs.gschur(A, wantZ=wantz)
+    C = gs.triangularize(S)
+    assert np.all(np.tril(C.T, -1) == 0)
+    w = np.sort_complex(np.diag(C.T))
+    # the rotations are unitary: eigenvalues and norm stay to rounding
+    assert np.abs(np.linalg.norm(C.T) - np.linalg.norm(S.T)) <= 50 * n * EPS * np.linalg.norm(S.T)
+    assert np.array_equal(w, np.sort_complex(C.values))
+    if wantz:
+        R = A @ C.Z - C.Z @ C.T
+        assert np.linalg.norm(R) <= 100 * n * EPS * max(np.linalg.norm(A), 1.0)
