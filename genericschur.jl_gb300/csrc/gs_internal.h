@@ -18,9 +18,10 @@ constexpr size_t kMostSmem = kMaxDynSmem - 8 * 1024;
 
 // Lets a kernel's launches ask for up to `most` bytes of dynamic shared memory.  The limit belongs to the
 // function, not to a launch: `most` is the same in every call, so that a launch that another thread makes
-// in between cannot lower it below what this one needs.
-template <class F> cudaError_t allow_smem(F* kernel, size_t most) {
-  if (most <= 40 * 1024) return cudaSuccess;  // every kernel may have 48 KB, its static arrays included
+// in between cannot lower it below what this one needs.  A launch that needs little (`smem`, where given) leaves
+// the limit alone.
+template <class F> cudaError_t allow_smem(F* kernel, size_t most, size_t smem = kMaxDynSmem) {
+  if (most <= 40 * 1024 || smem <= 40 * 1024) return cudaSuccess;  // every kernel may have 48 KB, its static arrays included
   return cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
@@ -198,6 +199,7 @@ struct HeCtlBuf {
 };
 // where the control block holds the int that says that a grid-wide wait gave up
 template <class S> constexpr size_t kHeErrOffset = 2 * sizeof(S) + 4 * sizeof(unsigned);
+constexpr int kHeOneCta = 32;  // orders that one CTA tridiagonalizes alone (no grid-wide wait)
 // W: 2 n entries
 template <class S>
 cudaError_t launch_he_tridiag(const S* A, long long lda, int n, int upper, S* B, S* W, S* partial, int npart,

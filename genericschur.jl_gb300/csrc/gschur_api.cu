@@ -3122,7 +3122,8 @@ int heev_impl(gs_context* ctx, int64_t n, double* A, int64_t lda, int uplo, doub
   std::vector<double> dh(n);
   int gave_up = 0;
   CK(cudaMemcpyAsync(dh.data(), d, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&gave_up, base + L.o_ctl + kHeErrOffset<S>, sizeof(int), cudaMemcpyDeviceToHost, s));
+  if (n > kHeOneCta)
+    CK(cudaMemcpyAsync(&gave_up, base + L.o_ctl + kHeErrOffset<S>, sizeof(int), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   if (gave_up) return set_err(ctx, GS_CUDA, "tridiagonalization: a grid-wide wait gave up");
   std::vector<int> p(n);
@@ -3181,7 +3182,8 @@ int hetrd_impl(gs_context* ctx, int64_t n, double* A, int64_t lda, int uplo, dou
   std::vector<double> hd(n), he(n > 1 ? n - 1 : 1);
   std::vector<S> ht(n > 1 ? n - 1 : 1);
   int gave_up = 0;
-  CK(cudaMemcpyAsync(&gave_up, base + L.o_ctl + kHeErrOffset<S>, sizeof(int), cudaMemcpyDeviceToHost, s));
+  if (n > kHeOneCta)
+    CK(cudaMemcpyAsync(&gave_up, base + L.o_ctl + kHeErrOffset<S>, sizeof(int), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(hd.data(), dd, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   if (n > 1) {
     CK(cudaMemcpyAsync(he.data(), de, sizeof(double) * (n - 1), cudaMemcpyDeviceToHost, s));

@@ -36,7 +36,6 @@ namespace gsk {
 namespace {
 
 constexpr int kHeT = 256;
-constexpr int kHeOneCta = 32;  // orders of k_he_tridiag that one CTA takes alone
 constexpr int kHeCols = 4;     // columns per CTA above that, until every SM has a CTA
 #ifndef GS_HE_WAIT_POLLS  // polls of a grid-wide wait before it gives up, some seconds (a test builds with 0)
 #define GS_HE_WAIT_POLLS (1 << 22)
@@ -1006,6 +1005,10 @@ cudaError_t launch_he_tridiag(const S* A, long long lda, int n, int upper, S* B,
   const int G = n <= kHeOneCta ? 1 : std::min(num_sms, (n + kHeCols - 1) / kHeCols);
   const size_t smem = ((size_t)((n + G - 1) / G) + 2) * n * sizeof(S);
   if (smem <= kMaxDynSmem) {
+    if (G == 1) {  // (a cooperative launch takes 4 us longer)
+      k_he_tridiag<S><<<1, kHeT, smem, s>>>(B, n, W, ctl, tau, d, e);
+      return cudaGetLastError();
+    }
     err = allow_smem(k_he_tridiag<S>, kMaxDynSmem);
     if (err != cudaSuccess) return err;
     void* args[] = {&B, &n, &W, &ctl, &tau, &d, &e};
@@ -1031,7 +1034,7 @@ cudaError_t launch_he_formq(const S* B, int n, const S* tau, S* Q, int num_sms, 
   const int nw = (int)std::min<size_t>(kHeT / 32, kMaxDynSmem / ((size_t)n * sizeof(S)));
   if (nw >= 4) {
     const size_t smem = (size_t)nw * n * sizeof(S);
-    cudaError_t err = allow_smem(k_he_formq_cols<S>, kMaxDynSmem);
+    cudaError_t err = allow_smem(k_he_formq_cols<S>, kMaxDynSmem, smem);
     if (err != cudaSuccess) return err;
     k_he_formq_cols<S><<<std::min(n, num_sms), 32 * nw, smem, s>>>(B, n, tau, Q);
     return cudaGetLastError();

@@ -1774,7 +1774,7 @@ cudaError_t launch_ggschur_real(const QzrBatch& bt, int num_sms, cudaStream_t s)
     if (bt.ns && cap < most / 2) cap = std::max(cap, std::min((size_t)(4 * one), most / 2));
   }
   const size_t smem = sizeof(double) * cap;
-  cudaError_t e = allow_smem(k_ggschur_real, most * sizeof(double));
+  cudaError_t e = allow_smem(k_ggschur_real, most * sizeof(double), smem);
   if (e != cudaSuccess) return e;
   const int grid = std::min(bt.count, 8 * num_sms);
   k_ggschur_real<<<grid, kQrT, smem, s>>>(bt, (int)cap);

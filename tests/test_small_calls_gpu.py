@@ -23,3 +23,18 @@ def test_triangularize_one_cta_bound(gs, n, wantz):
     if wantz:
         R = A @ C.Z - C.Z @ C.T
         assert np.linalg.norm(R) <= 100 * n * EPS * max(np.linalg.norm(A), 1.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [np.float64, np.complex128])
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 32, 33, 34])
+def test_hermitian_one_cta_bound(gs, dtype, n):
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)).astype(dtype)
+    if dtype == np.complex128:
+        A = A + 1j * rng.standard_normal((n, n))
+    A = (A + A.conj().T) / 2
+    E = gs.geigen(gs.Hermitian(A, "L"), alg="DivideAndConquer")
+    w, V = E.values, E.vectors
+    assert np.linalg.norm(A @ V - V * w) <= 100 * n * EPS * np.linalg.norm(A)
+    assert np.linalg.norm(V.conj().T @ V - np.eye(n)) <= 100 * n * EPS
