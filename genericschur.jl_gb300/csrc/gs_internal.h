@@ -49,6 +49,7 @@ struct RealBatchT {
   int scale;
   int maxiter_mult;  // maxiter = maxiter_mult * n (reference default 100)
   long long maxiter_abs;  // when > 0, overrides maxiter_mult
+  unsigned empty;    // bit i: size bin i is known to hold no matrix, its kernels are not launched
 };
 using RealBatch = RealBatchT<double>;
 
@@ -67,6 +68,7 @@ struct CplxBatch {
   int maxinner_mult; // maxinner = maxinner_mult * n (reference default 30)
   long long maxiter_abs;   // when > 0, overrides maxiter_mult
   long long maxinner_abs;  // when > 0, overrides maxinner_mult
+  unsigned empty;    // as in RealBatchT
 };
 // One complex matrix of order n > 128 on the whole GPU (schur_large_cplx.cu): Hessenberg
 // reduction, multishift QR, blocks <= 128 by the batched kernel.  A (device, ld n) <- T,
@@ -197,9 +199,9 @@ cudaError_t launch_ggschur_real(const QzrBatch& bt, int num_sms, cudaStream_t s)
 struct HeCtlBuf {
   alignas(16) unsigned char bytes[64];
 };
+constexpr int kHeOneCta = 32;  // orders that one CTA tridiagonalizes alone (no grid-wide wait)
 // where the control block holds the int that says that a grid-wide wait gave up
 template <class S> constexpr size_t kHeErrOffset = 2 * sizeof(S) + 4 * sizeof(unsigned);
-constexpr int kHeOneCta = 32;  // orders that one CTA tridiagonalizes alone (no grid-wide wait)
 // W: 2 n entries
 template <class S>
 cudaError_t launch_he_tridiag(const S* A, long long lda, int n, int upper, S* B, S* W, S* partial, int npart,

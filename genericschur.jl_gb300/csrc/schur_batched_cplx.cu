@@ -883,6 +883,7 @@ cudaError_t launch_schur_batched_cplx_tuned(const CplxBatch& bt, const int* orde
   // largest bin first: it carries most of the work
   for (int i = 0; i < kNumBins; ++i) {
     const int bin = kNumBins - 1 - i;
+    if (bt.empty >> bin & 1) continue;
     cudaError_t e = launch_shape_c(bt, order, sched, bin, t.bounds[bin], t.nt[bin], t.ctas[bin], num_sms,
                                    streams[i % nstreams]);
     if (e != cudaSuccess) return e;

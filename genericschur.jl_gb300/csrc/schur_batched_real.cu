@@ -1296,6 +1296,7 @@ cudaError_t launch_all_bins(const RealBatchT<T, W>& bt, const int* order, int* s
   // largest bin first: it carries most of the work
   for (int i = 0; i < kNumBins; ++i) {
     const int bin = kNumBins - 1 - i;
+    if (bt.empty >> bin & 1) continue;
     cudaError_t e = launch_shape(bt, order, sched, bin, t.bounds[bin], t.nt[bin], t.ctas[bin], num_sms,
                                  streams[i % nstreams]);
     if (e != cudaSuccess) return e;

@@ -38,3 +38,21 @@ def test_hermitian_one_cta_bound(gs, dtype, n):
     w, V = E.values, E.vectors
     assert np.linalg.norm(A @ V - V * w) <= 100 * n * EPS * np.linalg.norm(A)
     assert np.linalg.norm(V.conj().T @ V - np.eye(n)) <= 100 * n * EPS
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex128])
+@pytest.mark.parametrize("orders", [[1], [0, 5], [32, 33], [64, 65, 0], [128], [2] * 160 + [128], [40] * 153, [96, 97, 3]])
+def test_batches_without_some_bins(gs, dtype, orders):
+    # every matrix as in a batch that has matrices in all size bins and more of them than SMs
+    rng = np.random.default_rng(len(orders) + orders[0])
+    mats = [rng.standard_normal((n, n)).astype(dtype) for n in orders]
+    rest = [rng.standard_normal((n, n)).astype(dtype) for n in [5, 40, 70, 100, 128] * 40]
+    for wantz in (True, False):
+        Ts, Zs, ws, st = gs.gschur_batched(mats, wantZ=wantz)
+        Tr, Zr, wr, sr = gs.gschur_batched(mats + rest, wantZ=wantz)
+        assert np.all(st == 0) and np.all(sr == 0)
+        for k in range(len(mats)):
+            assert np.array_equal(Ts[k], Tr[k]) and np.array_equal(ws[k], wr[k])
+            if wantz:
+                assert np.array_equal(Zs[k], Zr[k])
