@@ -1764,7 +1764,9 @@ cudaError_t launch_ggordschur_real(int n, double* S, double* T, double* Q, doubl
 cudaError_t launch_ggschur_real(const QzrBatch& bt, int num_sms, cudaStream_t s) {
   if (bt.count <= 0) return cudaSuccess;
   // shared memory for the largest pencil's four matrices, or two, as far as it reaches (bt.nmax, 0:
-  // not known, two CTAs per SM)
+  // not known, two CTAs per SM).  Beyond a pencil per SM two CTAs are ahead: 1000 of orders 9 to 65 60.7 ms, one
+  // by the largest pencil's size 93.5 (139.6 with all matrices in global memory); 600 of 66 to 82 99.8, 169, 190;
+  // 1000 of 8 to 16 7.5, by their own size 6.5, 11.8.
   const size_t most = (kMaxDynSmem - 4 * 1024) / sizeof(double);
   const long long one = (long long)bt.nmax * (bt.nmax | 1);
   size_t cap = most / 2;

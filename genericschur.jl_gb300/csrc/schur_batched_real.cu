@@ -1187,7 +1187,8 @@ __device__ void solve_real(const RealBatchT<T, W>& bt, int b, int nmax, T* smem,
 }
 #undef HH
 
-// 768 threads per SM: at most 80 registers
+// 768 threads per SM: at most 80 registers, at which FP64 spills 72 bytes (for one matrix too, where the
+// occupancy is of no use)
 template <class T, class W, int NT>
 __global__ void __launch_bounds__(NT, 768 / NT) k_schur_real(RealBatchT<T, W> bt, const int* __restrict__ order,
                                                    int* __restrict__ sched, int bin, int nmax, int num_sms, int once) {
