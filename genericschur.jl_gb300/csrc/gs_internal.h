@@ -494,8 +494,11 @@ cudaError_t launch_schur_batched_real32_tuned(const RealBatchT<float, float>& bt
                                               int num_sms, cudaStream_t* streams, int nstreams, const BinTuning& tun);
 cudaError_t launch_schur_batched_cplx(const CplxBatch& bt, const int* order, int* sched,
                                       int num_sms, cudaStream_t* streams, int nstreams);
+// iterate false: the reductions alone, for launch_schur_cplx_all.
 cudaError_t launch_schur_batched_cplx_tuned(const CplxBatch& bt, const int* order, int* sched, int num_sms,
-                                            cudaStream_t* streams, int nstreams, const BinTuning& tun);
+                                            cudaStream_t* streams, int nstreams, const BinTuning& tun,
+                                            bool iterate = true);
+cudaError_t launch_schur_cplx_all(const CplxBatch& bt, const int* order, int num_sms, cudaStream_t s);
 // One bin's kernels (the queue prepared, shapes from `tun`).
 template <class T, class W>
 cudaError_t launch_schur_real_bin(const RealBatchT<T, W>& bt, const int* order, int* sched, int bin,

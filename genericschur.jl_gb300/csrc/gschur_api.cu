@@ -964,9 +964,17 @@ static int run_batched_cplx(gs_context* ctx, CplxBatch bt, const int32_t* host_n
   auto enqueue = [&](cudaStream_t s) -> int {
     cudaError_t e = launch_bin_sort(bt.ns, bt.count, order, sched, bounds, s);
     if (e != cudaSuccess) return set_err(ctx, GS_CUDA, "bin sort launch: %s", cudaGetErrorString(e));
-    return fork_join(ctx, s, [&](cudaStream_t* aux) {
-      return launch_schur_batched_cplx_tuned(bt, order, sched, ctx->num_sms, aux, kNumBins, ctx->tun_cplx);
+    // up to six matrices per SM the iterations in one launch (above that the bins' threads and residency
+    // matter more: 1,024 of order 64 72 ms in one launch, 65 by bins; 800 of 8 to 80 41, 45 to 70)
+    bool all = bt.count > 1 && bt.count <= 6 * ctx->num_sms;
+    for (int cap : ctx->tun_cplx.ctas) all = all && cap == 0;
+    const int rc = fork_join(ctx, s, [&](cudaStream_t* aux) {
+      return launch_schur_batched_cplx_tuned(bt, order, sched, ctx->num_sms, aux, kNumBins, ctx->tun_cplx, !all);
     });
+    if (rc || !all) return rc;
+    e = launch_schur_cplx_all(bt, order, ctx->num_sms, s);
+    if (e != cudaSuccess) return set_err(ctx, GS_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+    return GS_OK;
   };
   CK(cudaEventRecord(ctx->t0, ctx->stream));
   if (use_graph) {

@@ -799,6 +799,21 @@ __device__ void solve_cplx(const CplxBatch& bt, int b, int nmax, double2* smem, 
 }
 #undef HH
 
+// All matrices of a batch of a few per SM in one launch, whatever their bin, after all reductions.  The time of such
+// a batch is that of its largest matrices and of what shares an SM with them.  The bins' own launches left that
+// to chance: a bin's CTAs went where the next one's reductions were done first, four of the largest to an
+// SM (600 matrices of orders 8 to 128 114 to 117 ms, 101 to 135 with a persistent CTA per SM before).  Here
+// the sorted order is dealt to the SMs in rounds of num_sms, every other round backwards, so that the
+// largest shares its SM with the smallest; between two and four per SM the shared memory asked for keeps two
+// at a time, the rest as they end: 600 99 to 101 ms, 500 96 to 101 (104 to 118; 98 to 103), 304 of 112 to
+// 128 115 (150; 178).  With four at a time 600 take 111 to 114, 500 100 to 107.
+__global__ void __launch_bounds__(128, 4) k_schur_cplx_all(CplxBatch bt, const int* __restrict__ order, int num_sms) {
+  extern __shared__ double2 smemz[];
+  const int round = blockIdx.x / num_sms, at = blockIdx.x % num_sms;
+  const int job = round * num_sms + (round & 1 ? num_sms - 1 - at : at);
+  if (job < bt.count) solve_cplx<128>(bt, order[job], kSmallMax, smemz, round & 3);
+}
+
 template <int NT>
 __global__ void __launch_bounds__(NT, NT <= 128 ? 512 / NT : 2) k_schur_cplx(CplxBatch bt, const int* __restrict__ order,
                                                                 int* __restrict__ sched, int bin, int nmax,
@@ -844,11 +859,11 @@ cudaError_t launch_hess_c(const CplxBatch& bt, const int* order, const int* sche
 
 template <int NT>
 cudaError_t launch_bin_c(const CplxBatch& bt, const int* order, int* sched, int bin, int nmax, int ctas, int num_sms,
-                         cudaStream_t s) {
+                         cudaStream_t s, bool iterate) {
   cudaError_t e = nmax <= 32 ? launch_hess_c<32>(bt, order, sched, bin, nmax, num_sms, s)
                              : (nmax <= 64 ? launch_hess_c<64>(bt, order, sched, bin, nmax, num_sms, s)
                                            : launch_hess_c<128>(bt, order, sched, bin, nmax, num_sms, s));
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || !iterate) return e;
   const size_t smem = ciqr_smem_bytes();
   e = allow_smem(k_schur_cplx<NT>, smem);
   if (e != cudaSuccess) return e;
@@ -867,9 +882,9 @@ cudaError_t launch_bin_c(const CplxBatch& bt, const int* order, int* sched, int 
 
 // One bin with the requested thread count (kTuneThreads).
 cudaError_t launch_shape_c(const CplxBatch& bt, const int* order, int* sched, int bin, int nmax, int nt, int ctas,
-                           int num_sms, cudaStream_t s) {
+                           int num_sms, cudaStream_t s, bool iterate = true) {
 #define GS_SHAPE(NTV) \
-  if (nt == NTV) return launch_bin_c<NTV>(bt, order, sched, bin, nmax, ctas, num_sms, s);
+  if (nt == NTV) return launch_bin_c<NTV>(bt, order, sched, bin, nmax, ctas, num_sms, s, iterate);
   GS_SHAPE(64) GS_SHAPE(96) GS_SHAPE(128) GS_SHAPE(160) GS_SHAPE(192) GS_SHAPE(256)
 #undef GS_SHAPE
   return cudaErrorInvalidValue;
@@ -877,15 +892,24 @@ cudaError_t launch_shape_c(const CplxBatch& bt, const int* order, int* sched, in
 
 }  // namespace
 
+cudaError_t launch_schur_cplx_all(const CplxBatch& bt, const int* order, int num_sms, cudaStream_t s) {
+  const int grid = (bt.count + num_sms - 1) / num_sms * num_sms;
+  const size_t pair = 100 * 1024;
+  const size_t smem = bt.count > 2 * num_sms && bt.count <= 4 * num_sms ? pair : ciqr_smem_bytes();
+  cudaError_t e = allow_smem(k_schur_cplx_all, pair, smem);
+  if (e != cudaSuccess) return e;
+  k_schur_cplx_all<<<grid, 128, smem, s>>>(bt, order, num_sms);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_schur_batched_cplx_tuned(const CplxBatch& bt, const int* order, int* sched, int num_sms,
-                                            cudaStream_t* streams, int nstreams, const BinTuning& t) {
+                                            cudaStream_t* streams, int nstreams, const BinTuning& t, bool iterate) {
   // largest bin first: it carries most of the work
   for (int i = 0; i < kNumBins; ++i) {
     const int bin = kNumBins - 1 - i;
     if (bt.empty >> bin & 1) continue;
     cudaError_t e = launch_shape_c(bt, order, sched, bin, t.bounds[bin], t.nt[bin], t.ctas[bin], num_sms,
-                                   streams[i % nstreams]);
+                                   streams[i % nstreams], iterate);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

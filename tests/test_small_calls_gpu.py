@@ -56,3 +56,24 @@ def test_batches_without_some_bins(gs, dtype, orders):
             assert np.array_equal(Ts[k], Tr[k]) and np.array_equal(ws[k], wr[k])
             if wantz:
                 assert np.array_equal(Zs[k], Zr[k])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [2, 151, 152, 153, 304, 305, 608, 609, 912, 913])
+def test_complex_rounds(gs, count):
+    # rounds of one launch over the SMs: every matrix once, each as by itself
+    rng = np.random.default_rng(count)
+    orders = rng.integers(0, 13, size=count)
+    orders[:2] = [30, 90]
+    mats = [rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) for n in orders]
+    Ts, Zs, ws, st = gs.gschur_batched(mats)
+    assert np.all(st == 0)
+    for k in list(range(0, count, 37)) + [1, count - 1]:
+        if orders[k] == 0:
+            continue
+        S = gs.gschur(mats[k])
+        assert np.array_equal(Ts[k], S.T) and np.array_equal(Zs[k], S.Z) and np.array_equal(ws[k], S.values)
+    for A, T, Z in zip(mats, Ts, Zs):
+        n = A.shape[0]
+        if n:
+            assert np.linalg.norm(A @ Z - Z @ T) <= 100 * n * EPS * np.linalg.norm(A)
